@@ -1529,28 +1529,10 @@ __global__ void k_ck_thin(const O1Ckpt *__restrict__ src, const unsigned long lo
 // under a scale refined for the one-cell floor, then single cells move by marginal coded size
 // (count / (n - 1/2) compared in integers) until the table is full.  An empty context gets all
 // cells on symbol 0, a context with one symbol all cells on it.
-__device__ __forceinline__ void warp_best(unsigned long long &bc, unsigned long long &bd, int &bs, bool want_max) {
-    // the best fraction bc / bd over the warp (ties: the lower symbol); bs < 0 marks no candidate
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long oc = __shfl_xor_sync(0xffffffffu, bc, o);
-        const unsigned long long od = __shfl_xor_sync(0xffffffffu, bd, o);
-        const int os = __shfl_xor_sync(0xffffffffu, bs, o);
-        bool take;
-        if (os < 0) take = false;
-        else if (bs < 0) take = true;
-        else {
-            const unsigned long long l = oc * bd, r = bc * od;
-            take = want_max ? (l > r || (l == r && os < bs)) : (l < r || (l == r && os < bs));
-        }
-        if (take) {
-            bc = oc;
-            bd = od;
-            bs = os;
-        }
-    }
-}
-
+// The moves are a serial chain (up to hundreds a table), so a move costs as little as it can: every
+// symbol's marginal size is kept as an integer key and only the moved symbol's is computed again;
+// the best key of the warp takes three warp reductions.  (Comparing the fractions themselves across
+// the warp on every move took 107 us for the 30 tables of a 384^3 float64 field, this 44 us.)
 __global__ void __launch_bounds__(256) k_o1_norm(const uint32_t *__restrict__ hist, int total_tables,
                                                  uint16_t *__restrict__ nf) {
     const int wt = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -1609,28 +1591,42 @@ __global__ void __launch_bounds__(256) k_o1_norm(const uint32_t *__restrict__ hi
         if (left == 0 || ones_count == total) break;
         mu = (double)(O1_M - ones) / (double)(total - ones_count);
     }
-    while (left != 0) {
+    if (left != 0) {
+        // 2 c / (2 n + 1) for a cell more, 2 c / (2 n - 1) for a cell less, as floor(. 2^29): two
+        // different fractions with denominators up to 16385 lie more than 2^-28.01 apart, so the keys
+        // compare as the fractions do.  The largest key moves (complemented for a cell less; 0: none).
         const bool add = left > 0;
-        unsigned long long bc = 0, bd = 1;
-        int bs = -1;
+        auto key_of = [&](uint32_t cnt_i, int n_i) -> unsigned long long {
+            if (!cnt_i || (!add && n_i < 2)) return 0;
+            const unsigned long long k = ((unsigned long long)cnt_i << 30) / (unsigned)(add ? 2 * n_i + 1 : 2 * n_i - 1);
+            return add ? k : ~k;
+        };
+        unsigned long long key[PER];
 #pragma unroll
-        for (int i = 0; i < PER; i++) {
-            if (!c[i] || (!add && n[i] < 2)) continue;
-            const unsigned long long c2 = 2ull * c[i], d = add ? 2ull * n[i] + 1 : 2ull * n[i] - 1;
-            if (bs < 0 || (add ? c2 * bd > bc * d : c2 * bd < bc * d)) {
-                bc = c2;
-                bd = d;
-                bs = lane + 32 * i;
+        for (int i = 0; i < PER; i++) key[i] = key_of(c[i], n[i]);
+        for (; left != 0; left += add ? -1 : 1) {
+            unsigned long long bk = key[0];
+            int bi = 0;
+#pragma unroll
+            for (int i = 1; i < PER; i++)
+                if (key[i] > bk) {
+                    bk = key[i];
+                    bi = i;
+                }
+            const uint32_t hi = (uint32_t)(bk >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+            const uint32_t lo = hi == mh ? (uint32_t)bk : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+            if ((mh | ml) == 0) break;  // nothing movable (cannot happen: fewer symbols than cells)
+            const bool mine = hi == mh && lo == ml;
+            const uint32_t bs = __reduce_min_sync(0xffffffffu, mine ? (uint32_t)(lane + 32 * bi) : ~0u);
+            if (mine && bs == (uint32_t)(lane + 32 * bi)) {  // ties: the lower symbol
+#pragma unroll
+                for (int i = 0; i < PER; i++)
+                    if (i == bi) {
+                        n[i] += add ? 1 : -1;
+                        key[i] = key_of(c[i], n[i]);
+                    }
             }
         }
-        warp_best(bc, bd, bs, add);
-        if (bs < 0) break;  // nothing movable (cannot happen: fewer symbols than cells)
-        if ((bs & 31) == lane) {
-#pragma unroll
-            for (int i = 0; i < PER; i++)
-                if (lane + 32 * i == bs) n[i] += add ? 1 : -1;
-        }
-        left += add ? -1 : 1;
     }
 #pragma unroll
     for (int i = 0; i < PER; i++) freq[lane + 32 * i] = (uint16_t)n[i];
@@ -1638,85 +1634,106 @@ __global__ void __launch_bounds__(256) k_o1_norm(const uint32_t *__restrict__ hi
 
 // ---- tANS tables for 15 contexts x 256 symbols, built by a whole CTA per table (zfse
 // fse_compress.c FSE_buildCTable_wksp / fse_decompress.c FSE_buildDTable, restated in parallel).
-constexpr int kTabThreads = 256;
+// A table is 8192 cells and there are as few as 15 of them, so what bounds the build is one CTA's
+// latency: 32 warps scan, spread and rank 256 cells each.  (One warp ranking all cells took 80 us
+// for 15 encode tables and 101 us for the decode tables; this takes 9 and 17 us.)
+constexpr int kTabThreads = 1024;
+constexpr int kTabCells = O1_M / kTabThreads;  // visits, then cells, per thread
+static_assert(kTabCells * 32 == O1_M / 32, "a warp ranks the 256 cells of its own span");
 struct TabSmem {
     int16_t norm[O1_NSYM];
     uint32_t cum[O1_NSYM + 1];   // cells before every symbol (a -1 symbol holds one cell)
     uint32_t occ[O1_NSYM + 1];   // spread occurrences before every symbol (positive counts only)
-    uint32_t cnt[O1_NSYM];       // running per-symbol counters of the rank pass
-    uint32_t part[kTabThreads];
+    uint32_t scan[3][32];
+    uint16_t cnt[32][O1_NSYM];   // cells of every symbol in every warp's span, then before it
     uint8_t sym[O1_M];
-    int bad;
 };
 
 // The spread (fse::spread): symbol s takes the occurrences occ[s] .. occ[s+1]-1 of the visit order
 // j -> (j * step) & mask that skips the cells above `high` (the -1 symbols' cells).  Every thread
-// maps one run of j; a block scan of the kept visits gives each its occurrence number.
-__device__ void cta_spread(TabSmem &w, unsigned tl) {
-    const uint32_t tsize = 1u << tl, mask = tsize - 1, step = fse::table_step(tsize);
-    if (threadIdx.x == 0) {
-        uint32_t c = 0, o = 0, high = tsize - 1;
-        for (int s2 = 0; s2 < O1_NSYM; s2++) {
-            w.cum[s2] = c;
-            w.occ[s2] = o;
-            const int nn = w.norm[s2];
-            if (nn == -1) {
-                w.sym[high--] = (uint8_t)s2;
-                c += 1;
-            } else if (nn > 0) {
-                c += (uint32_t)nn;
-                o += (uint32_t)nn;
-            }
-        }
-        w.cum[O1_NSYM] = c;
-        w.occ[O1_NSYM] = o;
-        w.bad = c != tsize;
+// maps one run of j; a block scan of the kept visits gives each its occurrence number.  Returns
+// false (for every thread) when the counts do not fill the table.
+__device__ bool cta_spread(TabSmem &w) {
+    constexpr uint32_t mask = O1_M - 1;
+    const uint32_t step = fse::table_step(O1_M);
+    uint32_t ones = 0, cells = 0;  // a -1 symbol's cell, the other symbols' cells
+    if (threadIdx.x < O1_NSYM) {
+        const int nn = w.norm[threadIdx.x];
+        ones = nn == -1;
+        cells = nn > 0 ? (uint32_t)nn : 0u;
     }
-    __syncthreads();
-    const uint32_t high = tsize - 1 - (w.cum[O1_NSYM] - w.occ[O1_NSYM]);
-    const uint32_t per = tsize / blockDim.x;  // tsize is a multiple of the block size
-    const uint32_t j0 = threadIdx.x * per;
+    uint32_t n_ones, n_cells;
+    const uint32_t o = block_excl_scan<uint32_t>(ones, w.scan[0], n_ones);
+    const uint32_t c = block_excl_scan<uint32_t>(cells, w.scan[1], n_cells);
+    if (n_ones + n_cells != (uint32_t)O1_M) return false;
+    if (threadIdx.x < O1_NSYM) {
+        w.cum[threadIdx.x] = o + c;
+        w.occ[threadIdx.x] = c;
+        if (ones) w.sym[mask - o] = (uint8_t)threadIdx.x;  // the -1 symbols take the top cells in order
+    }
+    if (threadIdx.x == 0) {
+        w.cum[O1_NSYM] = O1_M;
+        w.occ[O1_NSYM] = n_cells;
+    }
+    const uint32_t high = mask - n_ones, j0 = threadIdx.x * kTabCells;
     uint32_t kept = 0;
-    for (uint32_t j = j0; j < j0 + per; j++) kept += ((j * step) & mask) <= high;
-    w.part[threadIdx.x] = kept;
-    __syncthreads();
-    uint32_t k = 0;
-    for (uint32_t t2 = 0; t2 < threadIdx.x; t2++) k += w.part[t2];
-    for (uint32_t j = j0; j < j0 + per; j++) {
-        const uint32_t pos = (j * step) & mask;
+#pragma unroll
+    for (uint32_t j = 0; j < kTabCells; j++) kept += (((j0 + j) * step) & mask) <= high;
+    uint32_t all;
+    uint32_t k = block_excl_scan<uint32_t>(kept, w.scan[2], all);  // its barriers publish cum and occ
+    int sy = 0;  // the symbol whose occurrences hold k: occ[sy] <= k < occ[sy + 1]
+    for (int hi = O1_NSYM; hi - sy > 1;) {
+        const int mid = (sy + hi) >> 1;
+        if (w.occ[mid] <= k) sy = mid;
+        else hi = mid;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kTabCells; j++) {
+        const uint32_t pos = ((j0 + j) * step) & mask;
         if (pos > high) continue;
-        int lo = 0, hi = O1_NSYM;  // the symbol whose occurrences hold k: occ[lo] <= k < occ[lo+1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (w.occ[mid] <= k) lo = mid;
-            else hi = mid;
-        }
-        w.sym[pos] = (uint8_t)lo;
+        while (w.occ[sy + 1] <= k) sy++;
+        w.sym[pos] = (uint8_t)sy;
         k++;
     }
     __syncthreads();
+    return true;
 }
 
-// For every cell u in increasing order, f(u, s, rank) with rank = the cells of symbol s before u
-// (warp 0, 32 cells at a time with match ranks).
+// For every cell u, f(u, s, rank) with rank = the cells of symbol s before u: match ranks within 32
+// cells, counted up over the warp's span, then the counts of the spans before.
 template <class F>
-__device__ void cta_ranks(TabSmem &w, uint32_t tsize, F &&f) {
-    for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) w.cnt[s2] = 0;
+__device__ void cta_ranks(TabSmem &w, F &&f) {
+    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint16_t *cnt = w.cnt[wid];
+    for (int s2 = lane; s2 < O1_NSYM; s2 += 32) cnt[s2] = 0;
+    __syncwarp();
+    uint32_t rank[kTabCells];
+#pragma unroll
+    for (int i = 0; i < kTabCells; i++) {
+        const unsigned sy = w.sym[wid * (O1_M / 32) + i * 32 + lane];
+        const unsigned peers = __match_any_sync(0xffffffffu, sy);
+        const unsigned r = __popc(peers & ((1u << lane) - 1u));
+        rank[i] = cnt[sy] + r;
+        __syncwarp();
+        if (r == (unsigned)__popc(peers) - 1u) cnt[sy] = (uint16_t)(rank[i] + 1);
+        __syncwarp();
+    }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const unsigned lane = threadIdx.x;
-        for (uint32_t u0 = 0; u0 < tsize; u0 += 32) {
-            const uint32_t u = u0 + lane;
-            const unsigned sy = w.sym[u];
-            const unsigned peers = __match_any_sync(0xffffffffu, sy);
-            const unsigned rank = __popc(peers & ((1u << lane) - 1u));
-            f(u, sy, w.cnt[sy] + rank);
-            __syncwarp();
-            if (rank == (unsigned)__popc(peers) - 1u) w.cnt[sy] += rank + 1;
-            __syncwarp();
+    if (threadIdx.x < O1_NSYM) {
+        uint32_t run = 0;
+#pragma unroll 8
+        for (int v = 0; v < 32; v++) {
+            const uint32_t c = w.cnt[v][threadIdx.x];
+            w.cnt[v][threadIdx.x] = (uint16_t)run;
+            run += c;
         }
     }
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kTabCells; i++) {
+        const unsigned u = wid * (O1_M / 32) + i * 32 + lane, sy = w.sym[u];
+        f(u, sy, rank[i] + cnt[sy]);
+    }
 }
 
 __global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__restrict__ nf, uint16_t *__restrict__ stab,
@@ -1724,16 +1741,19 @@ __global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__res
                                                          int *__restrict__ err) {
     (void)scratch;
     __shared__ TabSmem w;
+    __shared__ uint4 s_st[O1_M / 8];  // the state table, written out whole
     const size_t t = blockIdx.x;
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) w.norm[s2] = (int16_t)nf[t * O1_NSYM + s2];
     __syncthreads();
-    cta_spread(w, O1_PB);
-    if (w.bad) {
+    if (!cta_spread(w)) {
         if (threadIdx.x == 0) atomicExch(err, 4);
         return;
     }
-    uint16_t *st = stab + t * O1_M;
-    cta_ranks(w, O1_M, [&](uint32_t u, unsigned sy, uint32_t r) { st[w.cum[sy] + r] = (uint16_t)(O1_M + u); });
+    uint16_t *st = reinterpret_cast<uint16_t *>(s_st);
+    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) { st[w.cum[sy] + r] = (uint16_t)(O1_M + u); });
+    __syncthreads();
+    uint4 *out = reinterpret_cast<uint4 *>(stab + t * O1_M);
+    for (int i = threadIdx.x; i < O1_M / 8; i += blockDim.x) out[i] = s_st[i];
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) {
         const int nn = w.norm[s2];
         const uint32_t total = w.cum[s2];
@@ -1763,13 +1783,12 @@ __global__ void __launch_bounds__(kTabThreads) k_o1_dtable(const uint16_t *__res
     const size_t t = blockIdx.x;
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) w.norm[s2] = (int16_t)nf[t * O1_NSYM + s2];
     __syncthreads();
-    cta_spread(w, O1_PB);
-    if (w.bad) {
+    if (!cta_spread(w)) {
         if (threadIdx.x == 0) atomicExch(err, 5);
         return;
     }
     uint32_t *d = dt + t * O1_M;
-    cta_ranks(w, O1_M, [&](uint32_t u, unsigned sy, uint32_t r) {
+    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) {
         const int nn = w.norm[sy];
         const uint32_t ns = (nn == -1 ? 1u : (uint32_t)nn) + r;
         const uint32_t nb = O1_PB - fse::highbit32(ns);
