@@ -1736,24 +1736,37 @@ __device__ void cta_ranks(TabSmem &w, F &&f) {
     }
 }
 
-__global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__restrict__ nf, uint16_t *__restrict__ stab,
-                                                         fse::SymTT *__restrict__ stt, uint8_t *__restrict__ scratch,
+// A table set as the chain encoder holds it in shared memory: the 15 packed state tables, then two words per key.
+constexpr unsigned kTabWords = O1_M * O1_PB / 32;  // packed words of a context's state table
+constexpr size_t kEncSmem = ((size_t)O1_NCTX * kTabWords + (size_t)O1_NCTX * O1_NSYM * 2) * 4;
+static_assert(kEncSmem % 16 == 0 && kEncSmem + 2048 <= 227 * 1024, "16-byte words; 2 KiB for the kernels' own arrays");
+// The words of key context << 8 | symbol: deltaNbBits (state x emits (x + deltaNbBits) >> 16 bits) and 13
+// times (deltaFindState + 8192 context), which added to 13 times the shifted state is the place of the next
+// state's packed entry.
+// The encoder's image of table blockIdx.x (k_o1_walk below): its state table packed, its symbol transforms.
+__global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__restrict__ nf, uint32_t *__restrict__ image,
                                                          int *__restrict__ err) {
-    (void)scratch;
     __shared__ TabSmem w;
-    __shared__ uint4 s_st[O1_M / 8];  // the state table, written out whole
+    __shared__ uint16_t st[O1_M + 4];  // cells by symbol, in increasing order
     const size_t t = blockIdx.x;
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) w.norm[s2] = (int16_t)nf[t * O1_NSYM + s2];
+    if (threadIdx.x < 4) st[O1_M + threadIdx.x] = 0;
     __syncthreads();
     if (!cta_spread(w)) {
         if (threadIdx.x == 0) atomicExch(err, 4);
         return;
     }
-    uint16_t *st = reinterpret_cast<uint16_t *>(s_st);
-    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) { st[w.cum[sy] + r] = (uint16_t)(O1_M + u); });
+    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) { st[w.cum[sy] + r] = (uint16_t)u; });
     __syncthreads();
-    uint4 *out = reinterpret_cast<uint4 *>(stab + t * O1_M);
-    for (int i = threadIdx.x; i < O1_M / 8; i += blockDim.x) out[i] = s_st[i];
+    uint32_t *img = image + (t / O1_NCTX) * (kEncSmem / 4), c = (uint32_t)(t % O1_NCTX);
+    for (unsigned wd = threadIdx.x; wd < kTabWords; wd += blockDim.x) {
+        // bits [32 wd, 32 wd + 32) of the entries (entry j at bit 13 j): at most 4 of them
+        const unsigned j0 = wd * 32 / O1_PB, sh = wd * 32 - j0 * O1_PB;
+        unsigned long long v = 0;
+#pragma unroll
+        for (unsigned u = 0; u < 4; u++) v |= (unsigned long long)st[j0 + u] << (O1_PB * u);
+        img[c * kTabWords + wd] = (uint32_t)(v >> sh);
+    }
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) {
         const int nn = w.norm[s2];
         const uint32_t total = w.cum[s2];
@@ -1770,7 +1783,8 @@ __global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__res
             tt.deltaNbBits = (maxBitsOut << 16) - minStatePlus;
             tt.deltaFindState = (int32_t)total - nn;
         }
-        stt[t * O1_NSYM + s2] = tt;
+        reinterpret_cast<uint2 *>(img + O1_NCTX * kTabWords)[c * O1_NSYM + s2] =
+            make_uint2(tt.deltaNbBits, (uint32_t)(tt.deltaFindState + (int32_t)(c << O1_PB)) * O1_PB);
     }
 }
 
@@ -1897,472 +1911,826 @@ __global__ void __launch_bounds__(kChainThreads) k_o1_decode_smem(const uint8_t 
     if (br.pos < br.start_bit(sb) - 16) atomicExch(err, 8);
 }
 
-// Context frequencies of one table set: the stationary distribution of the context chain implied
-// by the normalized tables (the next context is a function of the decoded code; escapes split
-// between the two large-magnitude contexts).  Returns (map, rev) for `slots` resident tables.
 // ---- parallel chain encoder
-// Every chain is cut into parts of `part` codes, one part per thread, all parts of a chain in one
-// CTA.  A tANS encoder walks its chain backwards and only its state carries from one code to the
-// next, so:
-//   1. every part runs from a guessed entering state (the top part from the exact initial state),
-//      writing its bits to its own staging area and keeping the state and the bit count at every
-//      64th index (`sparse`, `sparse_bits`) and its exit state;
-//   2. repair rounds: each part reruns from the exit state of the part above, writing the bits
-//      again into a second staging area, until its state equals a kept one (from there on the two
-//      runs, and their bits, are identical); a part that never meets its kept states has a new
-//      exit state, so the part below repairs again in the next round.  Encoder states from
-//      different starting points meet after a few hundred codes, so one round nearly always
-//      suffices, and the loop ends after at most one round per part;
-//   3. (the bits of a part: the repaired bits above the meeting index, then the speculative ones)
-//   4. the bit counts give every part its offset in the chain's stream; every part shifts its
-//      staged bits into place (words shared with a neighbour are merged with atomicOr);
-//   5. every part start is a decode checkpoint: state, bit position, context and escape count.
+// Every chain is cut into parts of `part` codes, one part per thread.  A tANS encoder walks its
+// chain backwards and only its state carries from one code to the next, so the parts are coded in
+// steps, each a launch over all parts of all chains:
+//   1. k_o1_walk: every part runs from a guessed entering state (the top part from the exact initial
+//      state), writing the bits of every 8 codes as one record and keeping the state and the bit count
+//      at every 64th index (`kept`, `kept_bits`) and its exit state;
+//   2. k_o1_repair: every part runs again from the exit state of the part above, writing its records
+//      and kept states over, until its state equals the one kept there (from there on the two runs, and
+//      their records, are identical); a part that never meets has a new exit state;
+//   3. k_o1_rounds, a CTA per chain: the parts whose entering state changed run again, in rounds;
+//   4. where many parts did not meet, or rounds did not settle them: k_o1_maps, k_o1_compose and
+//      k_o1_walk again (below);
+//   5. k_o1_settle, a CTA per chain: scans the bit counts into every part's offset and writes the decode
+//      checkpoints: state, bit position, context and escape count at every part start;
+//   6. k_o1_place: joins the records' bits in the chain's slot.
 // The stream is bit-identical to a sequential encoder's (the tANS states are fully determined).
-// All 15 context state tables stay in shared memory: the two contexts that carry most codes (from
-// the table set's histogram) as 16-bit states, the other 13 as 13-bit entries (state - 8192)
-// packed into words; one word per key holds the symbol transform.  k_spec_image lays this out once
-// per table set in global memory, and every CTA copies it in.
-constexpr int kSpecThreads = 1024;
-constexpr int kSpecHot = 2;
-constexpr unsigned kSpecPackWords = (O1_NCTX - kSpecHot) * O1_M * O1_PB / 32 + 1;  // + 1: a read of w + 1
-constexpr size_t kSpecSmem =
-    ((size_t)kSpecHot * O1_M * 2 + (size_t)kSpecPackWords * 4 + (size_t)O1_NCTX * O1_NSYM * 4 + 15) & ~(size_t)15;
-// Which table slot every context of a table set takes (4 bits each; slots 0 and 1 are the 16-bit
-// tables).
-struct SpecMeta {
-    unsigned long long map;
-};
-constexpr int kSparseShift = 6;  // kept speculative states: every 64th index
-struct SpecCta {
+//
+// What bounds it: a walk is a serial chain of table lookups, so its time is the codes of a part times
+// the latency of a step where few parts share an SM, and the shared-memory pipe (three lookups a code,
+// each about 3.4 bank conflicts deep) where an SM is full of them.  So the parts of all chains are
+// spread evenly over the SMs whatever chain they belong to (with all parts of a chain in one CTA, a
+// field of one segment ran on 16 of the 148 SMs), over about kEncWarps warps of a CTA (fewer lanes a
+// warp wait less for one another, more warps cost issue slots); the transforms of 8 codes are looked
+// up ahead of their steps; and records of a fixed 16 bytes per 8 codes leave as whole coalesced
+// vectors, where words stored as they filled hit a line a lane.  All launches together, before (one
+// kernel, a CTA a chain) and now: 64^3 points 289 -> 118 us, 211 x 307 x 401 1144 -> 485 us, 1800 x 3600 at
+// 1.4 bits a code 36.2 -> 1.1 ms, 512^3 at 8.5 bits 1021 -> 800 us, at 1.6 bits 62 -> 5.3 ms.
+//
+// All 15 context state tables stay in shared memory, as 13-bit entries (state - 8192) packed into
+// words, so that no lookup leaves the SM and every context takes the same instructions (two 16-bit
+// tables beside 13 packed ones cost every warp both paths); two words per key hold the symbol
+// transform (one word fits too, but takes a dozen more instructions a code to unpack).  k_o1_ctable lays this image out once per table set; every CTA copies it in.
+constexpr int kEncThreads = 1024;
+constexpr uint32_t kEncWarps = 4, kMinEncPart = 256;
+constexpr int kKeptShift = 6;  // kept states: every 64th index
+
+// Parts [first, first + count) of one table set: warp w codes the parts first + w * lanes + l, l < lanes.
+// Its records interleave (record r of lane l at rec + (w * records of a part + r) * lanes + l).
+struct EncCta {
     int table;
-    int first;  // first chain
-    int count;  // chains
-    int ppc;    // threads per chain (>= parts of every chain of the CTA)
-    unsigned long long map, rev;
+    uint32_t first, count, lanes;
+    uint32_t chain;          // chain of the first part
+    unsigned long long rec;  // records of the CTAs before
+};
+struct EncChain {
+    unsigned long long lo, hi;  // its codes
+};
+struct EncArgs {
+    const uint16_t *keys;        // context of code i (0 at a chain's first code) << 8 | symbol, by k_o1_hist
+    const EncChain *chains;
+    const uint32_t *pstart;      // first part of every chain, then the number of parts
+    uint32_t nchains, part, recs;  // codes per part, records per part
+    const uint32_t *image;       // table sets, kEncSmem bytes each
+    const EncCta *ctas;
+    // per part: exit state of the first walk and of the last one, entering state of the last one (map
+    // path: the exact one, written ahead of its walk), bits, escapes, first record | lanes << 56, first bit in the slots, records to place (bit
+    // 31: and the final state's)
+    uint16_t *exit1, *exit2, *entry;
+    uint32_t *bits, *esc, *nrec;
+    unsigned long long *column, *at;
+    uint16_t *kept, *kept_bits;
+    uint4 *rec;
+    int *err;                    // [0] error, [2] codes run again, [3] rounds, [5] parts that did not meet,
+                                 // [6] chains that the rounds did not settle
 };
 
-// Staging words of one part: 13 bits per code at most, plus the final state and end mark.
-__host__ __device__ __forceinline__ size_t spec_stage_words(uint32_t part) { return ((size_t)part * 13 + 64) / 32 + 4; }
+// Records of one part: its groups of 8 codes (by index) and the final state's.
+inline uint32_t part_records(uint32_t part) { return part / 8 + 2; }
 
-// keys[i] = context of code i (from code i-1; 0 at a chain's first code) << 8 | symbol of code i,
-// written by k_o1_hist.
+// Whether rounds are left out, and whether the map path codes this call: where more than one part in
+// eight did not meet its kept states, rounds pass a changed state down part by part, and where fewer did
+// not, but several in a row, kMaxRounds do not settle them.  A round is a part's walk, 55 us, the map path
+// 0.9 ms at 6.5 M codes and 4.2 ms at 134 M.
+constexpr uint32_t kMaxRounds = 16;
+__device__ __forceinline__ bool many_unmet(const EncArgs &A) {
+    return (uint32_t)__ldcg(A.err + 5) > __ldg(A.pstart + A.nchains) / 2;
+}
+__device__ __forceinline__ bool map_path(const EncArgs &A) { return many_unmet(A) || __ldcg(A.err + 6) != 0; }
 
-// Calls f(i, keys[i]) for i = top down to bottom, reading the keys through aligned 16-byte vectors
-// (8 keys) fetched two vectors ahead.
-template <class F>
-__device__ __forceinline__ void walk_keys(const uint16_t *__restrict__ keys, long long top, long long bottom, F &&f) {
-    long long i = top;
-    for (; i >= bottom && (i & 7) != 7; i--) f(i, (uint32_t)__ldg(keys + i));
-    if (i - 7 >= bottom) {
-        const uint4 *kv = reinterpret_cast<const uint4 *>(keys);
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        uint4 v0 = __ldg(kv + ((i - 7) >> 3));
-        uint4 v1 = i - 15 >= 0 ? __ldg(kv + ((i - 15) >> 3)) : z;
-        while (i - 7 >= bottom) {
-            const uint4 v2 = i - 23 >= 0 ? __ldg(kv + ((i - 23) >> 3)) : z;
-            f(i, v0.w >> 16);
-            f(i - 1, v0.w & 0xFFFFu);
-            f(i - 2, v0.z >> 16);
-            f(i - 3, v0.z & 0xFFFFu);
-            f(i - 4, v0.y >> 16);
-            f(i - 5, v0.y & 0xFFFFu);
-            f(i - 6, v0.x >> 16);
-            f(i - 7, v0.x & 0xFFFFu);
-            i -= 8;
-            v0 = v1;
-            v1 = v2;
-        }
+struct EncPartPos {
+    uint32_t chain, p, nparts;
+    long long a, first;  // the part's lowest code; the first (highest) one it codes
+    bool is_top;         // the chain's last code initialises the state
+};
+// Part `id` (of a chain at or after `chain`).
+__device__ __forceinline__ EncPartPos enc_part(const EncArgs &A, uint32_t id, uint32_t chain) {
+    uint32_t hi = A.nchains;  // pstart[chain] <= id < pstart[hi]
+    while (hi - chain > 1) {
+        const uint32_t mid = (chain + hi) >> 1;
+        if (__ldg(A.pstart + mid) <= id) chain = mid;
+        else hi = mid;
     }
-    for (; i >= bottom; i--) f(i, (uint32_t)__ldg(keys + i));
+    EncPartPos r;
+    const uint32_t p0 = __ldg(A.pstart + chain);
+    const EncChain c = A.chains[chain];
+    r.chain = chain;
+    r.p = id - p0;
+    r.nparts = __ldg(A.pstart + chain + 1) - p0;
+    r.a = (long long)c.lo + (long long)r.p * A.part;
+    r.is_top = r.p + 1 == r.nparts;
+    r.first = r.is_top ? (long long)c.hi - 2 : r.a + A.part - 1;
+    return r;
 }
 
-// As walk_keys, but stops (and returns true) at the first index for which f returns true.
+__device__ __forceinline__ void load_image(uint4 *smem, const uint32_t *image, int table) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(image + (size_t)table * (kEncSmem / 4));
+#pragma unroll 4
+    for (unsigned i = threadIdx.x; i < kEncSmem / 16; i += blockDim.x) smem[i] = __ldg(src + i);
+}
+
+// A record: bits 0-103 those of up to 8 codes (LSB first, as the stream), 120-127 their count.
+__device__ __forceinline__ uint4 make_record(unsigned long long lo, unsigned long long hi, uint32_t n) {
+    return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32) | (n << 24));
+}
+
+// The table set in the CTA's dynamic shared memory.
+struct EncTables {
+    static __device__ __forceinline__ const uint32_t *words() {
+        extern __shared__ uint4 smem_raw[];
+        return reinterpret_cast<const uint32_t *>(smem_raw);
+    }
+    // the transform of a key
+    static __device__ __forceinline__ uint2 transform(uint32_t key) {
+        return reinterpret_cast<const uint2 *>(words() + O1_NCTX * kTabWords)[key];
+    }
+    static __device__ __forceinline__ uint32_t entry(uint32_t bit) {
+        const uint32_t *w = words() + (bit >> 5);
+        return (__funnelshift_r(w[0], w[1], bit) & (O1_M - 1)) | O1_M;
+    }
+    // state x codes a key with transform e: the bits it emits, their number, the next state
+    static __device__ __forceinline__ uint32_t next(uint32_t x, uint2 e, uint32_t &v, uint32_t &nb) {
+        nb = (x + e.x) >> 16;
+        const uint32_t r = x >> nb;
+        v = x - (r << nb);
+        return entry(r * O1_PB + e.y);
+    }
+    // FSE_initCState2: the state that codes symbol k with the fewest bits
+    static __device__ __forceinline__ uint32_t init(uint32_t key) {
+        const uint2 e = transform(key);
+        const uint32_t nb = (e.x + (1u << 15)) >> 16;
+        return entry((((nb << 16) - e.x) >> nb) * O1_PB + e.y);
+    }
+    // The 8 codes of a vector of keys, the last one first: their record's bits, their number.
+    static __device__ __forceinline__ uint4 group(uint32_t &x, const uint4 &v, uint32_t &n) {
+        const uint32_t k[8] = {v.w >> 16, v.w & 0xFFFFu, v.z >> 16, v.z & 0xFFFFu,
+                               v.y >> 16, v.y & 0xFFFFu, v.x >> 16, v.x & 0xFFFFu};
+        uint2 e[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) e[j] = transform(k[j]);
+        unsigned long long q[2];
+        uint32_t nq[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t w[2], nw[2];
+#pragma unroll
+            for (int g = 0; g < 2; g++) {
+                uint32_t va, na, vb, nb;
+                x = next(x, e[4 * h + 2 * g], va, na);
+                x = next(x, e[4 * h + 2 * g + 1], vb, nb);
+                w[g] = va | (vb << na);
+                nw[g] = na + nb;
+            }
+            q[h] = (unsigned long long)w[0] | ((unsigned long long)w[1] << nw[0]);
+            nq[h] = nw[0] + nw[1];
+        }
+        n = nq[0] + nq[1];
+        return make_record(q[0] | (q[1] << nq[0]), nq[0] ? q[1] >> (64 - nq[0]) : 0ull, n);
+    }
+    // The same for the codes from i down to e of one vector's span.
+    static __device__ __forceinline__ uint4 partial(uint32_t &x, const uint16_t *keys, long long i, long long e,
+                                                    uint32_t &n) {
+        unsigned long long lo = 0, hi = 0;
+        n = 0;
+        for (; i >= e; i--) {
+            uint32_t v32, nb;
+            x = next(x, transform(__ldg(keys + i)), v32, nb);
+            const unsigned long long v = v32;
+            if (n < 64) {
+                lo |= v << n;
+                if (n + nb > 64) hi |= v >> (64 - n);
+            } else {
+                hi |= v << (n - 64);
+            }
+            n += nb;
+        }
+        return make_record(lo, hi, n);
+    }
+};
+
+// Codes keys[first] down to keys[a] by the vectors of 8 keys they lie in, fetched ahead: f(i, r, n, v) for every record r of n bits, i its lowest index and v its keys (only whole
+// vectors: `whole`); stops and returns true where f does.
 template <class F>
-__device__ __forceinline__ bool walk_keys_until(const uint16_t *__restrict__ keys, long long top, long long bottom,
-                                                F &&f) {
-    long long i = top;
-    for (; i >= bottom && (i & 7) != 7; i--)
-        if (f(i, (uint32_t)__ldg(keys + i))) return true;
-    if (i - 7 >= bottom) {
+__device__ __forceinline__ bool walk_records(const uint16_t *__restrict__ keys, long long first,
+                                             long long a, uint32_t &x, F &&f) {
+    if (first < a) return false;
+    long long g = first >> 3;
+    const long long ga = a >> 3;
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    uint32_t n;
+    if ((first & 7) != 7 || g * 8 < a) {
+        const long long e = max(g * 8, a);
+        const uint4 r = EncTables::partial(x, keys, first, e, n);
+        if (f(e, r, n, z, false)) return true;
+        g--;
+    }
+    const long long gl = (a & 7) ? ga + 1 : ga;  // the lowest whole vector
+    if (g >= gl) {
+        // a ring of three vectors, each loaded into its place as soon as its keys are coded (a shift of
+        // the ring would wait for the load it moves)
         const uint4 *kv = reinterpret_cast<const uint4 *>(keys);
-        const uint4 z = make_uint4(0, 0, 0, 0);
-        uint4 v0 = __ldg(kv + ((i - 7) >> 3));
-        uint4 v1 = i - 15 >= 0 ? __ldg(kv + ((i - 15) >> 3)) : z;
-        while (i - 7 >= bottom) {
-            const uint4 v2 = i - 23 >= 0 ? __ldg(kv + ((i - 23) >> 3)) : z;
-            if (f(i, v0.w >> 16) || f(i - 1, v0.w & 0xFFFFu) || f(i - 2, v0.z >> 16) || f(i - 3, v0.z & 0xFFFFu) ||
-                f(i - 4, v0.y >> 16) || f(i - 5, v0.y & 0xFFFFu) || f(i - 6, v0.x >> 16) || f(i - 7, v0.x & 0xFFFFu))
-                return true;
-            i -= 8;
-            v0 = v1;
-            v1 = v2;
+        auto load = [&](long long j) { return j >= gl ? __ldg(kv + j) : z; };
+        auto one = [&](uint4 &v) {
+            const uint4 r = EncTables::group(x, v, n);
+            if (f(g * 8, r, n, v, true)) return true;
+            v = load(g - 3);
+            g--;
+            return false;
+        };
+        uint4 v0 = load(g), v1 = load(g - 1), v2 = load(g - 2);
+        for (;;) {
+            if (one(v0)) return true;
+            if (g < gl) break;
+            if (one(v1)) return true;
+            if (g < gl) break;
+            if (one(v2)) return true;
+            if (g < gl) break;
         }
     }
-    for (; i >= bottom; i--)
-        if (f(i, (uint32_t)__ldg(keys + i))) return true;
+    if (g >= ga) {
+        const uint4 r = EncTables::partial(x, keys, g * 8 + 7, a, n);
+        if (f(a, r, n, z, false)) return true;
+    }
     return false;
 }
 
-// Per key (context << 8 | symbol) the encoder's symbol transform, as one word: deltaFindState +
-// 8192 (bits 0-13), minStatePlus - 8192 (14-27) and maxBitsOut (28-31); the emitted bit count of
-// state x is maxBitsOut - (x < minStatePlus), which is (x + deltaNbBits) >> 16 with deltaNbBits =
-// (maxBitsOut << 16) - minStatePlus.
-__host__ __device__ __forceinline__ uint32_t enc_word(const fse::SymTT &t) {
-    const uint32_t mbo = (t.deltaNbBits + 0xFFFFu) >> 16, msp = (mbo << 16) - t.deltaNbBits;
-    return (uint32_t)(t.deltaFindState + O1_M) | ((msp - O1_M) << 14) | (mbo << 28);
+// Runs the state through the codes without recording their bits.
+__device__ __forceinline__ void walk_states(const uint16_t *keys, long long first, long long a,
+                                            uint32_t &x) {
+    walk_records(keys, first, a, x, [](long long, const uint4 &, uint32_t, const uint4 &, bool) { return false; });
 }
 
-// The chain encoder's shared-memory image of table set blockIdx.y (kSpecSmem bytes at image +
-// blockIdx.y * kSpecSmem / 4, laid out as k_o1_encode_spec's dynamic shared memory), filled by all
-// blocks of the grid's x dimension: the 16-bit tables of the two contexts with the most codes in
-// the set's histogram, the other contexts' 13-bit packed entries, and the transform word of every key.
-__global__ void __launch_bounds__(256) k_spec_image(const uint16_t *__restrict__ stab,
-                                                    const fse::SymTT *__restrict__ stt,
-                                                    const uint32_t *__restrict__ thist, uint32_t *__restrict__ image,
-                                                    SpecMeta *__restrict__ meta) {
-    __shared__ uint32_t s_tot[O1_NCTX];
-    __shared__ uint8_t s_rev[O1_NCTX];  // context of every slot
-    const size_t tb = (size_t)blockIdx.y * O1_NCTX;
-    const uint16_t *__restrict__ S = stab + tb * O1_M;
-    if (threadIdx.x < O1_NCTX) s_tot[threadIdx.x] = 0;
+// Escapes (symbol 255) among 8 keys.
+__device__ __forceinline__ uint32_t escapes_of(const uint4 &v) {
+    auto m = [](uint32_t w) { return ((w & 0x00FF00FFu) + 0x00010001u) & 0x01000100u; };  // bits 8 and 24
+    return __popc(m(v.x) | (m(v.y) >> 1) | (m(v.z) >> 2) | (m(v.w) >> 3));
+}
+
+// The walk of every part: EXACT = false from a guessed entering state (the state that codes the next
+// code with the fewest bits), true from the exact one (`entry`, the map path only).
+template <bool EXACT>
+__global__ void __launch_bounds__(kEncThreads) k_o1_walk(const EncArgs A) {
+    extern __shared__ uint4 smem_raw[];
+    if (EXACT && !map_path(A)) return;
+    const EncCta w = A.ctas[blockIdx.x];
+    load_image(smem_raw, A.image, w.table);
     __syncthreads();
-    {
-        // codes per context: 16 threads per context, 16 symbols each
-        const unsigned c = threadIdx.x / 16, s0 = (threadIdx.x % 16) * 16;
-        if (c < (unsigned)O1_NCTX) {
-            uint32_t v = 0;
-#pragma unroll
-            for (int u = 0; u < 16; u++) v += __ldg(thist + (tb + c) * O1_NSYM + s0 + u);
-            atomicAdd(&s_tot[c], v);
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u, item = wid * w.lanes + lane;
+    if (lane >= w.lanes || item >= w.count) return;
+    const uint32_t id = w.first + item;
+    const EncPartPos P = enc_part(A, id, w.chain);
+    const unsigned long long col = w.rec + (unsigned long long)wid * A.recs * w.lanes + lane;
+    uint4 *out = A.rec + col;
+    uint32_t x, esc = 0, bits = 0, span = 0;
+    if (P.is_top) {
+        const uint32_t k0 = __ldg(A.keys + P.first + 1);
+        x = EncTables::init(k0);
+        esc = (k0 & 0xFFu) == 0xFFu;
+    } else {
+        x = EXACT ? A.entry[id] : EncTables::init(__ldg(A.keys + P.first + 1));
+    }
+    walk_records(A.keys, P.first, P.a, x, [&](long long i, const uint4 &r, uint32_t n, const uint4 &v, bool whole) {
+        *out = r;
+        out += w.lanes;
+        bits += n;
+        span += n;
+        if (whole) {
+            esc += escapes_of(v);
+        } else {
+            long long j = i;  // the codes of the vector's span inside the part
+            do esc += (__ldg(A.keys + j) & 0xFFu) == 0xFFu;
+            while ((++j & 7) != 0 && j <= P.first);
+        }
+        if (((uint32_t)i & 63u) == 0) {
+            A.kept[i >> kKeptShift] = (uint16_t)x;
+            A.kept_bits[i >> kKeptShift] = (uint16_t)span;
+            span = 0;
+        }
+        return false;
+    });
+    if (P.p == 0) {  // the final state, then the end mark
+        A.rec[col + (unsigned long long)(A.recs - 1) * w.lanes] = make_record((x - O1_M) | (1u << O1_PB), 0, O1_PB + 1);
+        bits += O1_PB + 1;
+    }
+    A.exit1[id] = (uint16_t)x;
+    A.bits[id] = bits;
+    A.esc[id] = esc;
+    A.column[id] = col | ((unsigned long long)w.lanes << 56);
+    if (EXACT || P.is_top) A.exit2[id] = (uint16_t)x;  // nothing to repair
+}
+
+// Runs a part again from entering state x until its state meets a kept one, writing records and kept
+// states over.  Returns whether it met; `bits` is kept up to date.
+__device__ __forceinline__ bool rerun_part(const EncArgs &A, const EncPartPos &P, uint32_t &x,
+                                           unsigned long long column, uint32_t &bits, uint32_t &steps) {
+    const uint32_t lanes = (uint32_t)(column >> 56);
+    uint4 *const rec = A.rec + (column & ((1ULL << 56) - 1)), *out = rec;
+    uint32_t fresh = 0, stale = 0, span = 0;
+    // the state kept at the next 64th index below, loaded one kept index ahead
+    long long ki = P.first & ~63LL;
+    uint32_t kx = ki >= P.a ? A.kept[ki >> kKeptShift] : 0u, kb = ki >= P.a ? A.kept_bits[ki >> kKeptShift] : 0u;
+    const bool met = walk_records(A.keys, P.first, P.a, x, [&](long long i, const uint4 &r, uint32_t n, const uint4 &, bool) {
+        *out = r;
+        out += lanes;
+        fresh += n;
+        span += n;
+        if (i != ki) return false;
+        stale += kb;
+        A.kept_bits[i >> kKeptShift] = (uint16_t)span;
+        span = 0;
+        steps += 64;
+        if (kx == x) return true;
+        A.kept[i >> kKeptShift] = (uint16_t)x;
+        ki -= 64;
+        if (ki >= P.a) {
+            kx = A.kept[ki >> kKeptShift];
+            kb = A.kept_bits[ki >> kKeptShift];
+        }
+        return false;
+    });
+    if (met) {
+        bits += fresh - stale;
+    } else {
+        bits = fresh;
+        if (P.p == 0) {
+            rec[(unsigned long long)(A.recs - 1) * lanes] = make_record((x - O1_M) | (1u << O1_PB), 0, O1_PB + 1);
+            bits += O1_PB + 1;
         }
     }
+    return met;
+}
+
+__global__ void __launch_bounds__(kEncThreads) k_o1_repair(const EncArgs A) {
+    extern __shared__ uint4 smem_raw[];
+    const EncCta w = A.ctas[blockIdx.x];
+    load_image(smem_raw, A.image, w.table);
+    __syncthreads();
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u, item = wid * w.lanes + lane;
+    uint32_t steps = 0, unmet = 0;
+    if (lane < w.lanes && item < w.count) {
+            const uint32_t id = w.first + item;
+        const EncPartPos P = enc_part(A, id, w.chain);
+        if (!P.is_top) {
+            uint32_t x = A.exit1[id + 1], bits = A.bits[id];
+            const bool met = rerun_part(A, P, x, A.column[id], bits, steps);
+            const uint32_t ex1 = A.exit1[id];
+            A.entry[id] = A.exit1[id + 1];
+            A.exit2[id] = (uint16_t)(met ? ex1 : x);
+            A.bits[id] = bits;
+            unmet = !met && x != ex1;
+        }
+    }
+    steps = __reduce_add_sync(0xffffffffu, steps);
+    unmet = __reduce_add_sync(0xffffffffu, unmet);
+    if (lane == 0 && steps) atomicAdd(A.err + 2, (int)steps);
+    if (lane == 0 && unmet) atomicAdd(A.err + 5, (int)unmet);
+}
+
+// ---- the map path
+// Where codes take a few bits each (smooth fields at loose bounds), a step changes the distance of two
+// states by little more than a rounding, so runs from different states meet only after thousands to
+// millions of codes, and the exact states would have to pass down a chain part by part (249 rounds,
+// 36 ms, for 1800 x 3600 points at 1.4 bits a code).  Instead every run of parts (a super part) is
+// coded from all 8192 entering states at once, as the map from its entering to its leaving state:
+//   k_o1_maps     W warps a super part (four where the SMs hold few of them).  A step keeps the cyclic order of the states (within a
+//                 symbol the next state grows with the state), so states that have become equal are
+//                 neighbours: after 8, 16, 32 .. 512 codes and at every part end, neighbours that are equal
+//                 are merged into one class (about 8192 / (s sqrt(n)) classes are left after n codes,
+//                 with s the rounding of a step).  Every merge stores the map from the classes
+//                 before it to those after, and the classes' states.
+//   k_o1_compose  a CTA a chain: one thread follows the exact state from super part to super part
+//                 (two lookups each), then a thread per super part follows its entering state through
+//                 the merges to the entering state of every part.
+// and k_o1_walk<true> then codes every part from its exact state.  All lanes of a super part code the
+// same key, so a step is one conflicting shared-memory lookup a state.  A super part whose maps do
+// not fit its scratch (long runs of nearly certain codes merge nothing) is walked through by the
+// composing thread.
+constexpr uint32_t kMaxSuper = 32;                    // parts per super part, at most
+constexpr uint32_t kMapHdr = 4 + 2 * (7 + kMaxSuper);  // words of a super part's header
+struct MapArgs {
+    const uint32_t *sstart;  // first super part of every chain, then their number
+    uint32_t spp;            // parts per super part
+    uint32_t cap;            // 16-bit words of a super part's scratch
+    uint16_t *scratch;
+    uint32_t *hdr;           // [0] usable, [1] merges, [2] those before the first part end, [3] place of the
+                             // composed map; then per merge the places of its map and its states
+    const EncCta *ctas;      // super parts per CTA
+};
+
+// The barrier of a super part's W warps.
+template <int W>
+__device__ __forceinline__ void map_sync(unsigned bar) {
+    __syncwarp();
+    if (W > 1) asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * W) : "memory");
+}
+
+// Runs states src[j] for j < n through the codes from i down to e, states tid, tid + T, .. by thread tid of
+// T; dst[j] = the state after.  Warps without a state do nothing.
+template <int T, int R>
+__device__ __forceinline__ void map_run(const uint16_t *keys, long long i, long long e,
+                                        const uint16_t *src, uint16_t *dst, uint32_t n, uint32_t tid) {
+    if ((tid & ~31u) >= n) return;
+    uint32_t X[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const uint32_t j = tid + T * r;
+        X[r] = j < n ? (uint32_t)__ldcg(src + j) : (uint32_t)O1_M;
+    }
+    auto step = [&](const uint2 &en) {
+        uint32_t v, nb;
+#pragma unroll
+        for (int r = 0; r < R; r++) X[r] = EncTables::next(X[r], en, v, nb);
+    };
+    auto one = [&](long long j) { step(EncTables::transform(__ldg(keys + j))); };
+    for (; i >= e && (i & 7) != 7; i--) one(i);
+    if (i - 7 >= e) {
+        const uint4 *kv = reinterpret_cast<const uint4 *>(keys);
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        auto load = [&](long long j) { return j >= e ? __ldg(kv + (j >> 3)) : z; };
+        auto eight = [&](uint4 &v) {  // a ring of three vectors, as in walk_records
+            const uint32_t k[8] = {v.w >> 16, v.w & 0xFFFFu, v.z >> 16, v.z & 0xFFFFu,
+                                   v.y >> 16, v.y & 0xFFFFu, v.x >> 16, v.x & 0xFFFFu};
+            uint2 en[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) en[j] = EncTables::transform(k[j]);
+            v = load(i - 24);
+#pragma unroll
+            for (int j = 0; j < 8; j++) step(en[j]);
+            i -= 8;
+        };
+        uint4 v0 = load(i), v1 = load(i - 8), v2 = load(i - 16);
+        for (;;) {
+            eight(v0);
+            if (i - 7 < e) break;
+            eight(v1);
+            if (i - 7 < e) break;
+            eight(v2);
+            if (i - 7 < e) break;
+        }
+    }
+    for (; i >= e; i--) one(i);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const uint32_t j = tid + T * r;
+        if (j < n) __stcg(dst + j, (uint16_t)X[r]);
+    }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kEncThreads) k_o1_maps(const EncArgs A, const MapArgs M) {
+    extern __shared__ uint4 smem_raw[];
+    constexpr uint32_t T = 32 * W;
+    __shared__ uint32_t s_cnt[kEncThreads / 32];
+    if (!map_path(A)) return;
+    const EncCta w = M.ctas[blockIdx.x];
+    load_image(smem_raw, A.image, w.table);
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, tid = threadIdx.x % T, grp = threadIdx.x / T, wid = tid >> 5;
+    const unsigned bar = 1 + grp;
+    for (uint32_t it = grp; it < w.count; it += kEncThreads / T) {
+        const uint32_t sid = w.first + it;
+        uint32_t chain = w.chain, ch = A.nchains;
+        while (ch - chain > 1) {
+            const uint32_t mid = (chain + ch) >> 1;
+            if (__ldg(M.sstart + mid) <= sid) chain = mid;
+            else ch = mid;
+        }
+        const uint32_t nparts = __ldg(A.pstart + chain + 1) - __ldg(A.pstart + chain);
+        const uint32_t p0 = (sid - __ldg(M.sstart + chain)) * M.spp, p1 = min(p0 + M.spp, nparts);
+        const long long lo = (long long)A.chains[chain].lo, hi = (long long)A.chains[chain].hi;
+        const bool is_top = p1 == nparts;
+        uint16_t *ws = M.scratch + (size_t)sid * M.cap, *tmp = ws + M.cap - O1_M;
+        uint32_t *hd = M.hdr + (size_t)sid * kMapHdr;
+        const uint32_t room = M.cap - O1_M;
+        // the chain's top super part has one entering state, the exact initial one
+        uint32_t C = is_top ? 1u : (uint32_t)O1_M, at = 0, merges = 0, early = 0, C0 = 0;
+        const uint16_t *cur = nullptr;
+        if (is_top) {
+            if (tid == 0) __stcg(ws, (uint16_t)EncTables::init(__ldg(A.keys + hi - 1)));
+            cur = ws;
+            at = 1;
+            map_sync<W>(bar);
+        }
+        long long i = is_top ? hi - 2 : lo + (long long)p1 * A.part - 1;
+        const long long start = i;
+        uint32_t p = p1 - 1;  // the part being coded
+        bool ok = true;
+        for (;;) {
+            const long long bottom = lo + (long long)p * A.part;
+            long long e = bottom;
+            if (C > 1 && p + 1 == p1) {  // early merges within the first part
+                const long long done = start - i;
+                const long long t = done < 8 ? 8 : done < 512 ? 2 * done : 0;
+                if (t && start - t + 1 > bottom) e = start - t + 1;
+            }
+            for (uint32_t b = 0; b < C; b += 8 * T) {
+                const uint32_t n = min(C - b, 8u * T);
+                const uint16_t *src = cur ? cur + b : tmp + b;
+                if (!cur) {  // all states
+                    for (uint32_t j = tid; j < n; j += T) __stcg(tmp + b + j, (uint16_t)(O1_M + b + j));
+                    map_sync<W>(bar);
+                }
+                if (n <= T) map_run<T, 1>(A.keys, i, e, src, tmp + b, n, tid);
+                else if (n <= 2 * T) map_run<T, 2>(A.keys, i, e, src, tmp + b, n, tid);
+                else if (n <= 4 * T) map_run<T, 4>(A.keys, i, e, src, tmp + b, n, tid);
+                else map_run<T, 8>(A.keys, i, e, src, tmp + b, n, tid);
+            }
+            map_sync<W>(bar);
+            // merge equal neighbours: every warp takes a run of whole 32s
+            const uint32_t per = (C + T - 1) / T * 32, j0 = min(C, wid * per), j1 = min(C, j0 + per);
+            auto kept = [&](uint32_t j) {  // lanes whose state differs from the one before it
+                const uint32_t v = j + lane < j1 ? (uint32_t)__ldcg(tmp + j + lane) : 0u;
+                uint32_t prev = __shfl_up_sync(0xffffffffu, v, 1);
+                if (lane == 0) prev = j > 0 ? (uint32_t)__ldcg(tmp + j - 1) : 0u;  // 0 is no state
+                return make_uint2(__ballot_sync(0xffffffffu, j + lane < j1 && v != prev), v);
+            };
+            uint32_t idx = 0, Cn = 0;
+#pragma unroll 4
+            for (uint32_t j = j0; j < j1; j += 32) Cn += __popc(kept(j).x);
+            if (W > 1) {
+                if (lane == 0) s_cnt[threadIdx.x >> 5] = Cn;
+                map_sync<W>(bar);
+                Cn = 0;
+#pragma unroll
+                for (uint32_t v = 0; v < W; v++) {
+                    idx += v < wid ? s_cnt[grp * W + v] : 0u;
+                    Cn += s_cnt[grp * W + v];
+                }
+            }
+            const long long done = start - e + 1;
+            if (at + C + Cn > room || (done >= 64 && Cn > 2048) || (done >= 1024 && Cn > 1024)) {
+                ok = false;
+                break;
+            }
+            uint16_t *map = ws + at, *list = map + C;
+#pragma unroll 4
+            for (uint32_t j = j0; j < j1; j += 32) {
+                const uint2 k = kept(j);
+                const uint32_t me = idx + __popc(k.x & ((2u << lane) - 1u)) - 1u;  // class of this lane's state
+                if (j + lane < j1) {
+                    __stcg(map + j + lane, (uint16_t)me);
+                    if ((k.x >> lane) & 1u) __stcg(list + me, (uint16_t)k.y);
+                }
+                idx += __popc(k.x);
+            }
+            if (tid == 0) {
+                hd[4 + 2 * merges] = at;
+                hd[5 + 2 * merges] = at + C;
+            }
+            at += C + Cn;
+            if (merges == 0) C0 = Cn;
+            merges++;
+            C = Cn;
+            cur = list;
+            map_sync<W>(bar);
+            i = e - 1;
+            if (e > bottom) {
+                early++;
+                continue;
+            }
+            if (p == p0) break;
+            p--;
+        }
+        // the classes of the first merge, composed to the leaving state
+        if (ok && at + C0 > room) ok = false;
+        if (ok) {
+            constexpr uint32_t kAhead = 8;  // chains of lookups in flight per thread
+            for (uint32_t b = tid; b < C0; b += kAhead * T) {
+                uint32_t idx[kAhead];
+#pragma unroll
+                for (uint32_t u = 0; u < kAhead; u++) idx[u] = min(b + u * T, C0 - 1);
+                for (uint32_t m = 1; m < merges; m++) {
+                    const uint16_t *map = ws + hd[4 + 2 * m];
+#pragma unroll
+                    for (uint32_t u = 0; u < kAhead; u++) idx[u] = __ldcg(map + idx[u]);
+                }
+                const uint16_t *last = ws + hd[5 + 2 * (merges - 1)];
+#pragma unroll
+                for (uint32_t u = 0; u < kAhead; u++)
+                    if (b + u * T < C0) __stcg(ws + at + b + u * T, __ldcg(last + idx[u]));
+            }
+        }
+        if (tid == 0) {
+            hd[0] = ok;
+            hd[1] = merges;
+            hd[2] = early;
+            hd[3] = at;
+        }
+        map_sync<W>(bar);
+    }
+}
+
+constexpr int kComposeThreads = 256;
+__global__ void __launch_bounds__(kComposeThreads) k_o1_compose(const EncArgs A, const MapArgs M,
+                                                                const int *__restrict__ chain_table) {
+    extern __shared__ uint4 smem_raw[];
+    __shared__ uint16_t s_in[kEncThreads];  // entering state of every super part (at most one a part)
+    if (!map_path(A)) return;
+    const uint32_t chain = blockIdx.x, s0 = M.sstart[chain], ns = M.sstart[chain + 1] - s0;
+    if (ns == 0) return;
+    const uint32_t part0 = A.pstart[chain], nparts = A.pstart[chain + 1] - part0;
+    bool bad = false;
+    for (uint32_t s = threadIdx.x; s < ns; s += kComposeThreads) {
+        // places of its first and its composed map (where the tables go, unless they are needed)
+        const uint32_t *hd = M.hdr + (size_t)(s0 + s) * kMapHdr;
+        reinterpret_cast<uint2 *>(smem_raw)[s] = make_uint2(hd[4], hd[3]);
+        bad |= hd[0] == 0;
+    }
+    const bool walk = __syncthreads_or(bad);
+    static_assert(kEncThreads * sizeof(uint2) <= kEncSmem, "the places fit the tables' space");
+    if (walk) load_image(smem_raw, A.image, chain_table[chain]);
     __syncthreads();
     if (threadIdx.x == 0) {
-        int h0 = 0, h1 = 1;
-        if (s_tot[h1] > s_tot[h0]) h0 = 1, h1 = 0;
-        for (int c = 2; c < O1_NCTX; c++) {
-            if (s_tot[c] > s_tot[h0]) h1 = h0, h0 = c;
-            else if (s_tot[c] > s_tot[h1]) h1 = c;
+        const long long lo = (long long)A.chains[chain].lo, hi = (long long)A.chains[chain].hi;
+        uint32_t x = 0;
+        for (uint32_t s = ns; s-- > 0;) {
+            s_in[s] = (uint16_t)x;
+            const uint16_t *ws = M.scratch + (size_t)(s0 + s) * M.cap;
+            const bool is_top = s + 1 == ns;
+            const uint32_t *hd = M.hdr + (size_t)(s0 + s) * kMapHdr;
+            if (!walk || hd[0]) {
+                const uint2 m = walk ? make_uint2(hd[4], hd[3]) : reinterpret_cast<const uint2 *>(smem_raw)[s];
+                x = __ldcg(ws + m.y + __ldcg(ws + m.x + (is_top ? 0u : x - O1_M)));
+                continue;
+            }
+            const uint32_t p0 = s * M.spp, p1 = min(p0 + M.spp, nparts);
+            if (is_top) x = EncTables::init(__ldg(A.keys + hi - 1));
+            for (uint32_t p = p1; p-- > p0;) {
+                const long long a = lo + (long long)p * A.part;
+                const bool tp = p + 1 == nparts;
+                if (!tp) A.entry[part0 + p] = (uint16_t)x;
+                walk_states(A.keys, tp ? hi - 2 : a + (long long)A.part - 1, a, x);
+            }
         }
-        unsigned long long m = 0;
-        int slot = kSpecHot;
-        s_rev[0] = (uint8_t)h0;
-        s_rev[1] = (uint8_t)h1;
-        for (int c = 0; c < O1_NCTX; c++) {
-            const int sl = c == h0 ? 0 : c == h1 ? 1 : slot++;
-            m |= (unsigned long long)sl << (4 * c);
-            if (sl >= kSpecHot) s_rev[sl] = (uint8_t)c;
-        }
-        if (blockIdx.x == 0) meta[blockIdx.y].map = m;
     }
     __syncthreads();
-    uint32_t *img = image + (size_t)blockIdx.y * (kSpecSmem / 4);
-    uint32_t *hot2 = img;                                    // 16-bit tables, two entries per word
-    uint32_t *pk = img + kSpecHot * O1_M / 2;                // packed state tables
-    uint32_t *r_enc = pk + kSpecPackWords;                   // symbol transform per key
-    constexpr unsigned kHotWords = kSpecHot * O1_M / 2, kKeys = O1_NCTX * O1_NSYM;
-    constexpr unsigned kPacked = (O1_NCTX - kSpecHot) * O1_M;
-    const unsigned total = kHotWords + kSpecPackWords + kKeys;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        if (i < kHotWords) {
-            const unsigned e = 2 * i;  // entries e, e + 1 of the same context
-            const uint16_t *row = S + (size_t)s_rev[e / O1_M] * O1_M + (e % O1_M);
-            hot2[i] = (uint32_t)__ldg(row) | ((uint32_t)__ldg(row + 1) << 16);
-        } else if (i < kHotWords + kSpecPackWords) {
-            // word wd holds the bits [32 wd, 32 wd + 32) of the packed entries (entry j at bit 13 j;
-            // entry j is state u = j % 8192 of the context in slot kSpecHot + j / 8192)
-            const unsigned wd = i - kHotWords;
-            uint32_t v = 0;
-            const unsigned j0 = wd * 32 / O1_PB, j1 = min((wd * 32 + 31) / O1_PB, kPacked - 1);
-            uint32_t ev[4];  // a word spans at most 4 entries
-#pragma unroll
-            for (unsigned u = 0; u < 4; u++) {
-                const unsigned j = min(j0 + u, kPacked - 1);
-                ev[u] = (uint32_t)__ldg(S + (size_t)s_rev[kSpecHot + j / O1_M] * O1_M + (j % O1_M)) - O1_M;  // 13 bits
-            }
-#pragma unroll
-            for (unsigned u = 0; u < 4; u++) {
-                const unsigned j = j0 + u;
-                if (j > j1 || j >= kPacked) break;
-                const int sh = (int)(j * O1_PB) - (int)(wd * 32);
-                v |= sh >= 0 ? ev[u] << sh : ev[u] >> -sh;
-            }
-            pk[wd] = v;
-        } else {
-            const unsigned k = i - kHotWords - kSpecPackWords;
-            r_enc[k] = enc_word(stt[tb * O1_NSYM + k]);
+    for (uint32_t s = threadIdx.x; s < ns; s += kComposeThreads) {
+        const uint32_t *hd = M.hdr + (size_t)(s0 + s) * kMapHdr;
+        if (!hd[0]) continue;
+        const uint16_t *ws = M.scratch + (size_t)(s0 + s) * M.cap;
+        const uint32_t p1 = min((s + 1) * M.spp, nparts), early = hd[2], merges = hd[1];
+        uint32_t p = p1 - 1;
+        A.entry[part0 + p] = s_in[s];
+        uint32_t idx = s + 1 == ns ? 0u : (uint32_t)s_in[s] - O1_M;
+        for (uint32_t m = 0; m + 1 < merges; m++) {
+            idx = __ldcg(ws + hd[4 + 2 * m] + idx);
+            if (m >= early) A.entry[part0 + --p] = __ldcg(ws + hd[5 + 2 * m] + idx);
         }
     }
 }
 
-__global__ void __launch_bounds__(kSpecThreads) k_o1_encode_spec(
-    const uint16_t *__restrict__ keys, const SegInfo *__restrict__ segs, const SpecCta *__restrict__ ctas,
-    const uint32_t *__restrict__ image, const SpecMeta *__restrict__ meta,
-    uint16_t *__restrict__ sparse,
-    uint16_t *__restrict__ sparse_bits, uint32_t *__restrict__ stage, uint32_t *__restrict__ rstage,
-    uint8_t *__restrict__ slots, const unsigned long long *__restrict__ slot_off,
-    unsigned long long *__restrict__ blen, uint32_t part, O1Ckpt *__restrict__ cks,
-    const unsigned long long *__restrict__ ck_off, uint32_t ck_every, int *__restrict__ err) {
+// Rounds over the parts of this CTA's chain (one a thread, at most): a part runs again while the exit
+// state of the part above is not the state it was last run from.  Returns whether all are settled after
+// `limit` rounds; s_exit holds the exit states.
+__device__ __forceinline__ bool repair_rounds(const EncArgs &A, uint32_t chain, int table, uint32_t limit,
+                                              uint16_t *s_exit) {
     extern __shared__ uint4 smem_raw[];
-    uint16_t *hot = reinterpret_cast<uint16_t *>(smem_raw);           // kSpecHot 16-bit tables
-    uint32_t *pk = reinterpret_cast<uint32_t *>(hot + kSpecHot * O1_M);  // packed state tables
-    uint32_t *r_enc = pk + kSpecPackWords;                              // symbol transform per key
-    // after the walks, the transforms' space holds the parts' bit and escape counts
-    uint16_t *s_bits = reinterpret_cast<uint16_t *>(r_enc), *s_esc = s_bits + kSpecThreads;
-    __shared__ uint16_t s_exit[kSpecThreads + 1];
-    __shared__ uint8_t s_chg[kSpecThreads + 1];
-    const SpecCta w = ctas[blockIdx.x];
-    const unsigned long long smap = meta[w.table].map;  // table slot of every context (4 bits each)
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(image + (size_t)w.table * (kSpecSmem / 4));
-        for (unsigned i = threadIdx.x; i < kSpecSmem / 16; i += blockDim.x) smem_raw[i] = __ldg(src + i);
-    }
-    const int t = threadIdx.x;
-    const int ci = t / w.ppc, p = t % w.ppc;
-    const int chain = w.first + ci;
-    long long lo = 0, hi = 0;
-    if (ci < w.count) {
-        const int g = chain / kMaxK, k = chain % kMaxK;
-        const SegInfo sg = segs[g];
-        if (k < sg.K) {
-            lo = (long long)(sg.lo + (unsigned long long)k * sg.cs);
-            hi = min(lo + (long long)sg.cs, (long long)(sg.lo + sg.n));
-        }
-        if (p == 0 && hi <= lo) blen[chain] = 0;
-    }
-    const int nparts = hi > lo ? (int)((hi - lo + part - 1) / part) : 0;
-    const bool active = ci < w.count && p < nparts;
-    const bool is_top = active && p == nparts - 1;
-    const long long a = lo + (long long)p * part;
-    const long long top = active ? min(a + (long long)part, hi) - 1 : 0;
-    s_chg[t] = 0;
-    s_exit[t] = 0;
-    if (t == 0) {
-        s_chg[kSpecThreads] = 0;
-        s_exit[kSpecThreads] = 0;
-    }
+    constexpr uint32_t kChanged = 0x8000u;  // bit 15 of an exit state: changed in the last round
+    const uint32_t t = threadIdx.x, part0 = A.pstart[chain], nparts = A.pstart[chain + 1] - part0, id = part0 + t;
+    const bool active = t < nparts;
+    if (active) s_exit[t] = A.exit2[id];
     __syncthreads();
-    // a key's transform word and table slot
-    struct EncRec {
-        uint32_t e, slot;
-    };
-    auto rec_of = [&](uint32_t k) -> EncRec {
-        return EncRec{r_enc[k], (uint32_t)(smap >> (4 * (k >> 8))) & 15u};
-    };
-    auto nbits = [](uint32_t x, const EncRec r) -> uint32_t {
-        return (r.e >> 28) - ((x - (((r.e >> 14) & 0x3FFFu) + O1_M)) >> 31);
-    };
-    auto next_state = [&](uint32_t x, const EncRec r, uint32_t nb) -> uint32_t {
-        const uint32_t idx = (x >> nb) + (r.e & 0x3FFFu) - O1_M;  // within the context's table
-        if (r.slot < (uint32_t)kSpecHot) return hot[(r.slot << O1_PB) + idx];
-        const uint32_t bit = (((r.slot - kSpecHot) << O1_PB) + idx) * O1_PB;
-        const uint32_t wd = bit >> 5;
-        return O1_M + (__funnelshift_r(pk[wd], pk[wd + 1], bit & 31u) & (O1_M - 1));
-    };
-    auto init_state = [&](uint32_t k) -> uint32_t {
-        // FSE_initCState2: the state that codes symbol k with the fewest bits
-        const EncRec r = rec_of(k);
-        const uint32_t mbo = r.e >> 28, msp = ((r.e >> 14) & 0x3FFFu) + O1_M;
-        const uint32_t dnb = (mbo << 16) - msp;
-        const uint32_t nb = (dnb + (1u << 15)) >> 16;
-        return next_state((nb << 16) - dnb, r, nb);
-    };
-    // the first code of a chain has context 0, so index lo is coded apart from the walks
-    const long long istart = is_top ? hi - 2 : top;
-    const long long bottom = p == 0 ? a + 1 : a;
-    const uint32_t k_lo = p == 0 && active ? ((uint32_t)__ldg(keys + lo) & 0xFFu) : 0u;
-    // Bit writer into a part's staging words (LSB first, as the stream).  The CTA's staging areas
-    // are interleaved (word j of thread t at j * kSpecThreads + t), so that the placement step's
-    // reads of the same word j by a warp share cache lines.
-    struct Stager {
-        uint32_t *w;
-        uint64_t acc = 0;
-        uint32_t accn = 0, nw = 0, bits = 0;
-        __device__ void put(uint32_t v, uint32_t nb) {
-            acc |= (uint64_t)(v & ((1u << nb) - 1u)) << accn;
-            accn += nb;
-            bits += nb;
-            if (accn >= 32) {
-                w[(size_t)(nw++) * kSpecThreads] = (uint32_t)acc;
-                acc >>= 32;
-                accn -= 32;
-            }
-        }
-        __device__ void flush() {
-            if (accn > 0) w[(size_t)nw * kSpecThreads] = (uint32_t)acc;
-        }
-    };
-    const size_t stw = spec_stage_words(part);
-    uint32_t *sw = stage + (size_t)blockIdx.x * kSpecThreads * stw + t;   // speculative bits
-    uint32_t *rw = rstage + (size_t)blockIdx.x * kSpecThreads * stw + t;  // repaired bits
-    // 1. speculative pass: walk and emit from the guessed state, keeping the state and the bit
-    //    count after every 64th index
-    uint32_t esc = 0, spec_bits = 0, spec_exit = 0;
+    bool need = t + 1 < nparts && s_exit[t + 1] != A.entry[id];
+    if (!__syncthreads_or(need)) return true;
+    load_image(smem_raw, A.image, table);
+    __syncthreads();
+    EncPartPos P{};
+    uint32_t bits = 0, steps = 0;
     if (active) {
-        Stager sg{sw};
-        uint32_t x;
-        if (is_top) {
-            const uint32_t k0 = hi - 1 == lo ? k_lo : (uint32_t)__ldg(keys + hi - 1);
-            x = init_state(k0);
-            esc += (k0 & 0xFFu) == 0xFFu;
-            if (((hi - 1) & 63) == 0) {
-                sparse[(hi - 1) >> 6] = (uint16_t)x;
-                sparse_bits[(hi - 1) >> 6] = 0;
-            }
-        } else {
-            x = init_state((uint32_t)__ldg(keys + top + 1));
-        }
-        auto step = [&](long long i, uint32_t k) {
-            const EncRec r = rec_of(k);
-            const uint32_t nb = nbits(x, r);
-            sg.put(x, nb);
-            x = next_state(x, r, nb);
-            esc += (k & 0xFFu) == 0xFFu;
-            if (((uint32_t)i & 63u) == 0) {
-                sparse[i >> 6] = (uint16_t)x;
-                sparse_bits[i >> 6] = (uint16_t)sg.bits;
-            }
-        };
-        walk_keys(keys, istart, bottom, step);
-        if (p == 0 && istart >= lo) step(lo, k_lo);
-        if (p == 0) {
-            sg.put(x & (O1_M - 1), O1_PB);  // the final state, then the end mark
-            sg.put(1u, 1u);
-        }
-        sg.flush();
-        spec_bits = sg.bits;
-        spec_exit = x;
-        s_exit[t] = (uint16_t)x;
+        P = enc_part(A, id, chain);
+        bits = A.bits[id];
     }
-    // every part's speculative exit state is read by the part below it, which may be in another warp
-    __syncthreads();
-    // 2. repair rounds (err[2] counts the re-run codes, err[3] the rounds, for diagnostics): a part
-    //    whose entering state changed walks again from it, emitting into its repair staging, until
-    //    its state meets a kept one at index m; its bits are then the repaired bits of the codes
-    //    above m followed by the speculative bits from m on.  A part that never meets has all its
-    //    bits in the repair staging and a new exit state, so the part below repairs again.
-    bool need = active && !is_top;
-    uint32_t repaired = 0;
-    int mode = 0;                    // 0 speculative bits, 1 met, 2 repaired whole
-    uint32_t rep_bits = 0, cut = 0;  // repaired bits; speculative bit where the suffix starts
-    for (int round = 0;; round++) {
-        if (round > nparts + 2 && need) atomicExch(err, 5);
-        if (t == 0) atomicMax(err + 3, round);
-        const uint32_t E = need ? s_exit[t + 1] : 0u;
-        // an entering state outside the table would index outside the shared tables: refuse it
-        const bool valid = E >= (uint32_t)O1_M && E < 2u * O1_M;
-        if (need && !valid) atomicExch(err, 6);
+    bool settled = false;
+    for (uint32_t round = 1; round <= limit && !settled; round++) {
+        uint32_t x = need ? s_exit[t + 1] & (kChanged - 1u) : 0u;
         __syncthreads();
-        bool changed = false;
-        if (need && valid && round <= nparts + 2) {
-            Stager rg{rw};
-            uint32_t x = E;
-            // the kept state of the next 64th index below, loaded one kept index ahead
-            long long ck_i = top & ~63LL;
-            uint32_t ck_x = ck_i >= a ? sparse[ck_i >> 6] : 0u;
-            auto rstep = [&](long long i, uint32_t k) -> bool {
-                const EncRec r = rec_of(k);
-                const uint32_t nb = nbits(x, r);
-                rg.put(x, nb);
-                x = next_state(x, r, nb);
-                repaired++;
-                if (i != ck_i) return false;
-                if (ck_x == x) {
-                    cut = sparse_bits[i >> 6];
-                    return true;
-                }
-                ck_i -= 64;
-                ck_x = ck_i >= a ? sparse[ck_i >> 6] : 0u;
-                return false;
-            };
-            // index lo (a chain's first code, context 0) is coded apart from the walk
-            bool met = walk_keys_until(keys, top, p == 0 ? a + 1 : a, rstep);
-            if (!met && p == 0) met = rstep(lo, k_lo);
-            if (!met && p == 0) {
-                rg.put(x & (O1_M - 1), O1_PB);
-                rg.put(1u, 1u);
+        if (active) {
+            uint32_t ex = s_exit[t] & (kChanged - 1u);
+            if (need) {
+                // a run that meets the kept states leaves as the run before it did
+                A.entry[id] = (uint16_t)x;
+                if (!rerun_part(A, P, x, A.column[id], bits, steps) && x != ex) ex = x | kChanged;
             }
-            rg.flush();
-            rep_bits = rg.bits;
-            // the exit state: the speculative run's once met, else this run's
-            const uint32_t ex = met ? spec_exit : x;
-            mode = met ? 1 : 2;
-            changed = ex != s_exit[t];
             s_exit[t] = (uint16_t)ex;
         }
-        s_chg[t] = changed;
+        if (t == 0) atomicMax(A.err + 3, (int)round);
         __syncthreads();
-        need = active && !is_top && s_chg[t + 1] != 0;
-        if (!__syncthreads_or(need)) break;
+        need = t + 1 < nparts && (s_exit[t + 1] & kChanged);
+        settled = !__syncthreads_or(need);
     }
-    if (repaired) atomicAdd(err + 2, (int)repaired);
-    // the part's bits: [rw bits 0, rep_bits) then [sw bits cut, spec_bits)
-    const uint32_t bits = mode == 0 ? spec_bits : mode == 1 ? rep_bits + (spec_bits - cut) : rep_bits;
-    // 4. offsets (the top part's bits come first), escapes below each part, placement
-    __syncthreads();  // the symbol transforms' space is reused for the counts
-    s_bits[t] = active ? (uint16_t)bits : (uint16_t)0;
-    s_esc[t] = active ? (uint16_t)esc : (uint16_t)0;
-    __syncthreads();
-    uint32_t off = 0, esc_below = 0;
     if (active) {
-        for (int q = p + 1; q < nparts; q++) off += s_bits[t - p + q];
-        for (int q = 0; q < p; q++) esc_below += s_esc[t - p + q];
+        s_exit[t] &= kChanged - 1u;
+        A.exit2[id] = s_exit[t];
+        A.bits[id] = bits;
     }
-    uint32_t *ow = active ? reinterpret_cast<uint32_t *>(slots + slot_off[chain]) : nullptr;
-    if (active) ow[off >> 5] = 0u;  // the first word may be shared with the part above: zeroed, then OR-ed
+    if (steps) atomicAdd(A.err + 2, (int)steps);
     __syncthreads();
-    if (active) {
-        // Output words [w0, wend).  Word w0 was zeroed by this part; the last word, when the part
-        // ends inside it and a part follows, is the next part's first word (zeroed by it).  Both are
-        // merged with atomicOr, every other word is this part's alone.
-        const uint32_t w0 = off >> 5, wend = (off + bits + 31) >> 5;
-        const uint32_t shared_last = (p > 0 && ((off + bits) & 31u)) ? wend - 1 : 0xFFFFFFFFu;
-        uint32_t wi = w0;
-        auto store = [&](uint32_t v) {
-            if (wi == w0 || wi == shared_last) atomicOr(ow + wi, v);
-            else ow[wi] = v;
-            wi++;
-        };
-        uint64_t acc = 0;
-        uint32_t accn = off & 31u;
-        // appends bits [b0, b1) of staging words src, loading kBatch + 1 staging words (those
-        // inside the part's staging column) before placing kBatch words
-        constexpr uint32_t kBatch = 8;
-        auto append = [&](const uint32_t *src, uint32_t b0, uint32_t b1) {
-            const uint32_t sh = b0 & 31u;
-            for (uint32_t bp = b0; bp < b1; bp += 32 * kBatch) {
-                const uint32_t j0 = bp >> 5;
-                uint32_t wv[kBatch + 1];
-#pragma unroll
-                for (uint32_t u = 0; u <= kBatch; u++)
-                    wv[u] = j0 + u < (uint32_t)stw ? src[(size_t)(j0 + u) * kSpecThreads] : 0u;
-#pragma unroll
-                for (uint32_t u = 0; u < kBatch; u++) {
-                    const uint32_t q = bp + 32 * u;
-                    if (q >= b1) break;
-                    const uint32_t n = min(32u, b1 - q);
-                    uint32_t v = sh ? __funnelshift_r(wv[u], wv[u + 1], sh) : wv[u];
-                    if (n < 32) v &= (1u << n) - 1u;
-                    acc |= (uint64_t)v << accn;
-                    accn += n;
-                    if (accn >= 32) {
-                        store((uint32_t)acc);
-                        acc >>= 32;
-                        accn -= 32;
-                    }
-                }
-            }
-        };
-        if (mode != 0) append(rw, 0, rep_bits);
-        if (mode != 2) append(sw, mode == 1 ? cut : 0u, spec_bits);
-        if (accn > 0) store((uint32_t)acc);
-        if (p == 0) blen[chain] = ((unsigned long long)off + bits + 7) / 8;
-        // 5. decode checkpoint at every ck_every-th part start: the state the decoder holds
-        // before index a
-        if (p > 0 && cks && (uint32_t)p % ck_every == 0)
-            cks[ck_off[chain] + (uint32_t)p / ck_every - 1] = O1Ckpt{off + bits, esc_below, (uint16_t)(s_exit[t] & (O1_M - 1)),
-                                                (uint16_t)(__ldg(keys + a) >> 8)};
+    return settled;
+}
+
+__global__ void __launch_bounds__(kEncThreads) k_o1_rounds(const EncArgs A, const int *__restrict__ chain_table) {
+    __shared__ uint16_t s_exit[kEncThreads];
+    if (many_unmet(A) || A.pstart[blockIdx.x + 1] == A.pstart[blockIdx.x]) return;
+    if (!repair_rounds(A, blockIdx.x, chain_table[blockIdx.x], kMaxRounds, s_exit) && threadIdx.x == 0)
+        atomicAdd(A.err + 6, 1);
+}
+
+// A CTA per chain: every part's bit offset (the top part's bits come first), the decode checkpoints, and
+// zeros in the words that k_o1_place merges.  (The rounds in front find nothing left to do.)
+__global__ void __launch_bounds__(kEncThreads) k_o1_settle(const EncArgs A, const int *__restrict__ chain_table,
+                                                          uint8_t *__restrict__ slots,
+                                                          const unsigned long long *__restrict__ slot_off,
+                                                          unsigned long long *__restrict__ blen,
+                                                          O1Ckpt *__restrict__ cks,
+                                                          const unsigned long long *__restrict__ ck_off,
+                                                          uint32_t ck_every) {
+    extern __shared__ uint4 smem_raw[];
+    __shared__ uint16_t s_exit[kEncThreads];
+    const uint32_t chain = blockIdx.x, t = threadIdx.x, part0 = A.pstart[chain];
+    const uint32_t nparts = A.pstart[chain + 1] - part0;  // at most one a thread
+    if (nparts == 0) {
+        if (t == 0) blen[chain] = 0;
+        return;
     }
+    if (!repair_rounds(A, chain, chain_table[chain], nparts + 2, s_exit) && t == 0) atomicExch(A.err, 5);
+    const bool active = t < nparts;
+    const uint32_t id = part0 + t;
+    EncPartPos P{};
+    uint32_t bits = 0, esc = 0;
+    if (active) {
+        P = enc_part(A, id, chain);
+        bits = A.bits[id];
+        esc = A.esc[id];
+    }
+    uint32_t *s_sum = reinterpret_cast<uint32_t *>(smem_raw);  // the tables are done with
+    uint32_t total, esc_total;
+    __syncthreads();
+    const uint32_t below = block_excl_scan<uint32_t>(active ? bits : 0u, s_sum, total);
+    const uint32_t esc_below = block_excl_scan<uint32_t>(active ? esc : 0u, s_sum + 32, esc_total);
+    if (!active) return;
+    const uint32_t off = total - below - bits;
+    uint32_t *ow = reinterpret_cast<uint32_t *>(slots + slot_off[chain]);
+    ow[off >> 5] = 0u;
+    if (t == 0) {
+        ow[total >> 5] = 0u;
+        blen[chain] = ((unsigned long long)total + 7) / 8;
+    }
+    A.at[id] = slot_off[chain] * 8 + off;
+    A.nrec[id] = (P.first < P.a ? 0u : (uint32_t)((P.first >> 3) - (P.a >> 3)) + 1u) | (t == 0 ? 0x80000000u : 0u);
+    // decode checkpoint at every ck_every-th part start: the state the decoder holds before index a
+    if (t > 0 && cks && t % ck_every == 0)
+        cks[ck_off[chain] + t / ck_every - 1] =
+            O1Ckpt{off + bits, esc_below, (uint16_t)(s_exit[t] - O1_M), (uint16_t)(__ldg(A.keys + P.a) >> 8)};
+}
+
+// Joins the parts' records in the slots, a warp per part and a record per lane: a warp scan of the bit
+// counts gives every record its bit offset, the bits are merged in shared memory, and whole words leave
+// coalesced; the part's first and last word, shared with its neighbours, by atomicOr (k_o1_settle zeroed
+// them).  142 us for the 141 MB of a 512^3 field (2.9 TB/s with the records): bound by the issue of the
+// merges.
+constexpr int kPlaceWarps = 8;
+constexpr uint32_t kPlaceWords = 32 * 104 / 32 + 2;  // 32 records, the word in front, one behind
+__global__ void __launch_bounds__(kPlaceWarps * 32) k_o1_place(const EncArgs A, uint32_t *__restrict__ slots) {
+    __shared__ uint32_t s_buf[kPlaceWarps][kPlaceWords];
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u, id = blockIdx.x * kPlaceWarps + wid;
+    if (id >= __ldg(A.pstart + A.nchains)) return;
+    uint32_t *buf = s_buf[wid];
+    const unsigned long long column = A.column[id], at = A.at[id];
+    const uint32_t lanes = (uint32_t)(column >> 56), nr = A.nrec[id] & 0x7FFFFFFFu, nrec = nr + (A.nrec[id] >> 31);
+    const uint4 *rec = A.rec + (column & ((1ULL << 56) - 1));
+    uint32_t *o = slots + (at >> 5);
+    uint32_t pos = (uint32_t)(at & 31u);  // bits in front of the next record in the words from o on
+    bool shared_first = true;
+    for (uint32_t z = lane; z < kPlaceWords; z += 32) buf[z] = 0u;
+    auto load = [&](uint32_t r) -> uint4 {
+        const uint32_t q = r < nr ? r : A.recs - 1;  // the final state's record comes last
+        return r < nrec ? __ldcg(rec + (unsigned long long)q * lanes) : make_uint4(0, 0, 0, 0);
+    };
+    uint4 v = load(lane);
+    __syncwarp();
+    for (uint32_t r0 = 0; r0 < nrec; r0 += 32) {
+        const uint4 nxt = load(r0 + 32 + lane);
+        const uint32_t n = v.w >> 24, incl = warp_incl_scan(n), p = pos + incl - n;
+        if (n) {
+            const uint32_t w = p >> 5, sh = p & 31u, top = v.w & 0x00FFFFFFu, end = sh + n;
+            atomicOr(buf + w, v.x << sh);
+            if (end > 32) atomicOr(buf + w + 1, __funnelshift_l(v.x, v.y, sh));
+            if (end > 64) atomicOr(buf + w + 2, __funnelshift_l(v.y, v.z, sh));
+            if (end > 96) atomicOr(buf + w + 3, __funnelshift_l(v.z, top, sh));
+            if (end > 128) atomicOr(buf + w + 4, __funnelshift_l(top, 0u, sh));
+        }
+        const uint32_t tot = pos + __shfl_sync(0xffffffffu, incl, 31), full = tot >> 5;
+        __syncwarp();
+        for (uint32_t z = lane; z < full; z += 32) {
+            if (z == 0 && shared_first) atomicOr(o, buf[0]);
+            else o[z] = buf[z];
+        }
+        __syncwarp();
+        const uint32_t rest = buf[full];
+        __syncwarp();
+        for (uint32_t z = lane; z <= full; z += 32) buf[z] = 0u;
+        __syncwarp();
+        if (lane == 0) buf[0] = rest;
+        __syncwarp();
+        shared_first = shared_first && full == 0;
+        o += full;
+        pos = tot & 31u;
+        v = nxt;
+    }
+    if (lane == 0 && pos) atomicOr(o, buf[0]);
 }
 
 // A decode table entry of a context not resident in shared memory (kept out of line so that the
@@ -2618,9 +2986,127 @@ void enable_big_smem() {
                                   kDecSlots * O1_M * 4));
     FB2_CUDA(cudaFuncSetAttribute(k_o1_decode_parts, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kDecSlots * O1_M * 4));
-    FB2_CUDA(cudaFuncSetAttribute(k_o1_encode_spec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpecSmem));
+    for (const void *k : {(const void *)k_o1_walk<false>, (const void *)k_o1_walk<true>, (const void *)k_o1_repair,
+                          (const void *)k_o1_maps<1>,
+                          (const void *)k_o1_maps<4>, (const void *)k_o1_compose, (const void *)k_o1_rounds, (const void *)k_o1_settle})
+        FB2_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEncSmem));
     FB2_CUDA(cudaFuncSetAttribute(k_o1_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHistSmem));
     done.fetch_or(bit, std::memory_order_acq_rel);
+}
+
+// The parts of every chain and the CTAs that code them.
+struct ChainParts {
+    std::vector<EncChain> chains;   // kMaxK a segment
+    std::vector<int> table;         // table set of every chain
+    std::vector<uint32_t> pstart, sstart;  // first part and first super part of every chain
+    uint32_t spp = 1;               // parts per super part
+    std::vector<EncCta> ctas, map_ctas;
+    unsigned long long records = 0;
+};
+ChainParts chain_parts(const std::vector<SegInfo> &segs, const std::vector<int> &seg_region, int K, uint32_t part) {
+    ChainParts cp;
+    const size_t n = segs.size() * kMaxK;
+    cp.pstart.assign(n + 1, 0);
+    cp.sstart.assign(n + 1, 0);
+    for (size_t c = 0; c < n; c++) {
+        const SegInfo &sg = segs[c / kMaxK];
+        const unsigned long long k = c % kMaxK, lo = sg.lo + k * sg.cs;
+        const unsigned long long hi = k < (unsigned long long)K ? std::min(lo + sg.cs, sg.lo + sg.n) : lo;
+        cp.chains.push_back({lo, std::max(lo, hi)});
+        cp.table.push_back(seg_region[c / kMaxK]);
+        cp.pstart[c + 1] = cp.pstart[c] + (hi > lo ? (uint32_t)((hi - lo + part - 1) / part) : 0);
+    }
+    // super parts: about eight an SM (the states of a super part's first codes cost as much as its next
+    // 8 Ki codes), more where that would make them long
+    while (cp.spp < kMaxSuper && cp.pstart[n] / cp.spp > (uint32_t)(sm_count() * 8)) cp.spp *= 2;
+    for (size_t c = 0; c < n; c++)
+        cp.sstart[c + 1] = cp.sstart[c] + (cp.pstart[c + 1] - cp.pstart[c] + cp.spp - 1) / cp.spp;
+    int tables = 0;
+    for (int t : cp.table) tables = std::max(tables, t + 1);
+    const std::vector<unsigned long long> none((size_t)tables, 0);
+    auto ctas = [&](const std::vector<uint32_t> &start, size_t max_per) {
+        std::vector<ItemRun> runs = table_runs(cp.table);
+        for (auto &r : runs) r = ItemRun{start[r.first], start[r.first + r.len] - start[r.first], r.table};
+        runs.erase(std::remove_if(runs.begin(), runs.end(), [](const ItemRun &r) { return r.len == 0; }), runs.end());
+        std::vector<EncCta> out;
+        for (const ChainCta &c : run_ctas(runs, start[n], none, none, max_per)) {
+            EncCta e{c.table, (uint32_t)c.first, (uint32_t)c.count, 1, 0, 0};
+            e.chain = (uint32_t)(std::upper_bound(start.begin(), start.end(), e.first) - start.begin()) - 1;
+            out.push_back(e);
+        }
+        return out;
+    };
+    cp.ctas = ctas(cp.pstart, kEncThreads);
+    cp.map_ctas = ctas(cp.sstart, kEncThreads);
+    for (EncCta &e : cp.ctas) {
+        e.lanes = std::min(32u, (e.count + kEncWarps - 1) / kEncWarps);
+        e.rec = cp.records;
+        cp.records += (unsigned long long)((e.count + e.lanes - 1) / e.lanes) * e.lanes * part_records(part);
+    }
+    return cp;
+}
+
+void encode_chains(Pool &pool, const ChainParts &cp, const uint16_t *keys, size_t N, const uint32_t *image, uint32_t part,
+                   uint8_t *slots, const unsigned long long *d_soff, unsigned long long *blen, O1Ckpt *cks,
+                   const unsigned long long *d_ck_off, uint32_t ck_every, int *d_err, cudaStream_t st) {
+    const uint32_t nchains = (uint32_t)cp.chains.size(), nparts = cp.pstart.back(), nsuper = cp.sstart.back();
+    int *d_table = h2d(pool, cp.table, st);
+    EncArgs A{};
+    A.keys = keys;
+    A.chains = h2d(pool, cp.chains, st);
+    A.pstart = h2d(pool, cp.pstart, st);
+    A.nchains = nchains;
+    A.part = part;
+    A.recs = part_records(part);
+    A.image = image;
+    A.ctas = h2d(pool, cp.ctas, st);
+    uint16_t *p16 = pool.get<uint16_t>((size_t)nparts * 3);
+    A.exit1 = p16;
+    A.exit2 = p16 + nparts;
+    A.entry = p16 + 2 * (size_t)nparts;
+    uint32_t *p32 = pool.get<uint32_t>((size_t)nparts * 3);
+    A.bits = p32;
+    A.esc = p32 + nparts;
+    A.nrec = p32 + 2 * (size_t)nparts;
+    A.column = pool.get<unsigned long long>((size_t)nparts * 2);
+    A.at = A.column + nparts;
+    A.kept = pool.get<uint16_t>(2 * ((N >> kKeptShift) + 2));
+    A.kept_bits = A.kept + (N >> kKeptShift) + 2;
+    A.err = d_err;
+    // The maps' scratch takes the records' place: the map path writes them anew after its maps are used.
+    MapArgs M{};
+    M.sstart = h2d(pool, cp.sstart, st);
+    M.spp = cp.spp;
+    M.cap = (uint32_t)(O1_M + 28 * 1024 + 320 * cp.spp);
+    uint8_t *area = pool.get<uint8_t>(std::max((size_t)cp.records * sizeof(uint4), (size_t)nsuper * M.cap * 2));
+    A.rec = reinterpret_cast<uint4 *>(area);
+    M.scratch = reinterpret_cast<uint16_t *>(area);
+    M.hdr = pool.get<uint32_t>((size_t)nsuper * kMapHdr);
+    M.ctas = h2d(pool, cp.map_ctas, st);
+    enable_big_smem();
+    const unsigned nc = (unsigned)cp.ctas.size();
+    k_o1_walk<false><<<nc, kEncThreads, kEncSmem, st>>>(A);
+    FB2_CHECK_LAUNCH();
+    k_o1_repair<<<nc, kEncThreads, kEncSmem, st>>>(A);
+    FB2_CHECK_LAUNCH();
+    k_o1_rounds<<<nchains, kEncThreads, kEncSmem, st>>>(A, d_table);
+    FB2_CHECK_LAUNCH();
+    // a warp a super part where they fill the SMs' warps, four (the first codes' many states go faster)
+    // where not: 6.5 M codes take 850 us with four and 1265 with one, 134 M 11.7 and 3.9 ms
+    if (nsuper > (uint32_t)sm_count() * kEncThreads / 128)
+        k_o1_maps<1><<<(unsigned)cp.map_ctas.size(), kEncThreads, kEncSmem, st>>>(A, M);
+    else
+        k_o1_maps<4><<<(unsigned)cp.map_ctas.size(), kEncThreads, kEncSmem, st>>>(A, M);
+    FB2_CHECK_LAUNCH();
+    k_o1_compose<<<nchains, kComposeThreads, kEncSmem, st>>>(A, M, d_table);
+    FB2_CHECK_LAUNCH();
+    k_o1_walk<true><<<nc, kEncThreads, kEncSmem, st>>>(A);
+    FB2_CHECK_LAUNCH();
+    k_o1_settle<<<nchains, kEncThreads, kEncSmem, st>>>(A, d_table, slots, d_soff, blen, cks, d_ck_off, ck_every);
+    FB2_CHECK_LAUNCH();
+    k_o1_place<<<(nparts + kPlaceWarps - 1) / kPlaceWarps, kPlaceWarps * 32, 0, st>>>(
+        A, reinterpret_cast<uint32_t *>(slots));
+    FB2_CHECK_LAUNCH();
 }
 
 // Sum of the per-segment histograms of each table region (segments [rs[r], rs[r+1])).
@@ -2928,14 +3414,20 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
                               (unsigned long long)((ng + K - 1) / K), K, 0};
         }
         SegInfo *d_segs = h2d(pool, segs, st);
-        // encoder part size (also the decode checkpoint spacing): a chain's parts fit one CTA
+        // encoder part size, a power of two up to the decode checkpoint spacing: a chain's parts fit one
+        // CTA's threads, and a part is shorter than the spacing where the parts would not give every SM
+        // four full warps (a walk's time is then the length of a part: 67 us for 64^3 codes in parts of 1024, 26 us in parts of 256), but not so short
+        // that a run seldom meets the kept states within it
         unsigned long long max_cs = 1;
         for (const auto &sg : segs) max_cs = std::max<unsigned long long>(max_cs, sg.cs);
+        auto parts_of = [&](uint32_t part) { return (max_cs + part - 1) / part; };
         uint32_t enc_part = std::min<uint32_t>(cc.o1_part ? cc.o1_part : 1024u, 1024u);
-        while ((max_cs + enc_part - 1) / enc_part > (unsigned long long)kSpecThreads) enc_part *= 2;
+        while (parts_of(enc_part) > (unsigned long long)kEncThreads) enc_part *= 2;
         if (cc.o1_part && cc.o1_part < enc_part) cc.o1_part = enc_part;
+        while (enc_part > kMinEncPart && parts_of(enc_part / 2) <= (unsigned long long)kEncThreads &&
+               N / enc_part < (long long)sm_count() * 128)
+            enc_part /= 2;
         const uint32_t ck_every = cc.o1_part ? cc.o1_part / enc_part : 1u;
-        const int ppc = (int)((max_cs + enc_part - 1) / enc_part);
         // decode checkpoints of every chain: one before each index lo + q * part, q >= 1
         const long long nchains_all = S * kMaxK;
         std::vector<unsigned long long> ck_off(nchains_all + 1, 0);
@@ -3043,21 +3535,14 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         uint16_t *nf = pool.get<uint16_t>((size_t)ntab * O1_NSYM);
         k_o1_norm<<<(ntab + 7) / 8, 256, 0, st>>>(rhist, ntab, nf);
         FB2_CHECK_LAUNCH();
-        uint16_t *stab = pool.get<uint16_t>((size_t)ntab * O1_M);
-        fse::SymTT *stt = pool.get<fse::SymTT>((size_t)ntab * O1_NSYM);
-        uint8_t *spread = pool.get<uint8_t>((size_t)ntab * O1_M);
         int *d_err = pool.get<int>(8);
         FB2_CUDA(cudaMemsetAsync(d_err, 0, 32, st));
-        k_o1_ctable<<<ntab, kTabThreads, 0, st>>>(nf, stab, stt, spread, d_err);
-        FB2_CHECK_LAUNCH();
         // the chain encoder's shared-memory image of every table set
-        uint32_t *image = pool.get<uint32_t>((size_t)R * (kSpecSmem / 4));
-        SpecMeta *meta = pool.get<SpecMeta>((size_t)R);
-        {
-            const unsigned items = kSpecHot * O1_M / 2 + kSpecPackWords + O1_NCTX * O1_NSYM;
-            k_spec_image<<<dim3((items + 255) / 256, (unsigned)R), 256, 0, st>>>(stab, stt, rhist, image, meta);
-            FB2_CHECK_LAUNCH();
-        }
+        uint32_t *image = pool.get<uint32_t>((size_t)R * (kEncSmem / 4));
+        k_o1_ctable<<<ntab, kTabThreads, 0, st>>>(nf, image, d_err);
+        FB2_CHECK_LAUNCH();
+        const long long nchains = S * kMaxK;
+        const ChainParts cp = chain_parts(segs, seg_region, K, enc_part);
         // escapes in index order, on the second stream (the host waits here for their count; the
         // histogram pass and the table builds, launched above, run meanwhile)
         const std::vector<unsigned long long> gstart = d2h(d_gstart, (size_t)S + 1, es);
@@ -3073,12 +3558,11 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         // they take a few SMs of their own instead of waiting for the chain encoder's last wave
         const bool queue_first = fork && tune.queued_ev != nullptr;
         const GammaBlocks gblocks = gamma_launch(spool, evals, gstart, es, cc.fse_part,
-                                                 queue_first ? tune.queued_ev : nullptr, (size_t)(S * K));
+                                                 queue_first ? tune.queued_ev : nullptr, cp.ctas.size());
         tr.gpu("class blocks done", es);
         if (queue_first) FB2_CUDA(cudaStreamWaitEvent(st, tune.queued_ev, 0));
         tr.mark("class blocks launched");
         // chain output slots
-        const long long nchains = S * kMaxK;
         std::vector<unsigned long long> soff(nchains + 1, 0);
         for (long long g = 0; g < S; g++)
             for (int k = 0; k < kMaxK; k++) {
@@ -3088,28 +3572,11 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         unsigned long long *d_soff = h2d(pool, soff, st);
         uint8_t *slots = pool.get<uint8_t>(soff.back() + 16);
         unsigned long long *blen = pool.get<unsigned long long>(nchains);
-        {
-            tr.mark("tables launched");
-            const std::vector<unsigned long long> maps(R, 0), revs(R, 0);  // every table is resident
-            std::vector<int> chain_table((size_t)nchains);
-            for (long long ch = 0; ch < nchains; ch++) chain_table[ch] = seg_region[ch / kMaxK];
-            const std::vector<ChainCta> groups = chain_ctas(chain_table, maps, revs, (size_t)(kSpecThreads / ppc));
-            std::vector<SpecCta> ctas;
-            for (const ChainCta &c : groups) ctas.push_back(SpecCta{c.table, c.first, c.count, ppc, c.map, c.rev});
-            SpecCta *d_ctas = h2d(pool, ctas, st);
-            uint16_t *sparse = pool.get<uint16_t>(((size_t)N >> kSparseShift) + 2);
-            uint16_t *sparse_bits = pool.get<uint16_t>(((size_t)N >> kSparseShift) + 2);
-            uint32_t *stage = pool.get<uint32_t>(ctas.size() * kSpecThreads * spec_stage_words(enc_part));
-            uint32_t *rstage = pool.get<uint32_t>(ctas.size() * kSpecThreads * spec_stage_words(enc_part));
-            enable_big_smem();
-            tr.gpu("chain encoder start", st);
-            k_o1_encode_spec<<<(unsigned)ctas.size(), kSpecThreads, kSpecSmem, st>>>(
-                keys, d_segs, d_ctas, image, meta, sparse, sparse_bits, stage, rstage, slots, d_soff, blen, enc_part, o1ck,
-                d_ck_off, ck_every, d_err);
-            FB2_CHECK_LAUNCH();
-            tr.gpu("chain encoder done", st);
-            tr.mark("chains launched");
-        }
+        tr.mark("tables launched");
+        tr.gpu("chain encoder start", st);
+        encode_chains(pool, cp, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
+        tr.gpu("chain encoder done", st);
+        tr.mark("chains launched");
         GammaOut go = gamma_finish(spool, gblocks, evals, es);
         tr.gpu("escape mantissas packed", es);
         // the chains' escape counts (stream header) from the histogram pass; their sums per segment
@@ -3122,7 +3589,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         }
         tr.mark("escapes coded");
         std::vector<unsigned long long> h_blen = d2h(blen, (size_t)nchains, st);
-        std::vector<int> h_err = d2h(d_err, 5, st);
+        std::vector<int> h_err = d2h(d_err, 7, st);
         tr.gpu_dump();
         if (h_err[0]) throw std::runtime_error("tANS encoding failed (table construction or chain repair)");
         // Decode checkpoints cost 12 bytes each: keep them within 1.5 % of the chains' bytes by
@@ -3160,8 +3627,8 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
             }
         }
         if (tr.on)
-            std::fprintf(stderr, "[falcons trace] encode chain repair: %d codes re-run, %d rounds, %d far lookups; "
-                         "%lld segments, %d chains each\n", h_err[2], h_err[3], h_err[4], S, K);
+            std::fprintf(stderr, "[falcons trace] encode chain repair: %d codes re-run, %d rounds, %d of %u parts not met, %d chains unsettled; "
+                         "%lld segments, %d chains each\n", h_err[2], h_err[3], h_err[5], cp.pstart.back(), h_err[6], S, K);
         tr.mark("chains done");
         join();
         pool.ptrs.insert(pool.ptrs.end(), spool.ptrs.begin(), spool.ptrs.end());
