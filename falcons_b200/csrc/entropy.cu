@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <stdexcept>
+#include <type_traits>
 #include <vector>
 
 #include "assemble.cuh"
@@ -1788,29 +1789,112 @@ __global__ void __launch_bounds__(kTabThreads) k_o1_ctable(const uint16_t *__res
     }
 }
 
-// Decode tables, one packed u32 per cell: bits 0-12 newState, 13-16 nbBits, 17-20 the context
-// of the decoded code, 21 escape, 22-31 the code (10 bits, two's complement).
-__global__ void __launch_bounds__(kTabThreads) k_o1_dtable(const uint16_t *__restrict__ nf, uint32_t *__restrict__ dt,
-                                                         uint8_t *__restrict__ scratch, int *__restrict__ err) {
-    (void)scratch;
+// Decode tables of table blockIdx.x:
+//   cells  16 bits per cell: a symbol's cells are numbered in chunks of 128, the low 9 bits are the chunk (of
+//          all the table's, in symbol order: at most 256 + 8192 / 128), the high 7 the number within it; with
+//   info   one u32 per chunk: bits 0-3 the exponent of the lowest power of two above the symbol's count,
+//          4-7 the context of the code, 8-15 the code (-128: escape), 16 escape, 18-31 the state number
+//          (count + rank) of its first cell: 17 KiB a context, so that 11 to 13 of the 15 stay in shared memory
+// From a cell's state number n = info's + number and exponent x the decoder has nbBits = 14 - x - (n >> x)
+// and newState + 8192 = n << nbBits.  The last gridDim.x - ntab CTAs rank the contexts of a table set each.
+struct DecRank {
+    unsigned long long slot, ctx;  // 4 bits each: the slot of every context, the context of every slot
+};
+constexpr uint32_t kChunkBits = 7, kChunks = O1_NSYM + (O1_M >> kChunkBits);
+
+// Slots by how often a decoder is in a context: the stationary distribution of the context chain that the
+// counts imply (the next context is a function of the decoded code; escapes split between the two
+// large-magnitude contexts 13 and 14).  Those two take slots 0 and 1, so that an escape's sign is the slot.
+__device__ void rank_contexts(const uint16_t *__restrict__ nf, DecRank *__restrict__ out) {
+    __shared__ float P[2][O1_NCTX * O1_NCTX];
+    __shared__ float s_pi[O1_NCTX];
+    const uint32_t t = threadIdx.x;
+    if (t < O1_NCTX * O1_NCTX) P[0][t] = 0;
+    __syncthreads();
+    for (uint32_t k = t; k < O1_NCTX * O1_NSYM; k += blockDim.x) {
+        const int nn = (int16_t)nf[k];
+        if (nn == 0 || nn < -1) continue;
+        const uint32_t c = k / O1_NSYM, sy = k % O1_NSYM;
+        const float pr = (float)(nn < 0 ? 1 : nn) / O1_M;
+        if (sy == O1_NSYM - 1) {
+            atomicAdd(&P[0][c * O1_NCTX + 13], pr / 2);
+            atomicAdd(&P[0][c * O1_NCTX + 14], pr / 2);
+        } else {
+            atomicAdd(&P[0][c * O1_NCTX + o1_ctx(unzz(sy))], pr);
+        }
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int it = 0; it < 7; it++, cur ^= 1) {  // the chain's 128th power by squaring
+        if (t < O1_NCTX * O1_NCTX) {
+            float v = 0;
+            for (int k = 0; k < O1_NCTX; k++) v += P[cur][t / O1_NCTX * O1_NCTX + k] * P[cur][k * O1_NCTX + t % O1_NCTX];
+            P[cur ^ 1][t] = v;
+        }
+        __syncthreads();
+    }
+    if (t < O1_NCTX) {
+        float v = 0;
+        for (int k = 0; k < O1_NCTX; k++) v += P[cur][k * O1_NCTX + t];
+        s_pi[t] = v;
+    }
+    __syncthreads();
+    if (t == 0) {
+        DecRank r{0, 0};
+        auto put = [&](int c, int slot) {
+            r.slot |= (unsigned long long)slot << (4 * c);
+            r.ctx |= (unsigned long long)c << (4 * slot);
+        };
+        put(13, 0);
+        put(14, 1);
+        for (int c = 0; c < 13; c++) {
+            int rank = 2;
+            for (int d = 0; d < 13; d++) rank += s_pi[d] > s_pi[c] || (s_pi[d] == s_pi[c] && d < c);
+            put(c, rank);
+        }
+        *out = r;
+    }
+}
+
+__global__ void __launch_bounds__(kTabThreads) k_o1_dtable(const uint16_t *__restrict__ nf, uint32_t ntab,
+                                                         uint16_t *__restrict__ cells,
+                                                         uint32_t *__restrict__ info, DecRank *__restrict__ rank,
+                                                         int *__restrict__ err) {
     __shared__ TabSmem w;
     const size_t t = blockIdx.x;
+    if (t >= ntab) {
+        rank_contexts(nf + (t - ntab) * O1_NCTX * O1_NSYM, rank + (t - ntab));
+        return;
+    }
+    uint32_t *inf = info + t * kChunks;
+    uint16_t *ce = cells + t * O1_M;
     for (int s2 = threadIdx.x; s2 < O1_NSYM; s2 += blockDim.x) w.norm[s2] = (int16_t)nf[t * O1_NSYM + s2];
+    // chunks that no symbol takes, and all of a table that cannot be: emits nothing, stays in its state
+    constexpr uint32_t kStay = ((uint32_t)O1_M << 18) | 14u;
+    for (uint32_t c = threadIdx.x; c < kChunks; c += blockDim.x) inf[c] = kStay;
     __syncthreads();
     if (!cta_spread(w)) {
         if (threadIdx.x == 0) atomicExch(err, 5);
+        for (uint32_t u = threadIdx.x; u < O1_M; u += blockDim.x) ce[u] = 0;
         return;
     }
-    uint32_t *d = dt + t * O1_M;
-    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) {
-        const int nn = w.norm[sy];
-        const uint32_t ns = (nn == -1 ? 1u : (uint32_t)nn) + r;
-        const uint32_t nb = O1_PB - fse::highbit32(ns);
-        const uint32_t newState = (ns << nb) - O1_M;
+    const int my = threadIdx.x < O1_NSYM ? w.norm[threadIdx.x] : 0;
+    const uint32_t mine = my == -1 ? 1u : ((uint32_t)max(my, 0) + (1u << kChunkBits) - 1) >> kChunkBits;
+    uint32_t all;
+    const uint32_t first = block_excl_scan<uint32_t>(mine, w.scan[0], all);
+    if (threadIdx.x < O1_NSYM) {
+        const uint32_t sy = threadIdx.x;
         const bool esc = sy == O1_NSYM - 1;
-        const int code = esc ? 0 : unzz(sy);
-        const int ctx = esc ? 0 : o1_ctx(code);
-        d[u] = newState | (nb << 13) | ((uint32_t)ctx << 17) | ((uint32_t)esc << 21) | ((uint32_t)(code & 0x3FF) << 22);
+        const int code = esc ? -128 : unzz(sy);
+        const uint32_t n = w.norm[sy] == -1 ? 1u : (uint32_t)max((int)w.norm[sy], 0);
+        const uint32_t v = (n ? fse::highbit32(n) + 1 : 0u) | ((uint32_t)(esc ? 13 : o1_ctx(code)) << 4) |
+                           ((uint32_t)(code & 0xFF) << 8) | (esc ? 1u << 16 : 0u);
+        for (uint32_t j = 0; j < mine; j++) inf[first + j] = ((n + (j << kChunkBits)) << 18) | v;
+        w.occ[sy] = first;  // done with by the spread
+    }
+    __syncthreads();
+    cta_ranks(w, [&](uint32_t u, unsigned sy, uint32_t r) {
+        ce[u] = (uint16_t)((w.occ[sy] + (r >> kChunkBits)) | ((r & ((1u << kChunkBits) - 1)) << 9));
     });
 }
 
@@ -1825,91 +1909,12 @@ struct DecChain {
     uint32_t pad;
 };
 
-// One part of a chain decoded from a checkpoint (part 0 starts at the chain's stream end).
-struct DecPart {
-    uint32_t chain;
-    uint32_t part;
-};
-
-// ---- shared-memory resident context tables
-// A CTA encodes or decodes chains that share one table set; the tables of the contexts that carry
-// most symbols are staged in shared memory (the rest are read from global memory).  `map` packs,
-// per context, its shared-memory slot (4 bits, 15 = not resident); `rev` packs the context of
-// every slot.
-// A chain CTA holds up to 64 chains that share one table set (kept in shared memory, so one CTA
-// fills an SM).  The chains are spread over all 8 warps, 8 lanes each, so that every scheduler of
-// the SM has two warps of independent chain steps to interleave.
-constexpr int kChainThreads = 256;
-constexpr int kMaxChainsPerCta = 64;
-__device__ __forceinline__ int chain_slot() {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    return lane < kMaxChainsPerCta / (kChainThreads / 32) ? lane * (kChainThreads / 32) + warp : -1;
-}
-constexpr int kDecSlots = 7;   // 7 x 8192 x u32 decode tables = 224 KiB
+// Items [first, first + count) of one table set (chains or parts) that a CTA takes.
 struct ChainCta {
     int table;
     int first;
     int count;
-    int pad;
-    unsigned long long map, rev;
 };
-
-__global__ void __launch_bounds__(kChainThreads) k_o1_decode_smem(const uint8_t *__restrict__ in,
-                                                      const DecChain *__restrict__ chains,
-                                                      const ChainCta *__restrict__ ctas,
-                                                      const uint32_t *__restrict__ dt,
-                                                      const int16_t *__restrict__ ovf, unsigned long long n_ovf,
-                                                      int16_t *__restrict__ out, int *__restrict__ err) {
-    extern __shared__ uint4 smem_raw[];
-    uint32_t *sdt = reinterpret_cast<uint32_t *>(smem_raw);
-    const ChainCta w = ctas[blockIdx.x];
-    const uint32_t *__restrict__ tb = dt + (size_t)w.table * O1_NCTX * O1_M;
-    for (int j = 0; j < kDecSlots; j++) {
-        const int c = (int)((w.rev >> (4 * j)) & 15);
-        if (c >= O1_NCTX) continue;
-        const uint4 *src = reinterpret_cast<const uint4 *>(tb + (size_t)c * O1_M);
-        uint4 *dst = reinterpret_cast<uint4 *>(sdt + (size_t)j * O1_M);
-        for (int i = threadIdx.x; i < O1_M * 4 / 16; i += blockDim.x) dst[i] = __ldg(src + i);
-    }
-    __syncthreads();
-    const int lc = chain_slot();
-    if (lc < 0 || lc >= w.count) return;
-    const DecChain ch = chains[w.first + lc];
-    if (ch.n == 0) return;
-    fse::ReaderPF br;
-    const uint8_t *sb = in + ch.in;
-    if (ch.inlen == 0 || ch.inlen >= (1ull << 28) || !br.init(sb, (uint32_t)ch.inlen)) {
-        atomicExch(err, 6);
-        return;
-    }
-    const unsigned long long map = w.map;
-    uint32_t state = br.read(O1_PB);
-    uint32_t ctx = 0;
-    const int16_t *__restrict__ ov = ovf + ch.ovf;
-    const uint32_t nov = (uint32_t)min((unsigned long long)0x7fffffff, n_ovf - ch.ovf);
-    int16_t *o = out + ch.lo;
-    const uint32_t n = (uint32_t)ch.n;
-    uint32_t oi = 0;
-    // escape values queued two deep, so each load has several steps to arrive
-    int q0 = nov > 0 ? (int)__ldg(ov) : 0;
-    int q1 = nov > 1 ? (int)__ldg(ov + 1) : 0;
-    for (uint32_t j = 0; j < n; j++) {
-        const uint32_t sl = (uint32_t)(map >> (4 * ctx)) & 15u;
-        const uint32_t e = sl < (uint32_t)kDecSlots ? sdt[sl * O1_M + state] : __ldg(tb + ctx * O1_M + state);
-        const bool esc = (e >> 21) & 1u;
-        const int code = esc ? q0 : ((int)e >> 22);
-        ctx = esc ? 13u + (uint32_t)(code < 0) : ((e >> 17) & 15u);
-        if (esc) {
-            oi++;
-            q0 = q1;
-            q1 = oi + 1 < nov ? (int)__ldg(ov + oi + 1) : 0;
-        }
-        o[j] = (int16_t)code;
-        state = (e & 0x1FFFu) + br.read((e >> 13) & 15u);
-    }
-    if (oi > nov) atomicExch(err, 7);
-    if (br.pos < br.start_bit(sb) - 16) atomicExch(err, 8);
-}
 
 // ---- parallel chain encoder
 // Every chain is cut into parts of `part` codes, one part per thread.  A tANS encoder walks its
@@ -2733,193 +2738,307 @@ __global__ void __launch_bounds__(kPlaceWarps * 32) k_o1_place(const EncArgs A, 
     if (lane == 0 && pos) atomicOr(o, buf[0]);
 }
 
-// A decode table entry of a context not resident in shared memory (kept out of line so that the
-// global load is only issued when taken).
-__device__ __noinline__ uint32_t far_entry(const uint32_t *__restrict__ tb, uint32_t ctx, uint32_t state) {
-    return __ldg(tb + ctx * O1_M + state);
-}
-
-// Decodes the parts of tANS chains, one part per thread (the chains' checkpoints give every part's
-// starting bit position, state, context and escape offset).  The CTA's parts share one table set,
-// staged in shared memory as for k_o1_decode_smem.  Each part that ends at a checkpoint checks that
-// it arrived there (state, context, bit position, escapes); a mismatch sets err[1].
-constexpr int kPartThreads = 1024;
-__global__ void __launch_bounds__(kPartThreads) k_o1_decode_parts(const uint8_t *__restrict__ in,
-                                                                 const DecChain *__restrict__ chains,
-                                                                 const uint32_t *__restrict__ pstart,
-                                                                 uint32_t nchains,
-                                                                 const ChainCta *__restrict__ ctas,
-                                                                 const uint32_t *__restrict__ dt,
-                                                                 const int16_t *__restrict__ ovf,
-                                                                 unsigned long long n_ovf,
-                                                                 const O1Ckpt *__restrict__ cks, uint32_t part,
-                                                                 int16_t *__restrict__ out, int *__restrict__ err) {
+// ---- chain decoder
+// Decodes the parts of tANS chains, one part per thread: a part starts from the chain's checkpoint (bit
+// position, state, context, escapes before it) or, part 0, from the stream's end; without checkpoints
+// a chain is one part.  Each part that ends at a checkpoint checks that it arrived there; a mismatch sets err[1].
+// Escapes are written as kEscape and filled in by k_o1_fill; only an escape's sign, which selects the next
+// context, is read here.
+//
+// What bounds it: a part is a serial chain of lookups, so its time is the part's length times the
+// step's latency where few parts share an SM, and issue slots and the shared-memory pipe where many do.  What
+// a lane waits for, its whole warp waits for, so nothing on the chain may wait for memory beyond the SM:
+//   * tables: 16 bits a cell and a word a chunk (k_o1_dtable) keep 13 of 15 contexts in shared memory and the
+//     32 KiB of the two rarest mostly in L1 (with a word a cell 7 fit: 4 % of a 512^3 field's lookups then go to
+//     L2, three warp steps of four among them; and where one table set codes levels of unlike statistics, a
+//     part's busy contexts can be the rare ones of the whole: 1800 x 3600 points took 1.9 ms);
+//   * stream bits: every lane keeps the 8-byte pieces around its position in registers, loaded two pieces
+//     ahead; 64 bits are aligned for every 4 codes (at most 52 bits);
+//   * signs: one bit an escape (k_sign_bits), a word ahead.
+// Before (seven contexts of a word a cell, escapes and stream words read as they were needed) and now, with the
+// fill: 64^3 points 216 -> 118 us, 1800 x 3600 2800 -> 900 us, 211 x 307 x 401 1110 -> 440 us, 384^3 float64 (87 %
+// escapes) 3900 -> 975 us, 512^3 687 -> 595 us.
+constexpr int kDecThreads = 1024;
+constexpr uint32_t kDecWarps = 8;
+constexpr int16_t kEscape = -128;  // no code: codes are within +-127
+constexpr uint32_t kFillTile = 256;
+constexpr uint32_t kCellSlots = 13;  // contexts whose cells are in shared memory; the chunks of all are
+constexpr uint32_t kDecSmem = kCellSlots * O1_M * 2 + O1_NCTX * kChunks * 4;
+static_assert(kDecSmem <= 227 * 1024, "the tables fit an SM's shared memory");
+struct DecArgs {
+    const uint8_t *in;
+    const DecChain *chains;
+    const uint32_t *pstart;  // first part of every chain, then the number of parts
+    uint32_t nchains;
+    const EncCta *ctas;
+    const uint16_t *cells;
+    const uint32_t *info;
+    const DecRank *rank;
+    const uint32_t *signs;     // sign bits of the escapes
+    unsigned long long n_ovf;  // escapes
+    const O1Ckpt *cks;
+    unsigned long long part;   // codes per part
+    int16_t *out;
+    unsigned long long *tile;  // escapes before every kFillTile-th code
+    int *err;
+};
+__global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A) {
     extern __shared__ uint4 smem_raw[];
-    uint32_t *sdt = reinterpret_cast<uint32_t *>(smem_raw);
-    const ChainCta w = ctas[blockIdx.x];
-    const uint32_t *__restrict__ tb = dt + (size_t)w.table * O1_NCTX * O1_M;
-    for (int j = 0; j < kDecSlots; j++) {
-        const int c = (int)((w.rev >> (4 * j)) & 15);
-        if (c >= O1_NCTX) continue;
-        const uint4 *src = reinterpret_cast<const uint4 *>(tb + (size_t)c * O1_M);
-        uint4 *dst = reinterpret_cast<uint4 *>(sdt + (size_t)j * O1_M);
-        for (int i = threadIdx.x; i < O1_M * 4 / 16; i += blockDim.x) dst[i] = __ldg(src + i);
+    const EncCta w = A.ctas[blockIdx.x];
+    const DecRank rk = A.rank[w.table];
+    uint16_t *const cells = reinterpret_cast<uint16_t *>(smem_raw);
+    uint32_t *const info = reinterpret_cast<uint32_t *>(cells + kCellSlots * O1_M);
+    const size_t tab = (size_t)w.table * O1_NCTX;
+    auto ctx_of = [&](uint32_t slot) { return (uint32_t)(rk.ctx >> (4 * slot)) & 15u; };
+    auto slot_of = [&](uint32_t ctx) { return (uint32_t)(rk.slot >> (4 * ctx)) & 15u; };
+    // the tables come in by all threads, however few decode
+    for (uint32_t j = 0; j < kCellSlots; j++) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(A.cells + (tab + ctx_of(j)) * O1_M);
+        for (uint32_t i = threadIdx.x; i < O1_M / 8; i += kDecThreads) smem_raw[j * (O1_M / 8) + i] = __ldg(src + i);
+    }
+    for (uint32_t i = threadIdx.x; i < O1_NCTX * kChunks; i += kDecThreads) {
+        const uint32_t v = __ldg(A.info + (tab + ctx_of(i / kChunks)) * kChunks + i % kChunks);
+        info[i] = (v & ~0xF0u) | (slot_of((v >> 4) & 15u) << 4);
     }
     __syncthreads();
-    if ((int)threadIdx.x >= w.count) return;
-    // this thread's part: the last chain (from the CTA's first one on) whose first part is at or
-    // before the item
-    DecPart pp;
-    {
-        const uint32_t item = (uint32_t)(w.first + (int)threadIdx.x);
-        uint32_t lo = (uint32_t)w.pad, hi = nchains;  // pstart[lo] <= item < pstart[hi]
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(pstart + mid) <= item) lo = mid;
-            else hi = mid;
-        }
-        pp = DecPart{lo, item - __ldg(pstart + lo)};
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u, it = wid * w.lanes + lane;
+    if (lane >= w.lanes || it >= w.count) return;
+    const uint32_t id = w.first + it;
+    uint32_t c0 = w.chain, c1 = A.nchains;  // the chain of this part
+    while (c1 - c0 > 1) {
+        const uint32_t mid = (c0 + c1) >> 1;
+        if (__ldg(A.pstart + mid) <= id) c0 = mid;
+        else c1 = mid;
     }
-    const DecChain ch = chains[pp.chain];
-    const unsigned long long start = (unsigned long long)pp.part * part;
+    const DecChain ch = A.chains[c0];
+    const uint32_t pt = id - __ldg(A.pstart + c0);
+    const unsigned long long start = (unsigned long long)pt * A.part;
     if (ch.n == 0 || start >= ch.n || ch.inlen == 0 || ch.inlen >= (1ull << 28)) {
-        atomicExch(err, 6);
+        atomicExch(A.err, 6);
         return;
     }
-    const uint32_t n = (uint32_t)min((unsigned long long)part, ch.n - start);
+    const uint32_t n = (uint32_t)min(A.part, ch.n - start);
     const bool last = start + n >= ch.n;
-    const uint8_t *sb = in + ch.in;
-    const uint32_t sbits = (uint32_t)ch.inlen * 8u;
-    fse::ReaderPF br;
-    uint32_t state, ctx, oi0;
-    if (pp.part == 0) {
-        if (!br.init(sb, (uint32_t)ch.inlen)) {
-            atomicExch(err, 6);
+    const uint8_t *const sb = A.in + ch.in;
+    const uint2 *const base = reinterpret_cast<const uint2 *>(reinterpret_cast<uintptr_t>(sb) & ~uintptr_t(7));
+    const int32_t bit0 = (int32_t)(reinterpret_cast<uintptr_t>(sb) & 7) * 8;  // the stream's first bit from base
+    int32_t pos;                                                             // bits below it are unread
+    uint32_t s = 0, slot, oi0 = 0;                                           // state (8192 ..), context's slot
+    const uint32_t eend = last ? ch.nesc : A.cks[ch.ck + pt].esc;            // escapes up to the part's end
+    if (pt == 0) {
+        const uint8_t end = sb[ch.inlen - 1];
+        if (end == 0) {
+            atomicExch(A.err, 6);
             return;
         }
-        state = br.read(O1_PB);
-        ctx = 0;
-        oi0 = 0;
+        pos = bit0 + ((int32_t)ch.inlen - 1) * 8 + (int32_t)fse::highbit32(end);
+        slot = slot_of(0);
     } else {
-        const O1Ckpt c = cks[ch.ck + pp.part - 1];
-        if (c.bitpos >= sbits || c.state >= O1_M || c.ctx >= O1_NCTX || c.esc > ch.nesc) {
-            atomicExch(err + 1, 1);
+        const O1Ckpt k = A.cks[ch.ck + pt - 1];
+        if (k.bitpos >= (uint32_t)ch.inlen * 8u || k.state >= O1_M || k.ctx >= O1_NCTX || k.esc > ch.nesc) {
+            atomicExch(A.err + 1, 1);
             return;
         }
-        br.init_at(sb, (int32_t)c.bitpos);
-        state = c.state;
-        ctx = c.ctx;
-        oi0 = c.esc;
+        pos = bit0 + (int32_t)k.bitpos;
+        s = O1_M + k.state;
+        slot = slot_of(k.ctx);
+        oi0 = k.esc;
     }
-    const unsigned long long avail = n_ovf > ch.ovf + oi0 ? n_ovf - ch.ovf - oi0 : 0;
-    const uint32_t nov = (uint32_t)min((unsigned long long)(ch.nesc - oi0), avail);
-    int16_t *o = out + ch.lo + start;
-    const unsigned long long map = w.map;
-    uint32_t oi = 0;
-    // Escape values come in 16-byte chunks of eight (ovf is 16-byte aligned, with slack behind
-    // it); the chunk after the current one is loaded a whole chunk ahead, so that taking the next
-    // value never waits on memory.
-    const uint4 *ov4 = reinterpret_cast<const uint4 *>(ovf);
-    const long long eb = (long long)(ch.ovf + oi0);
-    long long ec = eb >> 3;
-    int ek = (int)(eb & 7);
-    auto echunk = [&](long long c) -> uint4 {
-        return (unsigned long long)(c << 3) < n_ovf ? __ldg(ov4 + c) : make_uint4(0, 0, 0, 0);
-    };
-    auto ext = [](const uint4 &u, int k) -> int {
-        const uint32_t wd = k < 4 ? (k < 2 ? u.x : u.y) : (k < 6 ? u.z : u.w);
-        return (int)(int16_t)(k & 1 ? wd >> 16 : wd & 0xFFFFu);
-    };
-    uint4 ecur = nov > 0 ? echunk(ec) : make_uint4(0, 0, 0, 0);
-    uint4 enxt = nov > 0 ? echunk(ec + 1) : make_uint4(0, 0, 0, 0);
-    int q0 = nov > 0 ? ext(ecur, ek) : 0;
-    auto step = [&]() -> int {
-        const uint32_t sl = (uint32_t)(map >> (4 * ctx)) & 15u;
-        uint32_t e;
-        if (sl < (uint32_t)kDecSlots) e = sdt[sl * O1_M + state];
-        else e = far_entry(tb, ctx, state);  // a real branch: the global load is never speculated
-        const bool esc = (e >> 21) & 1u;
-        const int code = esc ? q0 : ((int)e >> 22);
-        ctx = esc ? 13u + (uint32_t)(code < 0) : ((e >> 17) & 15u);
-        if (esc) {
-            oi++;
-            if (++ek == 8) {
-                ecur = enxt;
-                ec++;
-                enxt = echunk(ec + 1);
-                ek = 0;
-            }
-            q0 = oi < nov ? ext(ecur, ek) : 0;
+    // ---- the window: hi, lo = the 64 bits below pos, from the pieces q and q - 1 of 8 bytes (a, b), the piece
+    // q that holds bit pos; c and d come behind
+    int32_t q = pos >> 6;
+    // pieces before the input are not loaded (a damaged stream alone gets there)
+    const int32_t qmin = -(int32_t)min((unsigned long long)(1 << 20), (unsigned long long)(ch.in >> 3));
+    auto piece = [&](int32_t p) { return p >= qmin ? __ldg(base + p) : make_uint2(0, 0); };
+    uint2 a = piece(q), b = piece(q - 1), c = piece(q - 2), d = piece(q - 3);
+    uint32_t hi, lo;
+    auto align = [&]() {
+        if (pos >> 6 != q) {  // at most one piece on
+            q--;
+            a = b;
+            b = c;
+            c = d;
+            d = piece(q - 3);
         }
-        state = (e & 0x1FFFu) + br.read((e >> 13) & 15u);
-        return code;
+        const bool odd = pos & 32;
+        const uint32_t x = odd ? a.y : a.x, y = odd ? a.x : b.y, z = odd ? b.y : b.x;
+        hi = __funnelshift_r(y, x, pos);
+        lo = __funnelshift_r(z, y, pos);
+    };
+    align();
+    if (pt == 0) {
+        s = O1_M + (hi >> (32 - O1_PB));
+        pos -= O1_PB;
+        align();
+    }
+    // ---- signs of the escapes from oi0 on: words k, k + 1 and k + 2 of the sign bits
+    const unsigned long long e0 = ch.ovf + oi0;
+    const uint32_t avail = (uint32_t)min((unsigned long long)(ch.nesc - oi0), A.n_ovf > e0 ? A.n_ovf - e0 : 0ull);
+    const uint32_t *const sw = A.signs + (e0 >> 5);
+    const uint32_t words = (uint32_t)((A.n_ovf + 31) / 32 - min((A.n_ovf + 31) / 32, e0 >> 5));
+    auto sign_word = [&](uint32_t i) { return i < words ? __ldg(sw + i) : 0u; };
+    uint32_t k = 0, w0 = sign_word(0), w1 = sign_word(1), w2 = sign_word(2), sgn;
+    uint32_t oi = 0;
+    const uint32_t e5 = (uint32_t)(e0 & 31);
+    auto signs = [&]() {  // the next signs (at least 24) from bit 0 up
+        const uint32_t b = e5 + oi;
+        if ((b >> 5) != k) {
+            k++;
+            w0 = w1;
+            w1 = w2;
+            w2 = sign_word(k + 2);
+        }
+        sgn = __funnelshift_r(w0, w1, b);
+    };
+    signs();
+    uint32_t seen = 0;  // bit 16: an escape where none was expected
+    auto step = [&](auto esc_tag) -> uint32_t {  // one code: its chunk's word
+        constexpr bool ESC = decltype(esc_tag)::value;
+        uint32_t cell;
+        if (slot < kCellSlots) cell = cells[(slot << O1_PB) + s - O1_M];
+        else cell = __ldg(A.cells + (tab + ctx_of(slot)) * O1_M + s - O1_M);
+        const uint32_t e = info[slot * kChunks + (cell & 511u)];
+        const uint32_t ns = (e >> 18) + (cell >> 9), x = e & 15u, nb = 14u - x - (ns >> x);
+        s = __funnelshift_l(hi, ns, nb);  // ns << nb with the next nb bits below
+        hi = __funnelshift_l(lo, hi, nb);
+        lo <<= nb;
+        pos -= (int32_t)nb;
+        slot = (e >> 4) & 15u;
+        if (ESC) {
+            const uint32_t esc = (e >> 16) & 1u;
+            slot ^= esc & sgn;
+            sgn >>= esc;
+            oi += esc;
+        } else {
+            seen |= e;
+        }
+        return e;
+    };
+    int16_t *const o = A.out + ch.lo + start;
+    const unsigned long long i0 = ch.lo + start;
+    auto mark = [&](uint32_t j) {  // escapes before a tile's first code
+        if (((i0 + j) & (kFillTile - 1)) == 0) A.tile[(i0 + j) / kFillTile] = e0 + oi;
+    };
+    auto single = [&](uint32_t j) {
+        mark(j);
+        o[j] = (int16_t)(int8_t)(step(std::true_type()) >> 8);
+        align();
+        signs();
     };
     // codes leave in aligned groups of eight (one 16-byte store) between a scalar head and tail
-    const unsigned long long base = ch.lo + start;
     uint32_t j = 0;
-    for (; j < n && ((base + j) & 7); j++) o[j] = (int16_t)step();
-    for (; j + 8 <= n; j += 8) {
+    for (; j < n && ((i0 + j) & 7); j++) single(j);
+    auto eight = [&](auto esc_tag) {
+        mark(j);
+        if (decltype(esc_tag)::value) signs();
         uint32_t wv[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int a = step();
-            const int b = step();
-            wv[k] = (uint32_t)(uint16_t)a | ((uint32_t)(uint16_t)b << 16);
+        for (int g = 0; g < 2; g++) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t x = step(esc_tag), y = step(esc_tag);
+                // bytes 1 of both, sign-extended to 16 bits
+                asm("prmt.b32 %0, %1, %2, 0xD591;" : "=r"(wv[2 * g + h]) : "r"(x), "r"(y));
+            }
+            align();
         }
         *reinterpret_cast<uint4 *>(o + j) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+        j += 8;
+    };
+    // where no lane of the warp is to meet an escape, a quarter of a step's instructions are left out
+    if (__all_sync(__activemask(), oi0 + oi == eend)) {
+        while (j + 8 <= n) eight(std::false_type());
+        if (seen & 0x10000u) atomicExch(A.cks ? A.err + 1 : A.err, 7);
+    } else {
+        while (j + 8 <= n) eight(std::true_type());
     }
-    for (; j < n; j++) o[j] = (int16_t)step();
-    if (oi > nov) atomicExch(err, 7);
+    signs();
+    for (; j < n; j++) single(j);
+    if (oi > avail) atomicExch(A.err, 7);
     if (!last) {
-        const O1Ckpt c = cks[ch.ck + pp.part];
-        if (c.state != state || c.ctx != ctx || br.pos != br.start_bit(sb) + (int32_t)c.bitpos || c.esc != oi0 + oi)
-            atomicExch(err + 1, 1);
-    } else if (br.pos < br.start_bit(sb) - 16) {
-        atomicExch(err, 8);
+        const O1Ckpt k = A.cks[ch.ck + pt];
+        if (k.state != s - O1_M || k.ctx != ctx_of(slot) || pos != bit0 + (int32_t)k.bitpos ||
+            k.esc != oi0 + oi)
+            atomicExch(A.err + 1, 1);
+    } else if (pos < bit0 - 16) {
+        atomicExch(A.err, 8);
     }
 }
 
-std::pair<unsigned long long, unsigned long long> hot_contexts(const uint16_t *nf, int slots) {
-    double P[O1_NCTX][O1_NCTX] = {};
-    for (int c = 0; c < O1_NCTX; c++) {
-        for (int s = 0; s < O1_NSYM; s++) {
-            int f = (int16_t)nf[c * O1_NSYM + s];
-            if (f < 0) f = 1;
-            if (f == 0) continue;
-            const double pr = f / (double)O1_M;
-            if (s == O1_NSYM - 1) {
-                P[c][13] += pr / 2;
-                P[c][14] += pr / 2;
-            } else {
-                P[c][o1_ctx(unzz(s))] += pr;
-            }
+// Sign bits of the escape values: bit i of the bytes is value i's, a byte (a 16-byte vector) a thread.
+__global__ void __launch_bounds__(256) k_sign_bits(const int16_t *__restrict__ v, unsigned long long n,
+                                                   uint8_t *__restrict__ out) {
+    const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (8 * i >= n) return;  // (the vector's values past the last are in the allocation's slack)
+    const uint4 x = reinterpret_cast<const uint4 *>(v)[i];
+    auto two = [](uint32_t w) { return ((w >> 15) & 1u) | ((w >> 30) & 2u); };
+    out[i] = (uint8_t)(two(x.x) | (two(x.y) << 2) | (two(x.z) << 4) | (two(x.w) << 6));
+}
+
+// Fills in the escapes, a warp per kFillTiles tiles of 256 codes, 8 codes a lane: tile[t] is the number of
+// escapes before a tile, so a warp scan gives every escape its value's place.  Bound by memory (the codes once
+// in and once out, where a lane has an escape): and by issue: 145 us for 134 M codes, 14 % of them escapes.
+constexpr uint32_t kFillTiles = 4;
+__global__ void __launch_bounds__(256) k_o1_fill(int16_t *__restrict__ codes, long long n,
+                                                 const unsigned long long *__restrict__ tile,
+                                                 const int16_t *__restrict__ ovf, unsigned long long n_ovf) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const long long t0 = ((long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * kFillTiles;
+    uint4 v[kFillTiles];
+    unsigned long long at[kFillTiles];
+#pragma unroll
+    for (uint32_t k = 0; k < kFillTiles; k++) {
+        const long long i0 = (t0 + k) * kFillTile + lane * 8;
+        v[k] = i0 + 8 <= n ? *reinterpret_cast<const uint4 *>(codes + i0) : make_uint4(0, 0, 0, 0);
+        at[k] = (t0 + k) * (long long)kFillTile < n ? tile[t0 + k] : 0;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kFillTiles; k++) {
+        const long long i0 = (t0 + k) * kFillTile + lane * 8;
+        uint32_t wv[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+        if (i0 < n && i0 + 8 > n) {  // the last codes
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (i0 + u < n) wv[u >> 1] |= (uint32_t)(uint16_t)codes[i0 + u] << (16 * (u & 1));
+        }
+        uint32_t m[8], cnt = 0;  // which codes are escapes
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t x = wv[u] ^ 0xFF80FF80u;
+            m[2 * u] = (x & 0xFFFFu) == 0;
+            m[2 * u + 1] = x < 0x10000u;
+            cnt += m[2 * u] + m[2 * u + 1];
+        }
+        const uint32_t incl = warp_incl_scan(cnt);
+        if (cnt == 0) continue;
+        const unsigned long long e = at[k] + incl - cnt;
+        const int16_t *src = ovf + e;
+        const bool have = e + cnt <= n_ovf;  // else a damaged stream: its values are not read
+        uint32_t val[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            // a predicated load (a branch around each would cost as much again)
+            val[u] = 0;
+            asm("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p ld.global.nc.u16 %0, [%1];\n}"
+                : "+r"(val[u])
+                : "l"(src), "r"(have ? m[u] : 0u));
+            src += m[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t lo = m[2 * u] ? val[2 * u] : wv[u], hi = m[2 * u + 1] ? val[2 * u + 1] << 16 : wv[u];
+            wv[u] = (lo & 0xFFFFu) | (hi & 0xFFFF0000u);
+        }
+        if (i0 + 8 <= n) {
+            *reinterpret_cast<uint4 *>(codes + i0) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (i0 + u < n) codes[i0 + u] = (int16_t)(wv[u >> 1] >> (16 * (u & 1)));
         }
     }
-    double pi[O1_NCTX], nx[O1_NCTX];
-    for (int c = 0; c < O1_NCTX; c++) pi[c] = 1.0 / O1_NCTX;
-    for (int it = 0; it < 200; it++) {
-        for (int c = 0; c < O1_NCTX; c++) nx[c] = 0;
-        for (int a = 0; a < O1_NCTX; a++)
-            for (int b = 0; b < O1_NCTX; b++) nx[b] += pi[a] * P[a][b];
-        double sum = 0;
-        for (int c = 0; c < O1_NCTX; c++) sum += nx[c];
-        for (int c = 0; c < O1_NCTX; c++) pi[c] = sum > 0 ? nx[c] / sum : 1.0 / O1_NCTX;
-    }
-    int order[O1_NCTX];
-    for (int c = 0; c < O1_NCTX; c++) order[c] = c;
-    std::sort(order, order + O1_NCTX, [&](int a, int b) { return pi[a] > pi[b]; });
-    unsigned long long map = ~0ULL, rev = ~0ULL;
-    for (int j = 0; j < slots && j < O1_NCTX; j++) {
-        const int c = order[j];
-        map &= ~(15ULL << (4 * c));
-        map |= (unsigned long long)j << (4 * c);
-        rev &= ~(15ULL << (4 * j));
-        rev |= (unsigned long long)c << (4 * j);
-    }
-    return {map, rev};
 }
 
-// CTAs of up to 64 consecutive chains that share a table set.
 // Groups consecutive items (chains or parts) of one table into CTAs.  One CTA fills an SM (its
 // tables take the shared memory), so the CTAs should be at most one per SM: every run of one table
 // gets CTAs in proportion to its size (greedily, always to the run whose CTAs are largest), and
@@ -2942,8 +3061,7 @@ std::vector<ItemRun> table_runs(const std::vector<int> &chain_table) {
     return runs;
 }
 
-std::vector<ChainCta> run_ctas(const std::vector<ItemRun> &runs, size_t n, const std::vector<unsigned long long> &maps,
-                               const std::vector<unsigned long long> &revs, size_t max_per) {
+std::vector<ChainCta> run_ctas(const std::vector<ItemRun> &runs, size_t n, size_t max_per) {
     std::vector<ChainCta> out;
     const size_t sms = (size_t)sm_count();
     std::vector<size_t> ctas(runs.size(), 1);
@@ -2964,15 +3082,25 @@ std::vector<ChainCta> run_ctas(const std::vector<ItemRun> &runs, size_t n, const
         for (size_t k = 0; k < c; k++) {
             const size_t a = runs[r].first + runs[r].len * k / c;
             const size_t b = runs[r].first + runs[r].len * (k + 1) / c;
-            if (b > a) out.push_back(ChainCta{t, (int)a, (int)(b - a), 0, maps[t], revs[t]});
+            if (b > a) out.push_back(ChainCta{t, (int)a, (int)(b - a)});
         }
     }
     return out;
 }
 
-std::vector<ChainCta> chain_ctas(const std::vector<int> &chain_table, const std::vector<unsigned long long> &maps,
-                                 const std::vector<unsigned long long> &revs, size_t max_per = kMaxChainsPerCta) {
-    return run_ctas(table_runs(chain_table), chain_table.size(), maps, revs, max_per);
+// The CTAs over the items of every chain: item start[c] is the first of chain c's, start.back() their number.
+std::vector<EncCta> item_ctas(const std::vector<int> &chain_table, const std::vector<uint32_t> &start, size_t max_per) {
+    std::vector<ItemRun> runs = table_runs(chain_table);
+    for (auto &r : runs) r = ItemRun{start[r.first], start[r.first + r.len] - start[r.first], r.table};
+    runs.erase(std::remove_if(runs.begin(), runs.end(), [](const ItemRun &r) { return r.len == 0; }), runs.end());
+    std::vector<EncCta> out;
+    if (runs.empty()) return out;
+    for (const ChainCta &c : run_ctas(runs, start.back(), max_per)) {
+        EncCta e{c.table, (uint32_t)c.first, (uint32_t)c.count, 1, 0, 0};
+        e.chain = (uint32_t)(std::upper_bound(start.begin(), start.end(), e.first) - start.begin()) - 1;
+        out.push_back(e);
+    }
+    return out;
 }
 
 void enable_big_smem() {
@@ -2982,10 +3110,7 @@ void enable_big_smem() {
     FB2_CUDA(cudaGetDevice(&dev));
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
-    FB2_CUDA(cudaFuncSetAttribute(k_o1_decode_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kDecSlots * O1_M * 4));
-    FB2_CUDA(cudaFuncSetAttribute(k_o1_decode_parts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kDecSlots * O1_M * 4));
+    FB2_CUDA(cudaFuncSetAttribute(k_o1_decode_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecSmem));
     for (const void *k : {(const void *)k_o1_walk<false>, (const void *)k_o1_walk<true>, (const void *)k_o1_repair,
                           (const void *)k_o1_maps<1>,
                           (const void *)k_o1_maps<4>, (const void *)k_o1_compose, (const void *)k_o1_rounds, (const void *)k_o1_settle})
@@ -3021,23 +3146,8 @@ ChainParts chain_parts(const std::vector<SegInfo> &segs, const std::vector<int> 
     while (cp.spp < kMaxSuper && cp.pstart[n] / cp.spp > (uint32_t)(sm_count() * 8)) cp.spp *= 2;
     for (size_t c = 0; c < n; c++)
         cp.sstart[c + 1] = cp.sstart[c] + (cp.pstart[c + 1] - cp.pstart[c] + cp.spp - 1) / cp.spp;
-    int tables = 0;
-    for (int t : cp.table) tables = std::max(tables, t + 1);
-    const std::vector<unsigned long long> none((size_t)tables, 0);
-    auto ctas = [&](const std::vector<uint32_t> &start, size_t max_per) {
-        std::vector<ItemRun> runs = table_runs(cp.table);
-        for (auto &r : runs) r = ItemRun{start[r.first], start[r.first + r.len] - start[r.first], r.table};
-        runs.erase(std::remove_if(runs.begin(), runs.end(), [](const ItemRun &r) { return r.len == 0; }), runs.end());
-        std::vector<EncCta> out;
-        for (const ChainCta &c : run_ctas(runs, start[n], none, none, max_per)) {
-            EncCta e{c.table, (uint32_t)c.first, (uint32_t)c.count, 1, 0, 0};
-            e.chain = (uint32_t)(std::upper_bound(start.begin(), start.end(), e.first) - start.begin()) - 1;
-            out.push_back(e);
-        }
-        return out;
-    };
-    cp.ctas = ctas(cp.pstart, kEncThreads);
-    cp.map_ctas = ctas(cp.sstart, kEncThreads);
+    cp.ctas = item_ctas(cp.table, cp.pstart, kEncThreads);
+    cp.map_ctas = item_ctas(cp.table, cp.sstart, kEncThreads);
     for (EncCta &e : cp.ctas) {
         e.lanes = std::min(32u, (e.count + kEncWarps - 1) / kEncWarps);
         e.rec = cp.records;
@@ -3120,24 +3230,6 @@ __global__ void k_region_hist(const uint32_t *__restrict__ seg_hist, const int *
     reg_hist[(size_t)r * O1_NCTX * O1_NSYM + i] = s;
 }
 
-// Flags segments whose 15 x 256 table equals the previous segment's (decode-side deduplication).
-__global__ void k_table_same(const uint8_t *__restrict__ in, const unsigned long long *__restrict__ nf_off,
-                             int nseg, int *__restrict__ same) {
-    const int g = blockIdx.x;
-    if (g >= nseg) return;
-    __shared__ int diff;
-    if (threadIdx.x == 0) diff = (g == 0);
-    __syncthreads();
-    if (g > 0) {
-        const uint8_t *a = in + nf_off[g], *b = in + nf_off[g - 1];
-        for (int i = threadIdx.x; i < O1_NCTX * O1_NSYM * 2; i += blockDim.x)
-            if (a[i] != b[i]) diff = 1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) same[g] = !diff;
-}
-
-// Escape (|code| >= 128) extraction in index order: tile count + scan + scatter of zz+1 values.
 __global__ void __launch_bounds__(kScanThreads) k_esc_tiles(const int16_t *__restrict__ q, long long n,
                                                            uint32_t *__restrict__ cnt) {
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
@@ -3829,6 +3921,7 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         // escape values, decoded on the side stream while this stream builds the decode tables
         // (raw blocks are copied; gamma groups are unpacked straight into their place)
         int16_t *ovf = pool.get<int16_t>(ovf_total + 1);
+        uint32_t *signs = pool.get<uint32_t>(ovf_total / 32 + 1);
         SideFork fork(ctx, st);
         Pool spool(fork.side);
         {
@@ -3844,43 +3937,33 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
                              n_fck, d_cd, ovf);
             }
             launch_gather(spool, pcs, reinterpret_cast<uint8_t *>(ovf), fork.side);
+            if (ovf_total > 0) {
+                k_sign_bits<<<(unsigned)((ovf_total + 2047) / 2048), 256, 0, fork.side>>>(ovf, ovf_total,
+                                                                                         reinterpret_cast<uint8_t *>(signs));
+                FB2_CHECK_LAUNCH();
+            }
         }
         tr.gpu("escapes decoded", fork.side);
         tr.mark("escapes launched");
-        // decode tables: consecutive segments with identical tables share one decode table set
-        std::vector<int> uid(S, 0);
-        std::vector<unsigned long long> lead;
-        {
-            std::vector<unsigned long long> nfo(nf_off.begin(), nf_off.end());
-            unsigned long long *d_nfo = h2d(pool, nfo, st);
-            int *d_same = pool.get<int>(S);
-            k_table_same<<<(unsigned)S, 256, 0, st>>>(d_in, d_nfo, (int)S, d_same);
-            FB2_CHECK_LAUNCH();
-            std::vector<int> same = d2h(d_same, (size_t)S, st);
-            for (unsigned long long g = 0; g < S; g++) {
-                if (g == 0 || !same[g]) lead.push_back(nf_off[g]);
-                uid[g] = (int)lead.size() - 1;
-            }
-        }
-        tr.mark("shared tables found");
-        const int U = (int)lead.size();
-        const int ntab = U * O1_NCTX;
+        // decode tables of every segment (segments that share counts build the same tables: no one waits
+        // for a comparison)
+        const uint32_t ntab = (uint32_t)S * O1_NCTX;
         uint16_t *nf = pool.get<uint16_t>((size_t)ntab * O1_NSYM);
         {
             std::vector<Piece> pcs;
-            for (int u = 0; u < U; u++)
-                pcs.push_back(Piece{d_in + lead[u], (unsigned long long)u * O1_NCTX * O1_NSYM * 2, O1_NCTX * O1_NSYM * 2});
+            for (unsigned long long g = 0; g < S; g++) {
+                const size_t at = nf_off[g] ? nf_off[g] : nf_off[0];  // an empty segment has no counts of its own
+                pcs.push_back(Piece{d_in + at, g * O1_NCTX * O1_NSYM * 2, O1_NCTX * O1_NSYM * 2});
+            }
             launch_gather(pool, pcs, reinterpret_cast<uint8_t *>(nf), st);
         }
-        // the host ranks the tables' contexts while the device builds the decode tables
-        const std::vector<uint16_t> hnf = d2h(nf, (size_t)ntab * O1_NSYM, st);
-        tr.mark("tables read");
-        uint32_t *dt = pool.get<uint32_t>((size_t)ntab * O1_M);
-        uint8_t *spread = pool.get<uint8_t>(16);
-        k_o1_dtable<<<ntab, kTabThreads, 0, st>>>(nf, dt, spread, d_err);
+        DecArgs A{};
+        uint16_t *cells = pool.get<uint16_t>((size_t)ntab * O1_M);
+        uint32_t *info = pool.get<uint32_t>((size_t)ntab * kChunks);
+        DecRank *rank = pool.get<DecRank>(S);
+        k_o1_dtable<<<ntab + (unsigned)S, kTabThreads, 0, st>>>(nf, ntab, cells, info, rank, d_err);
         FB2_CHECK_LAUNCH();
         tr.gpu("decode tables built", st);
-        for (auto &c : chains) c.table = uid[c.table];
         // checkpoint base of every chain; the checkpoints are used only if their count matches
         bool parts_ok = false;
         if (o1ck) {
@@ -3891,58 +3974,49 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
             }
             parts_ok = tot == n_o1ck;
         }
-        DecChain *dch = h2d(pool, chains, st);
-        {
-            tr.mark("decode tables launched");
-            std::vector<unsigned long long> maps(U), revs(U);
-            for (int u = 0; u < U; u++) {
-                auto mr = hot_contexts(hnf.data() + (size_t)u * O1_NCTX * O1_NSYM, kDecSlots);
-                maps[u] = mr.first;
-                revs[u] = mr.second;
-            }
-            tr.mark("hot contexts ranked");
-            enable_big_smem();
-            fork.join();  // the chains consume the escape values
-            if (parts_ok) {
-                // parts of every chain (their first indices in pstart), CTAs over runs of one table
-                std::vector<uint32_t> pstart(chains.size() + 1, 0);
-                std::vector<int> chain_table(chains.size());
-                for (size_t i = 0; i < chains.size(); i++) {
-                    const unsigned long long np = chains[i].n ? 1 + (chains[i].n - 1) / o1_part : 0;
-                    pstart[i + 1] = pstart[i] + (uint32_t)np;
-                    chain_table[i] = chains[i].table;
-                }
-                std::vector<ItemRun> runs = table_runs(chain_table);
-                for (auto &r : runs) {
-                    const size_t a = pstart[r.first], b = pstart[r.first + r.len];
-                    r.first = a;
-                    r.len = b - a;
-                }
-                std::vector<ChainCta> ctas = run_ctas(runs, pstart.back(), maps, revs, kPartThreads);
-                for (auto &c : ctas)  // the chain of the CTA's first part
-                    c.pad = (int)(std::upper_bound(pstart.begin(), pstart.end(), (uint32_t)c.first) - pstart.begin()) - 1;
-                tr.mark("parts listed");
-                ChainCta *d_ctas = h2d(pool, ctas, st);
-                uint32_t *d_pstart = h2d(pool, pstart, st);
-                k_o1_decode_parts<<<(unsigned)ctas.size(), kPartThreads, kDecSlots * O1_M * 4, st>>>(
-                    d_in, dch, d_pstart, (uint32_t)chains.size(), d_ctas, dt, ovf, ovf_total, o1ck, o1_part, d_codes,
-                    d_err);
-                FB2_CHECK_LAUNCH();
-            } else {
-                std::vector<int> chain_table(chains.size());
-                for (size_t i = 0; i < chains.size(); i++) chain_table[i] = chains[i].table;
-                std::vector<ChainCta> ctas = chain_ctas(chain_table, maps, revs);
-                ChainCta *d_ctas = h2d(pool, ctas, st);
-                k_o1_decode_smem<<<(unsigned)ctas.size(), kChainThreads, kDecSlots * O1_M * 4, st>>>(
-                    d_in, dch, d_ctas, dt, ovf, ovf_total, d_codes, d_err);
-                FB2_CHECK_LAUNCH();
-            }
+        // without checkpoints a chain is one part
+        const unsigned long long part = parts_ok ? o1_part : 1ull << 31;
+        std::vector<uint32_t> pstart(chains.size() + 1, 0);
+        std::vector<int> chain_table(chains.size());
+        for (size_t i = 0; i < chains.size(); i++) {
+            pstart[i + 1] = pstart[i] + (chains[i].n ? 1 + (uint32_t)((chains[i].n - 1) / part) : 0);
+            chain_table[i] = chains[i].table;
+        }
+        std::vector<EncCta> ctas = item_ctas(chain_table, pstart, kDecThreads);
+        for (auto &c : ctas) c.lanes = std::min(32u, (c.count + kDecWarps - 1) / kDecWarps);
+        A.in = d_in;
+        A.chains = h2d(pool, chains, st);
+        A.pstart = h2d(pool, pstart, st);
+        A.nchains = (uint32_t)chains.size();
+        A.ctas = h2d(pool, ctas, st);
+        A.cells = cells;
+        A.info = info;
+        A.rank = rank;
+        A.signs = signs;
+        A.n_ovf = ovf_total;
+        A.cks = parts_ok ? o1ck : nullptr;
+        A.part = part;
+        A.out = d_codes;
+        A.tile = pool.get<unsigned long long>((size_t)N / kFillTile + 1);
+        A.err = d_err;
+        enable_big_smem();
+        fork.join();  // the chains consume the escapes' signs
+        tr.mark("parts listed");
+        if (!ctas.empty()) {
+            k_o1_decode_parts<<<(unsigned)ctas.size(), kDecThreads, kDecSmem, st>>>(A);
+            FB2_CHECK_LAUNCH();
+        }
+        tr.gpu("chains decoded", st);
+        if (ovf_total > 0) {
+            const long long per = 8ll * kFillTiles * kFillTile;  // codes a CTA
+            k_o1_fill<<<(unsigned)((N + per - 1) / per), 256, 0, st>>>(d_codes, N, A.tile, ovf, ovf_total);
+            FB2_CHECK_LAUNCH();
         }
     } else {
         throw std::invalid_argument("unsupported entropy method");
     }
     tr.mark("chains launched");
-    tr.gpu("chains decoded", st);
+    tr.gpu("escapes filled in", st);
     if (delta) undelta(pool, d_codes, N, st);
     std::vector<int> he = d2h(d_err, 2, st);
     tr.gpu_dump();
