@@ -661,6 +661,56 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
     }
 }
 
+// Backward reader of a bit stream: hi and lo are the 64 bits below `pos`, aligned in registers from the 8-byte
+// pieces q and q - 1 (q: the one that holds bit pos), with two more loaded behind them, so that neither a lane's
+// own loads nor those that other lanes of its warp just asked for are waited on.  align() after at most 52
+// bits taken.  Bits are counted from `base`, the stream's first byte rounded down to 8.
+struct BackWindow {
+    const uint2 *base;
+    int32_t pos, q, qmin;
+    uint2 a, b, c, d;
+    uint32_t hi, lo;
+    __device__ __forceinline__ uint2 piece(int32_t p) const { return p >= qmin ? __ldg(base + p) : make_uint2(0, 0); }
+    // Starts below bit `bit` of the stream at sb; `front`: readable bytes in front of sb (pieces further in
+    // front are not loaded: a damaged stream alone gets there).  Returns the stream's first bit.
+    __device__ __forceinline__ int32_t init(const uint8_t *sb, unsigned long long front, int32_t bit) {
+        const int32_t bit0 = (int32_t)(reinterpret_cast<uintptr_t>(sb) & 7) * 8;
+        base = reinterpret_cast<const uint2 *>(reinterpret_cast<uintptr_t>(sb) & ~uintptr_t(7));
+        qmin = -(int32_t)min((unsigned long long)(1 << 20), front >> 3);
+        pos = bit0 + bit;
+        q = pos >> 6;
+        a = piece(q);
+        b = piece(q - 1);
+        c = piece(q - 2);
+        d = piece(q - 3);
+        align();
+        return bit0;
+    }
+    __device__ __forceinline__ void align() {
+        if (pos >> 6 != q) {  // at most one piece on
+            q--;
+            a = b;
+            b = c;
+            c = d;
+            d = piece(q - 3);
+        }
+        const bool odd = pos & 32;
+        const uint32_t x = odd ? a.y : a.x, y = odd ? a.x : b.y, z = odd ? b.y : b.x;
+        hi = __funnelshift_r(y, x, pos);
+        lo = __funnelshift_r(z, y, pos);
+    }
+    __device__ __forceinline__ void skip(uint32_t nb) {
+        hi = __funnelshift_l(lo, hi, nb);
+        lo <<= nb;
+        pos -= (int32_t)nb;
+    }
+    __device__ __forceinline__ uint32_t take(uint32_t nb) {  // nb < 32
+        const uint32_t v = __funnelshift_l(hi, 0u, nb);
+        skip(nb);
+        return v;
+    }
+};
+
 // One CTA of kFseDecThreads per 64 Ki block: thread 0 reads the table header, the first warp
 // builds the decode table in shared memory (zfse/fse_decompress.c FSE_buildDTable), then the block
 // decodes either as one sequence (thread 0, two interleaved states,
@@ -671,19 +721,24 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
 constexpr int kFseDecThreads = 64;  // parts of a block decode one per thread
 constexpr unsigned kPartPad = 4;     // bytes between the parts' regions of the decoded block (>= 2:
                                      // the last part may hold two symbols past `part`)
-// the decoded block in shared memory: FBLK symbols plus kPartPad per part (parts of >= 64 symbols)
-constexpr int kFseDecSmem = FBLK + (FBLK / 64) * kPartPad;
+// Dynamic shared memory: the decoded block (FBLK symbols plus kPartPad per part), which the table's spread
+// uses first, then the decode table, when its log is at most kFseDecLog (a larger one, which no encoder
+// here writes, goes to `big`): 76 KB at parts of 1024 symbols, three blocks an SM.  (With room for the
+// largest table two fitted: 310 against 217 us for 758 blocks.)
+constexpr unsigned kFseDecLog = 11;
+inline size_t fse_dec_smem(uint32_t part) { return FBLK + (FBLK / part) * kPartPad + (sizeof(fse::DEntry) << kFseDecLog); }
 __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint8_t *__restrict__ in,
                                                          const BlockJob *__restrict__ jobs,
                                                          uint8_t *__restrict__ cls, int *__restrict__ err,
-                                                         uint32_t part, const FseCkpt *__restrict__ cks) {
-    __shared__ fse::DEntry dt[1 << fse::kMaxTableLog];
-    __shared__ uint8_t sym[1 << fse::kMaxTableLog];
+                                                         uint32_t part, const FseCkpt *__restrict__ cks,
+                                                         fse::DEntry *__restrict__ big) {
     __shared__ int16_t s_norm[256];
     __shared__ uint32_t s_scan[257], s_next[256];
     __shared__ unsigned tl_sh, hdr_sh, maxsv_sh, high_sh;
-    extern __shared__ uint4 s_out4[];  // the block's symbols (FBLK bytes), copied out at the end
-    uint8_t *s_out = reinterpret_cast<uint8_t *>(s_out4);
+    extern __shared__ uint4 s_out4[];
+    uint8_t *s_out = reinterpret_cast<uint8_t *>(s_out4), *sym = s_out;
+    fse::DEntry *const s_dt = reinterpret_cast<fse::DEntry *>(s_out + FBLK + (FBLK / part) * kPartPad);
+    fse::DEntry *const g_dt = big + ((size_t)blockIdx.x << fse::kMaxTableLog);
     const BlockJob jb = jobs[blockIdx.x];
     uint8_t *dst = cls + jb.src;
     const uint8_t *p = in + jb.in;
@@ -762,9 +817,12 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
             if (u < L) {
                 const uint32_t ns = s_next[sv] + rank;
                 const uint32_t nb = tl - fse::highbit32(ns);
-                dt[u].symbol = (uint8_t)sv;
-                dt[u].nbBits = (uint8_t)nb;
-                dt[u].newState = (uint16_t)((ns << nb) - L);
+                fse::DEntry e;
+                e.symbol = (uint8_t)sv;
+                e.nbBits = (uint8_t)nb;
+                e.newState = (uint16_t)((ns << nb) - L);
+                if (tl <= kFseDecLog) s_dt[u] = e;
+                else g_dt[u] = e;
             }
             __syncwarp();
             if (u < L && rank == (unsigned)__popc(peers) - 1u) s_next[sv] += rank + 1;
@@ -776,54 +834,65 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
     const uint32_t ssz = (uint32_t)(size - hdr_sh);
     const unsigned n = jb.n;
     const unsigned nparts = jb.ck == 0xFFFFFFFFu ? 1u : 1u + fse_ckpt_count(n, part);
-    for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) {
-        fse::ReaderPF br;
+    auto decode = [&](unsigned q, const fse::DEntry *dt) {
+        BackWindow br;
         uint32_t s0, s1;
+        int32_t bit0;
         const unsigned start = q * (nparts > 1 ? part : 0u);
         const unsigned end = q + 1 < nparts ? start + part : n;
+        const unsigned long long front = jb.in + hdr_sh;
         if (q == 0) {
-            if (!br.init(sp, ssz)) {
+            const uint8_t last = ssz ? sp[ssz - 1] : 0;
+            if (last == 0) {
                 atomicExch(err, 1);
-                continue;
+                return;
             }
-            s0 = br.read(tl);
-            s1 = br.read(tl);
+            bit0 = br.init(sp, front, (int32_t)(ssz - 1) * 8 + (int32_t)fse::highbit32(last));
+            s0 = br.take(tl);
+            s1 = br.take(tl);
+            br.align();
         } else {
             const FseCkpt c = cks[jb.ck + q - 1];
             if (c.bitpos >= ssz * 8u || (c.s0 >> tl) || (c.s1 >> tl)) {
                 atomicExch(err + 1, 1);
-                continue;
+                return;
             }
-            br.init_at(sp, (int32_t)c.bitpos);
+            bit0 = br.init(sp, front, (int32_t)c.bitpos);
             s0 = c.s0;
             s1 = c.s1;
         }
         // Part q's symbols go to its own region of shared memory, kPartPad bytes more than a part
         // apart, four to a word: the parts' word stores then fall on different banks.
         uint8_t *so = s_out + (size_t)q * (nparts > 1 ? part + kPartPad : 0u);
-        unsigned i = start;
-        uint32_t wv = 0;
-        unsigned k = 0;
-        for (; i + 1 < end; i += 2) {
+        auto pair = [&]() -> uint32_t {  // two symbols; at most 2 * 13 bits
             const fse::DEntry e0 = dt[s0];
             const fse::DEntry e1 = dt[s1];
-            wv |= ((uint32_t)e0.symbol | ((uint32_t)e1.symbol << 8)) << (8 * k);
-            k += 2;
-            if (k == 4) {
-                *reinterpret_cast<uint32_t *>(so + (i + 2 - start - 4)) = wv;
-                wv = 0;
-                k = 0;
-            }
-            s0 = e0.newState + br.read(e0.nbBits);
-            s1 = e1.newState + br.read(e1.nbBits);
+            s0 = e0.newState + br.take(e0.nbBits);
+            s1 = e1.newState + br.take(e1.nbBits);
+            return (uint32_t)e0.symbol | ((uint32_t)e1.symbol << 8);
+        };
+        unsigned i = start;
+        for (; i + 3 < end; i += 4) {
+            const uint32_t lo = pair(), hi = pair();
+            br.align();
+            *reinterpret_cast<uint32_t *>(so + (i - start)) = lo | (hi << 16);
         }
-        for (unsigned t = 0; t < k; t++) so[i - start - k + t] = (uint8_t)(wv >> (8 * t));
+        for (; i + 1 < end; i += 2) {
+            const uint32_t v = pair();
+            br.align();
+            so[i - start] = (uint8_t)v;
+            so[i - start + 1] = (uint8_t)(v >> 8);
+        }
         if (i < end) so[i - start] = dt[s0].symbol;
         if (q + 1 < nparts) {
             const FseCkpt c = cks[jb.ck + q];
-            if (c.s0 != s0 || c.s1 != s1 || br.pos != br.start_bit(sp) + (int32_t)c.bitpos) atomicExch(err + 1, 1);
+            if (c.s0 != s0 || c.s1 != s1 || br.pos != bit0 + (int32_t)c.bitpos) atomicExch(err + 1, 1);
         }
-    }
+    };
+    if (tl <= kFseDecLog)
+        for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, s_dt);
+    else
+        for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, g_dt);
     // the symbols leave in consecutive bytes across the CTA (each thread's part decoded into
     // shared memory, so that no warp store scatters over the parts)
     __syncthreads();
@@ -949,7 +1018,7 @@ void enable_fse_smem() {
                                   (int)(kFseGroups * kFseNxtBytes)));
     FB2_CUDA(cudaFuncSetAttribute(k_fse_encode_blocks<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kFseNxtBytes));
-    FB2_CUDA(cudaFuncSetAttribute(k_fse_decode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, kFseDecSmem));
+    FB2_CUDA(cudaFuncSetAttribute(k_fse_decode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fse_dec_smem(64)));
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
 
@@ -1162,7 +1231,7 @@ void add_class_pieces(Assembler &as, const GammaOut &go, int g, CkptCollector *c
 // with ustart[g] <= u.  A warp sums a unit's classes (its mantissa bits); an exclusive scan of the
 // unit sums gives every unit its first bit; a thread then reads its unit's mantissas in order
 // (MSB-first bits of the group's byte region, one aligned word at a time).
-constexpr unsigned kUnit = 1024;
+constexpr unsigned kUnit = 1024, kRun = 4;
 
 __device__ __forceinline__ int unit_group(const unsigned long long *__restrict__ ustart, int G, unsigned long long u) {
     int lo = 0, hi = G - 1;
@@ -1192,8 +1261,9 @@ __global__ void __launch_bounds__(256) k_unit_bits(const uint8_t *__restrict__ c
 
 // Escape values (zigzag + 1, gamma-coded) of every unit, a warp per unit: v[i] = (1 << k) |
 // mantissa, or, with `ovf`, the escape code unzz(v - 1) at its place gdst[g] + (i - gstart[g]).
-// uoff is the exclusive scan of the unit bit sums; the warp takes its unit's values 32 at a time,
-// a warp scan of their classes giving each lane its mantissa's bit offset.  A class above 31 sets
+// uoff is the exclusive scan of the unit bit sums; the warp takes its unit's values kRun a lane at a
+// time, a warp scan of their classes giving each lane its mantissas' bit offset (a scan for every 32 values
+// was most of the instructions: 250 us for 49 M values, this takes 116).  A class above 31 sets
 // err 2, a mantissa past its group's region err 3.
 __global__ void __launch_bounds__(256) k_gamma_unpack_units(
     const uint8_t *__restrict__ cls, const unsigned long long *__restrict__ gstart,
@@ -1212,39 +1282,65 @@ __global__ void __launch_bounds__(256) k_gamma_unpack_units(
     const uint8_t *rb = base + gman[g];
     unsigned long long run = uoff[u] - uoff[ustart[g]];  // bit offset of the values below
     bool bad2 = false, bad3 = false;
-    for (unsigned long long i0 = first; i0 < end; i0 += 32) {
-        const unsigned long long i = i0 + lane;
-        const bool act = i < end;
-        const unsigned k = act ? cls[i] : 0u;
-        uint32_t incl = k;
+    const uintptr_t ra = reinterpret_cast<uintptr_t>(rb);
+    const uint32_t *rw = reinterpret_cast<const uint32_t *>(ra & ~uintptr_t(3));
+    const unsigned lead = (unsigned)(ra & 3) * 8;
+    for (unsigned long long i0 = first; i0 < end; i0 += 32 * kRun) {
+        const unsigned long long i = i0 + lane * kRun;
+        unsigned k[kRun];
+        uint32_t sum = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (unsigned)o) incl += t;
+        for (unsigned j = 0; j < kRun; j++) {
+            k[j] = i + j < end ? cls[i + j] : 0u;
+            if (k[j] > 31) {
+                bad2 = true;
+                k[j] = 0;
+            }
+            sum += k[j];
         }
-        const unsigned long long bb = run + incl - k;
+        const uint32_t incl = warp_incl_scan(sum);
+        const unsigned long long bb = run + incl - sum;
         run += __shfl_sync(0xffffffffu, incl, 31);
-        if (!act) continue;
-        uint32_t m = 0;
-        if (k > 31) {
-            bad2 = true;
-        } else if (k > 0) {
-            if (((bb + k + 7) >> 3) > len) {
-                bad3 = true;
+        if (i >= end) continue;
+        uint32_t val[kRun];
+        if (((bb + sum + 7) >> 3) > len) {
+            bad3 = true;
+#pragma unroll
+            for (unsigned j = 0; j < kRun; j++) val[j] = 1u << k[j];
+        } else {
+            // the lane's bits from the first word on, as big-endian words; 96 bits at a time cover the word's
+            // offset and 64 bits (classes up to 16), more classes take a load a value
+            unsigned long long at = lead + bb;
+            auto word = [&](unsigned long long w, unsigned long long last) {  // words up to that of bit `last`
+                return w <= last >> 5 ? __byte_perm(__ldg(rw + w), 0, 0x0123) : 0u;
+            };
+            if (sum <= 64) {
+                const unsigned long long w = at >> 5, last = at + (sum ? sum - 1 : 0);
+                const uint32_t x0 = sum ? word(w, last) : 0u, x1 = word(w + 1, last), x2 = word(w + 2, last);
+                const unsigned o = (unsigned)(at & 31);
+                uint32_t hi = __funnelshift_l(x1, x0, o), lo = __funnelshift_l(x2, x1, o);
+#pragma unroll
+                for (unsigned j = 0; j < kRun; j++) {
+                    val[j] = __funnelshift_l(hi, 1u, k[j]);  // 1 << k with the mantissa below
+                    hi = __funnelshift_l(lo, hi, k[j]);
+                    lo <<= k[j];
+                }
             } else {
-                const uintptr_t a = reinterpret_cast<uintptr_t>(rb + (bb >> 3));
-                const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
-                const unsigned lead = (unsigned)(a & 3);
-                const unsigned need = lead + (unsigned)((((bb & 7) + k) + 7) >> 3);  // bytes from w[0]
-                const uint32_t w0 = __byte_perm(w[0], 0, 0x0123);
-                const uint32_t w1 = need > 4 ? __byte_perm(w[1], 0, 0x0123) : 0u;
-                const unsigned long long be = ((unsigned long long)w0 << 32) | w1;  // big-endian bytes
-                m = (uint32_t)((be << (lead * 8 + (unsigned)(bb & 7))) >> (64 - k));
+#pragma unroll
+                for (unsigned j = 0; j < kRun; j++) {
+                    const unsigned long long w = at >> 5, last = at + (k[j] ? k[j] - 1 : 0);
+                    const uint32_t x0 = k[j] ? word(w, last) : 0u, x1 = word(w + 1, last);
+                    val[j] = __funnelshift_l(__funnelshift_l(x1, x0, (unsigned)(at & 31)), 1u, k[j]);
+                    at += k[j];
+                }
             }
         }
-        const uint32_t val = k <= 31 ? ((1u << k) | m) : 0u;
-        if (ovf) ovf[gdst[g] + (i - g0)] = (int16_t)unzz(val - 1u);
-        else v[i] = val;
+#pragma unroll
+        for (unsigned j = 0; j < kRun; j++) {
+            if (i + j >= end) continue;
+            if (ovf) ovf[gdst[g] + (i + j - g0)] = (int16_t)unzz(val[j] - 1u);
+            else v[i + j] = val[j];
+        }
     }
     if (bad2) atomicExch(err, 2);
     if (bad3) atomicExch(err, 3);
@@ -2820,9 +2916,7 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
     const uint32_t n = (uint32_t)min(A.part, ch.n - start);
     const bool last = start + n >= ch.n;
     const uint8_t *const sb = A.in + ch.in;
-    const uint2 *const base = reinterpret_cast<const uint2 *>(reinterpret_cast<uintptr_t>(sb) & ~uintptr_t(7));
-    const int32_t bit0 = (int32_t)(reinterpret_cast<uintptr_t>(sb) & 7) * 8;  // the stream's first bit from base
-    int32_t pos;                                                             // bits below it are unread
+    int32_t pos;                                                             // the stream's bits below it are unread
     uint32_t s = 0, slot, oi0 = 0;                                           // state (8192 ..), context's slot
     const uint32_t eend = last ? ch.nesc : A.cks[ch.ck + pt].esc;            // escapes up to the part's end
     if (pt == 0) {
@@ -2831,7 +2925,7 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
             atomicExch(A.err, 6);
             return;
         }
-        pos = bit0 + ((int32_t)ch.inlen - 1) * 8 + (int32_t)fse::highbit32(end);
+        pos = ((int32_t)ch.inlen - 1) * 8 + (int32_t)fse::highbit32(end);
         slot = slot_of(0);
     } else {
         const O1Ckpt k = A.cks[ch.ck + pt - 1];
@@ -2839,37 +2933,16 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
             atomicExch(A.err + 1, 1);
             return;
         }
-        pos = bit0 + (int32_t)k.bitpos;
+        pos = (int32_t)k.bitpos;
         s = O1_M + k.state;
         slot = slot_of(k.ctx);
         oi0 = k.esc;
     }
-    // ---- the window: hi, lo = the 64 bits below pos, from the pieces q and q - 1 of 8 bytes (a, b), the piece
-    // q that holds bit pos; c and d come behind
-    int32_t q = pos >> 6;
-    // pieces before the input are not loaded (a damaged stream alone gets there)
-    const int32_t qmin = -(int32_t)min((unsigned long long)(1 << 20), (unsigned long long)(ch.in >> 3));
-    auto piece = [&](int32_t p) { return p >= qmin ? __ldg(base + p) : make_uint2(0, 0); };
-    uint2 a = piece(q), b = piece(q - 1), c = piece(q - 2), d = piece(q - 3);
-    uint32_t hi, lo;
-    auto align = [&]() {
-        if (pos >> 6 != q) {  // at most one piece on
-            q--;
-            a = b;
-            b = c;
-            c = d;
-            d = piece(q - 3);
-        }
-        const bool odd = pos & 32;
-        const uint32_t x = odd ? a.y : a.x, y = odd ? a.x : b.y, z = odd ? b.y : b.x;
-        hi = __funnelshift_r(y, x, pos);
-        lo = __funnelshift_r(z, y, pos);
-    };
-    align();
+    BackWindow br;
+    const int32_t bit0 = br.init(sb, ch.in, pos);
     if (pt == 0) {
-        s = O1_M + (hi >> (32 - O1_PB));
-        pos -= O1_PB;
-        align();
+        s = O1_M + br.take(O1_PB);
+        br.align();
     }
     // ---- signs of the escapes from oi0 on: words k, k + 1 and k + 2 of the sign bits
     const unsigned long long e0 = ch.ovf + oi0;
@@ -2899,10 +2972,8 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
         else cell = __ldg(A.cells + (tab + ctx_of(slot)) * O1_M + s - O1_M);
         const uint32_t e = info[slot * kChunks + (cell & 511u)];
         const uint32_t ns = (e >> 18) + (cell >> 9), x = e & 15u, nb = 14u - x - (ns >> x);
-        s = __funnelshift_l(hi, ns, nb);  // ns << nb with the next nb bits below
-        hi = __funnelshift_l(lo, hi, nb);
-        lo <<= nb;
-        pos -= (int32_t)nb;
+        s = __funnelshift_l(br.hi, ns, nb);  // ns << nb with the next nb bits below
+        br.skip(nb);
         slot = (e >> 4) & 15u;
         if (ESC) {
             const uint32_t esc = (e >> 16) & 1u;
@@ -2922,7 +2993,7 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
     auto single = [&](uint32_t j) {
         mark(j);
         o[j] = (int16_t)(int8_t)(step(std::true_type()) >> 8);
-        align();
+        br.align();
         signs();
     };
     // codes leave in aligned groups of eight (one 16-byte store) between a scalar head and tail
@@ -2940,7 +3011,7 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
                 // bytes 1 of both, sign-extended to 16 bits
                 asm("prmt.b32 %0, %1, %2, 0xD591;" : "=r"(wv[2 * g + h]) : "r"(x), "r"(y));
             }
-            align();
+            br.align();
         }
         *reinterpret_cast<uint4 *>(o + j) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
         j += 8;
@@ -2957,10 +3028,10 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
     if (oi > avail) atomicExch(A.err, 7);
     if (!last) {
         const O1Ckpt k = A.cks[ch.ck + pt];
-        if (k.state != s - O1_M || k.ctx != ctx_of(slot) || pos != bit0 + (int32_t)k.bitpos ||
+        if (k.state != s - O1_M || k.ctx != ctx_of(slot) || br.pos != bit0 + (int32_t)k.bitpos ||
             k.esc != oi0 + oi)
             atomicExch(A.err + 1, 1);
-    } else if (pos < bit0 - 16) {
+    } else if (br.pos < bit0 - 16) {
         atomicExch(A.err, 8);
     }
 }
@@ -3348,7 +3419,9 @@ void gamma_decode(Pool &pool, const uint8_t *d, const ByteView &h,
     uint8_t *cls = pool.get<uint8_t>(T);
     BlockJob *dj = h2d(pool, jobs, st);
     enable_fse_smem();
-    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, kFseDecSmem, st>>>(d, dj, cls, d_err, fpart ? fpart : FBLK, d_fck);
+    fse::DEntry *big = pool.get<fse::DEntry>(jobs.size() << fse::kMaxTableLog);
+    const uint32_t dpart = fpart ? fpart : FBLK;
+    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, fse_dec_smem(dpart), st>>>(d, dj, cls, d_err, dpart, d_fck, big);
     FB2_CHECK_LAUNCH();
     std::vector<unsigned long long> gman(G), glen(G), ust(G + 1, 0);
     for (int g = 0; g < G; g++) {
