@@ -962,48 +962,132 @@ __global__ void k_gamma_cls(const uint32_t *__restrict__ v, long long n, uint8_t
         cls[i] = (uint8_t)(31 - __clz(v[i]));
 }
 
-__device__ __forceinline__ int find_group(const unsigned long long *gstart, int G, unsigned long long i) {
+// The values of group g, [gstart[g], gstart[g + 1]), are cut into units of kUnit from the group's start; unit u of
+// the whole list belongs to the last group g with ustart[g] <= u.  A warp sums a unit's classes (its mantissa
+// bits) and an exclusive scan of the unit sums gives every unit its first bit; a warp then packs or unpacks the
+// unit's mantissas, kRun a lane at a time.
+constexpr unsigned kUnit = 1024, kRun = 4;
+
+__device__ __forceinline__ int unit_group(const unsigned long long *__restrict__ ustart, int G, unsigned long long u) {
     int lo = 0, hi = G - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (gstart[mid] <= i) lo = mid;
+        if (ustart[mid] <= u) lo = mid;
         else hi = mid - 1;
     }
     return lo;
 }
 
-// MSB-first packing of k low bits of each value into word-aligned per-group regions (zeroed).
-__global__ void __launch_bounds__(256) k_gamma_pack(const uint32_t *__restrict__ v, const uint8_t *__restrict__ cls,
-                                                    const unsigned long long *__restrict__ boff, long long n,
-                                                    const unsigned long long *__restrict__ gstart, int G,
-                                                    const unsigned long long *__restrict__ gword,
-                                                    uint32_t *__restrict__ words) {
-    __shared__ unsigned long long s_gs[1025];  // the group starts, when there are few groups
-    const bool in_smem = G + 1 <= 1025;
-    if (in_smem)
-        for (int g = threadIdx.x; g <= G; g += blockDim.x) s_gs[g] = gstart[g];
-    __syncthreads();
-    const unsigned long long *gs = in_smem ? s_gs : gstart;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int k = cls[i];
-        if (k == 0) continue;
-        const int g = find_group(gs, G, (unsigned long long)i);
-        const unsigned long long b = boff[i] - boff[gs[g]];
-        const uint32_t m = v[i] & ((1u << k) - 1u);
-        const unsigned long long w = gword[g] + (b >> 5);
-        const int o = (int)(b & 31);
-        const unsigned long long win = (unsigned long long)m << (64 - k - o);
-        const uint32_t hi = (uint32_t)(win >> 32), lo = (uint32_t)win;
-        if (hi) atomicOr(&words[w], __byte_perm(hi, 0, 0x0123));
-        if (lo) atomicOr(&words[w + 1], __byte_perm(lo, 0, 0x0123));
+__global__ void __launch_bounds__(256) k_unit_bits(const uint8_t *__restrict__ cls,
+                                                   const unsigned long long *__restrict__ gstart,
+                                                   const unsigned long long *__restrict__ ustart, int G,
+                                                   unsigned long long nunits, unsigned long long *__restrict__ usum) {
+    const unsigned long long u = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31u;
+    if (u >= nunits) return;
+    const int g = unit_group(ustart, G, u);
+    const unsigned long long first = gstart[g] + (u - ustart[g]) * kUnit;
+    const unsigned long long end = min(first + kUnit, gstart[g + 1]);
+    uint32_t s = 0;
+    for (unsigned long long i = first + lane; i < end; i += 32) s += cls[i];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) usum[u] = s;
+}
+
+// The gamma value of an escape code, or a value itself.
+__device__ __forceinline__ uint32_t gamma_value(int16_t code) { return zigzag((int)code) + 1u; }
+__device__ __forceinline__ uint32_t gamma_value(uint32_t v) { return v; }
+
+// Bits of every group (from the scan of the unit sums) and zeros in the words where a unit starts or a group
+// ends, which neighbours share.
+__global__ void k_gamma_heads(const unsigned long long *__restrict__ uoff, const unsigned long long *__restrict__ ustart,
+                              int G, unsigned long long nunits, const unsigned long long *__restrict__ gword,
+                              unsigned long long *__restrict__ gbits, uint32_t *__restrict__ words) {
+    const unsigned long long u = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u < nunits) {
+        const int g = unit_group(ustart, G, u);
+        words[gword[g] + ((uoff[u] - uoff[ustart[g]]) >> 5)] = 0u;
+    }
+    if (u < (unsigned long long)G) {
+        const unsigned long long b = uoff[ustart[u + 1]] - uoff[ustart[u]];
+        gbits[u] = b;
+        words[gword[u] + (b >> 5)] = 0u;
     }
 }
 
-// out[i] = src[idx[i]]
-__global__ void k_pick_u64(const unsigned long long *__restrict__ src, const unsigned long long *__restrict__ idx,
-                           long long n, unsigned long long *__restrict__ out) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = src[idx[i]];
+// MSB-first packing of the mantissas (the k low bits of each value, k its class), a warp per unit: a warp scan
+// of the lanes' bit counts gives each its place, the bits are merged in shared memory and whole big-endian words
+// leave coalesced; a unit's first and last word by atomicOr.  Bound by issue: 49 M escapes take 131 us (a scan
+// over all values, then an atomicOr of every mantissa into global memory, took 530).
+constexpr int kUnitWarps = 8;
+constexpr uint32_t kUnitWords = 32 * kRun * 31 / 32 + 2;
+template <class V>
+__global__ void __launch_bounds__(kUnitWarps * 32) k_gamma_pack_units(
+    const V *__restrict__ vals, const uint8_t *__restrict__ cls, const unsigned long long *__restrict__ gstart,
+    const unsigned long long *__restrict__ ustart, int G, unsigned long long nunits,
+    const unsigned long long *__restrict__ uoff, const unsigned long long *__restrict__ gword,
+    uint32_t *__restrict__ words) {
+    __shared__ uint32_t s_buf[kUnitWarps][kUnitWords];
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const unsigned long long u = (unsigned long long)blockIdx.x * kUnitWarps + wid;
+    if (u >= nunits) return;
+    uint32_t *buf = s_buf[wid];
+    for (uint32_t z = lane; z < kUnitWords; z += 32) buf[z] = 0u;
+    const int g = unit_group(ustart, G, u);
+    const unsigned long long first = gstart[g] + (u - ustart[g]) * kUnit, end = min(first + kUnit, gstart[g + 1]);
+    const unsigned long long b0 = uoff[u] - uoff[ustart[g]];
+    uint32_t *o = words + gword[g] + (b0 >> 5);
+    uint32_t pos = (uint32_t)(b0 & 31);
+    bool shared_first = true;
+    __syncwarp();
+    for (unsigned long long i0 = first; i0 < end; i0 += 32 * kRun) {
+        const unsigned long long i = i0 + lane * kRun;
+        uint32_t k[kRun], m[kRun], sum = 0;
+#pragma unroll
+        for (unsigned j = 0; j < kRun; j++) {
+            k[j] = i + j < end ? cls[i + j] : 0u;
+            m[j] = k[j] ? gamma_value(vals[i + j]) & ((1u << k[j]) - 1u) : 0u;
+            sum += k[j];
+        }
+        const uint32_t incl = warp_incl_scan(sum);
+        uint32_t p = pos + incl - sum;
+        auto put = [&](unsigned long long v, uint32_t n) {  // the n <= 64 low bits of v
+            const unsigned long long top = v << (64 - n);
+            const uint32_t A = (uint32_t)(top >> 32), B = (uint32_t)top, w = p >> 5, sh = p & 31u, e = sh + n;
+            atomicOr(buf + w, A >> sh);
+            if (e > 32) atomicOr(buf + w + 1, __funnelshift_r(B, A, sh));
+            if (e > 64) atomicOr(buf + w + 2, __funnelshift_r(0u, B, sh));
+            p += n;
+        };
+        if (sum && sum <= 64) {
+            unsigned long long v = 0;
+#pragma unroll
+            for (unsigned j = 0; j < kRun; j++) v = (v << k[j]) | m[j];
+            put(v, sum);
+        } else if (sum) {
+#pragma unroll
+            for (unsigned j = 0; j < kRun; j++)
+                if (k[j]) put(m[j], k[j]);
+        }
+        const uint32_t tot = pos + __shfl_sync(0xffffffffu, incl, 31), full = tot >> 5;
+        __syncwarp();
+        for (uint32_t z = lane; z < full; z += 32) {
+            const uint32_t w = __byte_perm(buf[z], 0, 0x0123);
+            if (z == 0 && shared_first) atomicOr(o, w);
+            else o[z] = w;
+        }
+        __syncwarp();
+        const uint32_t rest = buf[full];
+        __syncwarp();
+        for (uint32_t z = lane; z <= full; z += 32) buf[z] = 0u;
+        __syncwarp();
+        if (lane == 0) buf[0] = rest;
+        __syncwarp();
+        shared_first = shared_first && full == 0;
+        o += full;
+        pos = tot & 31u;
+    }
+    if (lane == 0 && pos) atomicOr(o, __byte_perm(buf[0], 0, 0x0123));
 }
 
 // The FSE block coders' shared-memory limits, set once per device (a function attribute set while
@@ -1039,8 +1123,8 @@ struct GammaBlocks {
 };
 
 // `beside`: CTAs of whole SMs that run next to the class blocks (the chain encoder's).
-GammaBlocks gamma_launch(Pool &pool, const uint32_t *d_vals, const std::vector<unsigned long long> &gstart,
-                         cudaStream_t st, uint32_t ckpt_part, cudaEvent_t queued = nullptr, size_t beside = 0) {
+GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned long long> &gstart, cudaStream_t st,
+                         uint32_t ckpt_part, cudaEvent_t queued = nullptr, size_t beside = 0) {
     GammaBlocks gb;
     gb.gstart = gstart;
     const int G = (int)gstart.size() - 1;
@@ -1050,10 +1134,7 @@ GammaBlocks gamma_launch(Pool &pool, const uint32_t *d_vals, const std::vector<u
         if (queued) FB2_CUDA(cudaEventRecord(queued, st));
         return gb;
     }
-    uint8_t *cls = pool.get<uint8_t>(T);
     gb.cls = cls;
-    k_gamma_cls<<<grid_for(T, 256), 256, 0, st>>>(d_vals, T, cls);
-    FB2_CHECK_LAUNCH();
     for (int g = 0; g < G; g++) {
         for (unsigned long long b = gstart[g]; b < gstart[g + 1]; b += FBLK) {
             gb.jobs.push_back(BlockJob{b, (unsigned)std::min<unsigned long long>(FBLK, gstart[g + 1] - b), 0, 0, 0});
@@ -1095,7 +1176,8 @@ GammaBlocks gamma_launch(Pool &pool, const uint32_t *d_vals, const std::vector<u
     return gb;
 }
 
-GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const uint32_t *d_vals, cudaStream_t st) {
+template <class V>
+GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const V *d_vals, cudaStream_t st) {
     Trace tr("gamma");
     const std::vector<unsigned long long> &gstart = gb.gstart;
     const int G = (int)gstart.size() - 1;
@@ -1110,30 +1192,39 @@ GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const uint32_t *d_vals,
     out.man_bytes.assign(G, 0);
     if (T == 0) return out;
     const uint8_t *cls = gb.cls;
-    unsigned long long *boff = pool.get<unsigned long long>(T + 1);
-    void *sc = pool.get<uint8_t>(scan_scratch_bytes(T, 8));
-    exclusive_scan<uint8_t, unsigned long long>(cls, T, boff, sc, st);
-    // per-group bit totals: the scan at every group start, gathered on the device, one copy back
-    unsigned long long *d_gstart = h2d(pool, gstart, st);
-    unsigned long long *d_gb = pool.get<unsigned long long>(G + 1);
-    k_pick_u64<<<grid_for(G + 1, 256), 256, 0, st>>>(boff, d_gstart, G + 1, d_gb);
-    FB2_CHECK_LAUNCH();
-    const std::vector<unsigned long long> gbits = d2h(d_gb, (size_t)G + 1, st);
-    tr.mark("group bits known");
-    std::vector<unsigned long long> gword(G);
+    // every group's words: room for the longest mantissas (16 bits of an escape code's value, 31 of any)
+    constexpr unsigned long long kMost = sizeof(V) == 2 ? 16 : 31;
+    std::vector<unsigned long long> gword(G), ust(G + 1, 0);
     unsigned long long words = 0;
     for (int g = 0; g < G; g++) {
-        const unsigned long long bits = gbits[g + 1] - gbits[g];
-        out.man_bytes[g] = (size_t)((bits + 7) / 8);
+        const unsigned long long c = gstart[g + 1] - gstart[g];
         gword[g] = words;
-        words += (bits + 31) / 32 + 2;
+        words += (c * kMost + 31) / 32 + 2;
+        ust[g + 1] = ust[g] + (c + kUnit - 1) / kUnit;
     }
+    const unsigned long long NU = ust[G];
     uint32_t *wbuf = pool.get<uint32_t>(words + 4);
-    FB2_CUDA(cudaMemsetAsync(wbuf, 0, (words + 4) * 4, st));
+    unsigned long long *d_gstart = h2d(pool, gstart, st);
+    unsigned long long *d_ust = h2d(pool, ust, st);
     unsigned long long *d_gword = h2d(pool, gword, st);
-    k_gamma_pack<<<grid_for(T, 256, 148 * 8), 256, 0, st>>>(d_vals, cls, boff, T, d_gstart, G, d_gword, wbuf);
+    unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);
+    unsigned long long *d_gb = pool.get<unsigned long long>(G);
+    k_unit_bits<<<grid_for((long long)NU * 32, 256), 256, 0, st>>>(cls, d_gstart, d_ust, G, NU, uoff);
     FB2_CHECK_LAUNCH();
-    for (int g = 0; g < G; g++) out.man_ptr[g] = reinterpret_cast<const uint8_t *>(wbuf + gword[g]);
+    k_scan_small<unsigned long long><<<1, 1024, 0, st>>>(uoff, (long long)NU);
+    FB2_CHECK_LAUNCH();
+    k_gamma_heads<<<grid_for((long long)std::max<unsigned long long>(NU, G), 256), 256, 0, st>>>(uoff, d_ust, G, NU, d_gword,
+                                                                                                d_gb, wbuf);
+    FB2_CHECK_LAUNCH();
+    k_gamma_pack_units<V><<<(unsigned)((NU + kUnitWarps - 1) / kUnitWarps), kUnitWarps * 32, 0, st>>>(
+        d_vals, cls, d_gstart, d_ust, G, NU, uoff, d_gword, wbuf);
+    FB2_CHECK_LAUNCH();
+    const std::vector<unsigned long long> gbits = d2h(d_gb, (size_t)G, st);
+    tr.mark("group bits known");
+    for (int g = 0; g < G; g++) {
+        out.man_bytes[g] = (size_t)((gbits[g] + 7) / 8);
+        out.man_ptr[g] = reinterpret_cast<const uint8_t *>(wbuf + gword[g]);
+    }
     std::vector<unsigned long long> hs = d2h(gb.sizes, gb.jobs.size(), st);
     tr.mark("class blocks coded");
     if (gb.phase && tr.on) {
@@ -1168,7 +1259,13 @@ GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const uint32_t *d_vals,
 
 GammaOut gamma_encode(Pool &pool, const uint32_t *d_vals, const std::vector<unsigned long long> &gstart,
                       cudaStream_t st, uint32_t ckpt_part) {
-    const GammaBlocks gb = gamma_launch(pool, d_vals, gstart, st, ckpt_part);
+    const long long T = (long long)gstart.back();
+    uint8_t *cls = pool.get<uint8_t>(T);
+    if (T > 0) {
+        k_gamma_cls<<<grid_for(T, 256), 256, 0, st>>>(d_vals, T, cls);
+        FB2_CHECK_LAUNCH();
+    }
+    const GammaBlocks gb = gamma_launch(pool, cls, gstart, st, ckpt_part);
     return gamma_finish(pool, gb, d_vals, st);
 }
 
@@ -1220,43 +1317,6 @@ void add_class_pieces(Assembler &as, const GammaOut &go, int g, CkptCollector *c
         as.shadow(h, hl);
         as.dev(p.first, p.second);
     }
-}
-
-// Gamma decode of n values in index order: value i = (1 << k) | k mantissa bits (MSB first, at
-// the group's running bit offset boff), k = cls[i].  The group starts (and, when there are few
-// groups, the group tables) sit in shared memory; the mantissa bits come from at most two
-// aligned words.
-// Gamma unpacking in units of kUnit values: the values of group g, [gstart[g], gstart[g + 1]),
-// are cut into units from the group's start; unit u of the whole list belongs to the last group g
-// with ustart[g] <= u.  A warp sums a unit's classes (its mantissa bits); an exclusive scan of the
-// unit sums gives every unit its first bit; a thread then reads its unit's mantissas in order
-// (MSB-first bits of the group's byte region, one aligned word at a time).
-constexpr unsigned kUnit = 1024, kRun = 4;
-
-__device__ __forceinline__ int unit_group(const unsigned long long *__restrict__ ustart, int G, unsigned long long u) {
-    int lo = 0, hi = G - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (ustart[mid] <= u) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-__global__ void __launch_bounds__(256) k_unit_bits(const uint8_t *__restrict__ cls,
-                                                   const unsigned long long *__restrict__ gstart,
-                                                   const unsigned long long *__restrict__ ustart, int G,
-                                                   unsigned long long nunits, unsigned long long *__restrict__ usum) {
-    const unsigned long long u = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31u;
-    if (u >= nunits) return;
-    const int g = unit_group(ustart, G, u);
-    const unsigned long long first = gstart[g] + (u - ustart[g]) * kUnit;
-    const unsigned long long end = min(first + kUnit, gstart[g + 1]);
-    uint32_t s = 0;
-    for (unsigned long long i = first + lane; i < end; i += 32) s += cls[i];
-    s = __reduce_add_sync(0xffffffffu, s);
-    if (lane == 0) usum[u] = s;
 }
 
 // Escape values (zigzag + 1, gamma-coded) of every unit, a warp per unit: v[i] = (1 << k) |
@@ -3339,7 +3399,7 @@ __global__ void __launch_bounds__(256) k_esc_before(const int16_t *__restrict__ 
 
 __global__ void __launch_bounds__(kScanThreads) k_esc_extract(const int16_t *__restrict__ q, long long n,
                                                              const uint32_t *__restrict__ tile_off,
-                                                             uint32_t *__restrict__ vals, int16_t *__restrict__ raw) {
+                                                             uint8_t *__restrict__ cls, int16_t *__restrict__ raw) {
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     int16_t v[kScanItems];
     uint32_t c = 0;
@@ -3369,7 +3429,7 @@ __global__ void __launch_bounds__(kScanThreads) k_esc_extract(const int16_t *__r
     const uint32_t t0 = tile_off[blockIdx.x];
     for (uint32_t k = threadIdx.x; k < tot; k += blockDim.x) {
         const int16_t e = sv[k];
-        vals[t0 + k] = zigzag((int)e) + 1u;
+        cls[t0 + k] = (uint8_t)(31 - __clz(gamma_value(e)));
         raw[t0 + k] = e;
     }
 }
@@ -3712,17 +3772,17 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         // histogram pass and the table builds, launched above, run meanwhile)
         const std::vector<unsigned long long> gstart = d2h(d_gstart, (size_t)S + 1, es);
         const unsigned long long E = gstart[S];
-        uint32_t *evals = spool.get<uint32_t>(E + 1);
+        uint8_t *ecls = spool.get<uint8_t>(E + 1);
         int16_t *eraw = spool.get<int16_t>(E + 1);
         if (E > 0) {
-            k_esc_extract<<<(unsigned)tiles, kScanThreads, 0, es>>>(q, N, tcnt, evals, eraw);
+            k_esc_extract<<<(unsigned)tiles, kScanThreads, 0, es>>>(q, N, tcnt, ecls, eraw);
             FB2_CHECK_LAUNCH();
         }
         tr.gpu("escapes extracted", es);
         // the class blocks (long sequential chains) reach the GPU before the chain encoder, so that
         // they take a few SMs of their own instead of waiting for the chain encoder's last wave
         const bool queue_first = fork && tune.queued_ev != nullptr;
-        const GammaBlocks gblocks = gamma_launch(spool, evals, gstart, es, cc.fse_part,
+        const GammaBlocks gblocks = gamma_launch(spool, ecls, gstart, es, cc.fse_part,
                                                  queue_first ? tune.queued_ev : nullptr, cp.ctas.size());
         tr.gpu("class blocks done", es);
         if (queue_first) FB2_CUDA(cudaStreamWaitEvent(st, tune.queued_ev, 0));
@@ -3742,7 +3802,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         encode_chains(pool, cp, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
         tr.gpu("chain encoder done", st);
         tr.mark("chains launched");
-        GammaOut go = gamma_finish(spool, gblocks, evals, es);
+        GammaOut go = gamma_finish(spool, gblocks, eraw, es);
         tr.gpu("escape mantissas packed", es);
         // the chains' escape counts (stream header) from the histogram pass; their sums per segment
         // are the escape groups counted above

@@ -42,3 +42,21 @@ def test_checkpointed_blocks_of_a_field(cuda, shape):
     s.synchronize()
     assert float((y.view(shape) - x).abs().max()) <= 1e-4
     assert np.array_equal(y.cpu().numpy(), z.reshape(-1))
+
+
+@pytest.mark.parametrize("n,gap", [(5000, 3), (76801, 40), (1 << 20, 1024), (3000001, 2999999), (4096 * 40, 4096)])
+def test_runs_and_values_round_trip(cuda, n, gap):
+    """Method 0: runs of zeros of any length (mantissas up to 21 bits) beside short values."""
+    import torch
+    from falcons_b200 import device as D
+    rng = np.random.default_rng(n)
+    q = np.zeros(n, np.int16)
+    at = np.arange(gap - 1, n, gap) if gap != 3 else np.arange(0, n, 3)[::5]
+    q[at] = rng.integers(1, 30000, at.size) * rng.choice([-1, 1], at.size)
+    q = torch.from_numpy(q).to(cuda)
+    torch.cuda.synchronize()
+    enc = D.encode_codes(q)
+    back = D.decode_codes(enc, n)
+    torch.cuda.synchronize()
+    assert enc.cpu().numpy()[0] & 0x7F == 0
+    assert torch.equal(back, q)
