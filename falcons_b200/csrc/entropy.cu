@@ -1569,93 +1569,108 @@ struct SegInfo {
 
 // Per segment: the count of every (context, symbol) key of its chains (a chain's first code has
 // context 0) and every chain's escape count; writes every code's key (context << 8 | symbol) for
-// the chain encoder.  CTA (g, u) takes the u-th of gridDim.y slices of every chain of segment g
-// (slice edges on multiples of 8 codes) and adds its counts to the segment's totals, which start
-// at zero.  Codes are read 8 at a time as 16-byte vectors when q is 16-byte aligned (the
-// code before a vector comes from the lane below); runs of equal keys within a vector are counted
+// the chain encoder.  CTA (g, k + K u) takes the u-th slice of chain k of segment g (slice edges on
+// multiples of 8 codes) and adds its counts to the segment's totals, which start at zero.  Codes are
+// read 8 at a time as 16-byte vectors when q is 16-byte aligned (the code before a vector comes from
+// the lane below); runs of equal keys within a vector are counted
 // with one atomic, and the lanes of a warp spread their atomics over kHistCopies histograms.
+// Bound by issue and the shared-memory pipe (a lookup and about one atomic a code): a table of the clamped
+// code gives symbol and context in one lookup, where computing both took 60 instructions a code
+// (134 M codes: 307 us, now 196).
 constexpr int kHistCopies = 4;
-constexpr size_t kHistSmem = (size_t)kHistCopies * O1_NCTX * O1_NSYM * 4;
+constexpr int kLutSize = 257;  // codes clamped to -128 .. 128
+constexpr size_t kHistSmem = (size_t)kHistCopies * O1_NCTX * O1_NSYM * 4 + (kLutSize + 7) / 8 * 16;
 __global__ void __launch_bounds__(1024, 2) k_o1_hist(const int16_t *__restrict__ q, const SegInfo *__restrict__ segs,
                                                     uint32_t *__restrict__ hist, uint32_t *__restrict__ nvk,
                                                     uint16_t *__restrict__ keys, int vec) {
-    extern __shared__ uint32_t hs[];  // kHistCopies histograms of O1_NCTX * O1_NSYM keys
-    __shared__ uint32_t esc[kMaxK];
+    extern __shared__ uint32_t hs[];  // kHistCopies histograms of O1_NCTX * O1_NSYM keys, then the table
+    __shared__ uint32_t s_esc;
     constexpr int HN = O1_NCTX * O1_NSYM;
+    uint16_t *const lut = reinterpret_cast<uint16_t *>(hs + kHistCopies * HN);  // 0x8000 escape | context << 8 | symbol
     const SegInfo sg = segs[blockIdx.x];
-    const unsigned long long U = gridDim.y, u = blockIdx.y;
-    for (int i = threadIdx.x; i < kHistCopies * HN; i += blockDim.x) hs[i] = 0;
-    if (threadIdx.x < kMaxK) esc[threadIdx.x] = 0;
+    const unsigned long long U = gridDim.y / sg.K, u = blockIdx.y / sg.K;
+    const int k = (int)(blockIdx.y % sg.K);
+    for (int i = threadIdx.x; i < kHistCopies * HN / 4; i += blockDim.x) reinterpret_cast<uint4 *>(hs)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < kLutSize; i += blockDim.x) {
+        const int sy = o1_sym(i - 128);
+        lut[i] = (uint16_t)((sy == O1_NSYM - 1 ? 0x8000 : 0) | (o1_ctx(i - 128) << 8) | sy);
+    }
+    if (threadIdx.x == 0) s_esc = 0;
     __syncthreads();
     const unsigned lane = threadIdx.x & 31u;
     uint32_t *h = hs + (lane % kHistCopies) * HN;
-    for (int k = 0; k < sg.K; k++) {
-        const long long b = (long long)(sg.lo + (unsigned long long)k * sg.cs);
-        const long long e = (long long)(sg.lo + min((unsigned long long)k * sg.cs + sg.cs, sg.n));
-        if (e <= b) continue;
-        // this CTA's slice [sb, se) of the chain [b, e)
-        const unsigned long long len = (unsigned long long)(e - b);
-        auto edge = [&](unsigned long long v) -> long long {
-            if (v == 0) return b;
-            if (v >= U) return e;
-            const long long x = (b + (long long)(len * v / U) + 7) & ~7LL;
-            return x < e ? x : e;
-        };
-        const long long sb = edge(u), se = edge(u + 1);
-        if (se <= sb) continue;
-        // codes [sb, hb) and [tb, se) one per thread, whole vectors [hb, tb) one per thread
-        long long hb = se, tb = se;
-        if (vec) {
-            hb = min(se, (sb + 7) & ~7LL);
-            tb = max(hb, se & ~7LL);
-        }
-        uint32_t ne = 0;
-        const long long nh = hb - sb, nt = se - tb;
-        for (long long j = threadIdx.x; j < nh + nt; j += blockDim.x) {
-            const long long i = j < nh ? sb + j : tb + (j - nh);
-            const int prev = i == b ? 0 : (int)q[i - 1];
-            const int sy = o1_sym((int)q[i]);
-            const uint32_t key = (uint32_t)(o1_ctx(prev) << 8) | (uint32_t)sy;
-            atomicAdd(&h[key], 1u);
-            keys[i] = (uint16_t)key;
-            ne += sy == O1_NSYM - 1;
-        }
-        const long long v0 = hb >> 3, v1 = tb >> 3;
-        const uint4 *q4 = reinterpret_cast<const uint4 *>(q);
-        uint4 *k4 = reinterpret_cast<uint4 *>(keys);
-        for (long long vb = v0 + (threadIdx.x & ~31u); vb < v1; vb += blockDim.x) {  // warp-uniform
-            const long long vi = vb + lane;
-            const bool act = vi < v1;
-            const uint4 w = act ? __ldg(q4 + vi) : make_uint4(0, 0, 0, 0);
-            const uint32_t below = __shfl_up_sync(0xffffffffu, w.w >> 16, 1);
-            if (!act) continue;
-            int prev = 0;  // the code before this vector (context 0 at the chain's start)
-            if (vi * 8 > b) prev = (lane && vi > v0) ? (int)(int16_t)below : (int)q[vi * 8 - 1];
-            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-            uint32_t kk[8];
-            uint32_t rkey = ~0u, rn = 0;
-#pragma unroll
-            for (int m = 0; m < 8; m++) {
-                const int code = (int)(int16_t)(ww[m >> 1] >> (16 * (m & 1)));
-                const int sy = o1_sym(code);
-                const uint32_t key = (uint32_t)(o1_ctx(prev) << 8) | (uint32_t)sy;
-                kk[m] = key;
-                ne += sy == O1_NSYM - 1;
-                if (key == rkey) {
-                    rn++;
-                } else {
-                    if (rn) atomicAdd(&h[rkey], rn);
-                    rkey = key;
-                    rn = 1;
-                }
-                prev = code;
-            }
-            atomicAdd(&h[rkey], rn);
-            k4[vi] = make_uint4(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16), kk[4] | (kk[5] << 16), kk[6] | (kk[7] << 16));
-        }
-        ne = __reduce_add_sync(0xffffffffu, ne);
-        if (lane == 0 && ne) atomicAdd(&esc[k], ne);
+    auto entry = [&](int code) -> uint32_t { return lut[min(max(code, -128), 128) + 128]; };
+    // the key of a code from its own entry and that of the code before it
+    auto key_of = [](uint32_t before, uint32_t e) -> uint32_t { return (before & 0xF00u) | (e & 0xFFu); };
+    const long long b = (long long)(sg.lo + (unsigned long long)k * sg.cs);
+    const long long e = (long long)(sg.lo + min((unsigned long long)k * sg.cs + sg.cs, sg.n));
+    if (e <= b) return;
+    // this CTA's slice [sb, se) of the chain [b, e)
+    const unsigned long long len = (unsigned long long)(e - b);
+    auto edge = [&](unsigned long long v) -> long long {
+        if (v == 0) return b;
+        if (v >= U) return e;
+        const long long x = (b + (long long)(len * v / U) + 7) & ~7LL;
+        return x < e ? x : e;
+    };
+    const long long sb = edge(u), se = edge(u + 1);
+    if (se <= sb) return;
+    // codes [sb, hb) and [tb, se) one per thread, whole vectors [hb, tb) one per thread
+    long long hb = se, tb = se;
+    if (vec) {
+        hb = min(se, (sb + 7) & ~7LL);
+        tb = max(hb, se & ~7LL);
     }
+    uint32_t ne = 0;
+    const long long nh = hb - sb, nt = se - tb;
+    for (long long j = threadIdx.x; j < nh + nt; j += blockDim.x) {
+        const long long i = j < nh ? sb + j : tb + (j - nh);
+        const uint32_t c = entry((int)q[i]), key = key_of(i == b ? 0u : entry((int)q[i - 1]), c);
+        atomicAdd(&h[key], 1u);
+        keys[i] = (uint16_t)key;
+        ne += c >> 15;
+    }
+    const uint32_t nv = (uint32_t)((tb >> 3) - (hb >> 3));
+    const uint4 *const q4 = reinterpret_cast<const uint4 *>(q) + (hb >> 3);
+    uint4 *const k4 = reinterpret_cast<uint4 *>(keys) + (hb >> 3);
+    const bool first = hb == b;  // the first vector starts the chain (context 0)
+    for (uint32_t vb = threadIdx.x & ~31u; vb < nv; vb += blockDim.x) {  // warp-uniform
+        const uint32_t vi = vb + lane;
+        const bool act = vi < nv;
+        const uint4 w = act ? __ldg(q4 + vi) : make_uint4(0, 0, 0, 0);
+        const uint32_t below = __shfl_up_sync(0xffffffffu, w.w >> 16, 1);
+        if (!act) continue;
+        int prev = (int)(int16_t)below;  // the code before this vector
+        if (lane == 0) prev = vi == 0 && first ? 0 : (int)reinterpret_cast<const int16_t *>(q4 + vi)[-1];
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+        uint32_t ent[8], kk[8];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            // two codes clamped to -128 .. 128 and biased to 0 .. 256 (no borrow between the halves)
+            const uint32_t t = (__vmins2(__vmaxs2(ww[m], 0xFF80FF80u), 0x00800080u) ^ 0x80008000u) - 0x7F807F80u;
+            ent[2 * m] = lut[t & 0xFFFFu];
+            ent[2 * m + 1] = lut[t >> 16];
+        }
+        uint32_t before = entry(prev), flags = 0;
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            kk[m] = key_of(before, ent[m]);
+            before = ent[m];
+            flags += ent[m] >> 15;
+        }
+        ne += flags;
+        uint32_t rn = 1;
+#pragma unroll
+        for (int m = 1; m < 8; m++) {
+            const bool same = kk[m] == kk[m - 1];
+            if (!same) atomicAdd(&h[kk[m - 1]], rn);
+            rn = same ? rn + 1 : 1;
+        }
+        atomicAdd(&h[kk[7]], rn);
+        k4[vi] = make_uint4(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16), kk[4] | (kk[5] << 16), kk[6] | (kk[7] << 16));
+    }
+    ne = __reduce_add_sync(0xffffffffu, ne);
+    if (lane == 0 && ne) atomicAdd(&s_esc, ne);
     __syncthreads();
     uint32_t *gh = hist + (size_t)blockIdx.x * HN;
     for (int i = threadIdx.x; i < HN; i += blockDim.x) {
@@ -1664,7 +1679,7 @@ __global__ void __launch_bounds__(1024, 2) k_o1_hist(const int16_t *__restrict__
         for (int c = 0; c < kHistCopies; c++) v += hs[c * HN + i];
         if (v) atomicAdd(gh + i, v);
     }
-    if (threadIdx.x < kMaxK && esc[threadIdx.x]) atomicAdd(nvk + blockIdx.x * kMaxK + threadIdx.x, esc[threadIdx.x]);
+    if (threadIdx.x == 0 && s_esc) atomicAdd(nvk + blockIdx.x * kMaxK + k, s_esc);
 }
 
 // Keeps every m-th decode checkpoint of every chain (the m-th, 2m-th, ... of chain c's
@@ -2106,7 +2121,7 @@ struct ChainCta {
 // tables beside 13 packed ones cost every warp both paths); two words per key hold the symbol
 // transform (one word fits too, but takes a dozen more instructions a code to unpack).  k_o1_ctable lays this image out once per table set; every CTA copies it in.
 constexpr int kEncThreads = 1024;
-constexpr uint32_t kEncWarps = 4, kMinEncPart = 256;
+constexpr uint32_t kEncWarps = 4, kMinEncPart = 512;
 constexpr int kKeptShift = 6;  // kept states: every 64th index
 
 // Parts [first, first + count) of one table set: warp w codes the parts first + w * lanes + l, l < lanes.
@@ -3641,8 +3656,9 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         SegInfo *d_segs = h2d(pool, segs, st);
         // encoder part size, a power of two up to the decode checkpoint spacing: a chain's parts fit one
         // CTA's threads, and a part is shorter than the spacing where the parts would not give every SM
-        // four full warps (a walk's time is then the length of a part: 67 us for 64^3 codes in parts of 1024, 26 us in parts of 256), but not so short
-        // that a run seldom meets the kept states within it
+        // four full warps (a walk's time is then the length of a part: 64^3 codes 67 us in parts of 1024,
+        // 38 in parts of 512), but not so short that a run seldom meets the kept states within it (parts of
+        // 256: a walk of 25 us, but the rounds after it took 44 instead of 29, and a mean step the same)
         unsigned long long max_cs = 1;
         for (const auto &sg : segs) max_cs = std::max<unsigned long long>(max_cs, sg.cs);
         auto parts_of = [&](uint32_t part) { return (max_cs + part - 1) / part; };
@@ -3721,10 +3737,15 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         enable_big_smem();
         tr.gpu("histogram start", st);
         {
-            // about four CTAs per SM over all segments, a slice at least 64 Ki codes long
-            const long long want = (4LL * 148 + S - 1) / S;
-            const long long U = std::max<long long>(1, std::min<long long>(want, (seg + 65535) / 65536));
-            k_o1_hist<<<dim3((unsigned)S, (unsigned)U), 1024, kHistSmem, st>>>(
+            // slices of a chain: at least 16 Ki codes (clearing and adding up its histogram costs a CTA as much
+            // as 8 Ki codes), 4 Ki where the chains would leave SMs idle, and at most as many as fill whole waves
+            // of two CTAs an SM, five at most.  (A CTA for every slice of all 16 chains had each chain's 1024 or
+            // so codes a trip of their own: 1800 x 3600 points 41 us, now 18; 64^3 38, now 7.)
+            const long long chains = S * K, wave = 2ll * sm_count();
+            long long U = std::max<long long>(1, (long long)max_cs / 16384);
+            while (chains * U < sm_count() && (long long)max_cs / U > 4096) U *= 2;
+            if (chains * U > wave) U = std::max<long long>(1, std::min<long long>(5, chains * U / wave) * wave / chains);
+            k_o1_hist<<<dim3((unsigned)S, (unsigned)(K * U)), 1024, kHistSmem, st>>>(
                 q, d_segs, hist, nvk, keys, (reinterpret_cast<uintptr_t>(q) & 15) == 0);
         }
         FB2_CHECK_LAUNCH();
