@@ -89,63 +89,65 @@ __host__ __device__ __forceinline__ uint32_t fse_ckpt_count(uint32_t n, uint32_t
     return n >= 3 ? (n - 3) / part : 0;
 }
 
-// FSE class block encoder (zfse/fse_compress.c FSE_compress), one group of 256 threads per 64
-// Ki-symbol block (four groups per CTA, below), the largest blocks first.  The group counts the
+// FSE class block encoder (zfse/fse_compress.c FSE_compress), one group of 128 threads per 64
+// Ki-symbol block (eight groups per CTA, below), the largest blocks first.  The group counts the
 // block; its thread 0 normalizes and writes the table header; the group builds the coding tables
-// in shared memory (the state table with warp match ranks, the symbol transforms per symbol, and,
-// where it fits, the next-state table); two warps then code the two state chains (symbols n-3 .. 0,
-// each coded by the state of its index parity) side by side, recording for every symbol only the
-// state before it (the emitted bits are its low bits, their count follows from the state and the
-// symbol); the group then packs in parallel: a scan of the bit counts gives every symbol its bit
-// position, each thread writes the bits of one run of symbols (words shared with a neighbour
-// merged with atomicOr), and thread 0 appends the two final states and the end mark.  (The
-// chains of these skewed class streams converge too slowly for a speculative split.)  Writes the
-// complete fse_enc record ([1][u32 len][data] | [0][raw] | [2][sym]) to the block's slot; the
-// record flag goes into bits 56-63 of `sizes`.  `recs` is scratch of kFseRecWords words per block
-// (the 16-bit step records of both chains).
+// in shared memory (the state table with warp match ranks, the symbol transforms per symbol, the
+// step rows); two lanes of one warp then code the two state chains (symbols n-3 .. 0, each coded by
+// the state of its index parity) side by side, recording every state with the bits that led to it;
+// the group then packs in parallel: warps sum the bits of units of positions, a scan gives every
+// unit its bit position, and the warps write the units (words shared with a neighbour merged with
+// atomicOr); thread 0 appends the two final states and the end mark.  (The chains of these skewed
+// class streams converge too slowly for a speculative split.)  Writes the complete fse_enc record
+// ([1][u32 len][data] | [0][raw] | [2][sym]) to the block's slot; the record flag goes into bits
+// 56-63 of `sizes`.  `recs` is scratch of kFseRecWords words per block (the 16-bit step records of
+// both chains).
 constexpr unsigned kFseMaxLog = 11;               // the block coder's table log never exceeds 11
-// Next-state table of the chains (dynamic shared memory): for every symbol s from the smallest
-// to the largest present one and every state x, twice the coded state minus L, which is the byte
-// offset of that state in a table row, so that a chain step is one add and one table load.
-// Blocks whose table would not fit (symbol span x L x 2 bytes) take the state-table path.
-constexpr size_t kFseNxtBytes = 40 * 1024;
-// Per-chain record scratch (16-bit records): a chain's records are indexed by step plus the
-// chain's lead (the steps that its first 16-byte symbol word holds above the chain's start).
+// Step rows: for every symbol, the next state and the emitted bits by state >> b, where b is the
+// smaller of the symbol's two bit counts (the states from which it emits b + 1 start at a multiple
+// of 2^(b + 1)).  A row has at most twice the symbol's cells, so all rows together fit 2 L entries.
+// (A row of all L states a symbol saves the shift, but takes 40 KB for ten symbols, so that only four
+// blocks fitted an SM: 758 blocks in two waves, 2.23 ms, now 1.05.)
+constexpr unsigned kFseRows = 2u << kFseMaxLog;
+// Records per chain: every state (times 16, plus the bits emitted on the way to it), the last one too.
 constexpr unsigned kFseChainRec = FBLK / 2 + 32;
 constexpr unsigned kFseRecWords = kFseChainRec;  // both chains, 2 records per word
-// The packer's chunk of emission positions and its word buffer (the chunk's bits, at most
-// kFseMaxLog per position, plus the partial word in front and one behind), staged with its records,
-// symbols and slice offsets in the next-state table's space.
-constexpr unsigned kPackChunk = 8192;
-constexpr unsigned kStageBatch = 16;  // loads a thread has in flight while staging a chunk
-constexpr unsigned kPackWords = kPackChunk * kFseMaxLog / 32 + 2;
-static_assert(kPackChunk * 3 + (kPackWords + kPackChunk / 32 + 1) * 4 <= kFseNxtBytes,
-              "the packer's staging fits the next-state table's space");
-static_assert(kPackChunk % 1024 == 0, "one warp scans the chunk's slices, a whole number per lane");
-static_assert(kFseChainRec % 8 == 0, "records of whole symbol words are stored as 16-byte vectors");
-struct FseSmem {
+static_assert(kFseChainRec % 8 == 0, "records are moved as 16-byte vectors");
+constexpr unsigned kFseBatch = 256;              // steps of a chain staged at a time, eight a lane and chain
+constexpr unsigned kPackUnit = 512;              // emission positions a warp packs at a time, 16 a lane
+constexpr unsigned kPackWords = (kPackUnit * kFseMaxLog + 31) / 32 + 1;
+// A CTA codes G blocks side by side, one group of kFseGroupThreads threads each, with its own
+// shared memory and its own named barrier.  G = 1 when the blocks and the chain encoder's CTAs
+// together fit the SMs (a block alone on an SM codes fastest); G = kFseGroups otherwise: the CTA
+// fills an SM (registers), so the blocks sit on an eighth as many SMs as one CTA per block would
+// spread over, and the chain encoder launched beside them keeps the other SMs.
+constexpr unsigned kFseGroups = 8, kFseGroupThreads = 128, kFseGroupWarps = kFseGroupThreads / 32;
+constexpr unsigned kCountCopies = 8;  // histograms of the count, interleaved
+struct FseGroupSmem {
+    union {
+        uint16_t row[kFseRows];
+        uint32_t copies[256 * kCountCopies];         // while the block is counted
+        uint32_t pack[kFseGroupWarps][kPackWords];   // after the walk: a warp's unit in words
+    };
+    union {
+        uint4 ring[2][kFseBatch / 4 + 1];            // the chains' steps of a batch
+        uint32_t unit[FBLK / kPackUnit];             // after the walk: bits before a unit
+    };
     uint32_t count[256];
     uint32_t cumul[257];
-    uint32_t scan[256];
+    uint32_t scan[257];
+    uint32_t step[256];  // of a symbol: its row's shared-memory address << 5 | b + 4
     fse::SymTT sym_tt[256];
     int16_t norm[256];
     uint16_t state_table[1 << kFseMaxLog];
     uint8_t sym[1 << kFseMaxLog];
-};
-// A CTA codes G blocks side by side, one group of kFseGroupThreads threads each, with its own
-// shared memory and its own named barrier.  G = 1 when the blocks and the chain encoder's CTAs
-// together fit the SMs (a block alone on an SM codes fastest); G = kFseGroups otherwise: the CTA
-// fills an SM (registers), so the blocks sit on a quarter as many SMs as one CTA per block would
-// spread over, and the chain encoder launched beside them keeps the other SMs.
-constexpr unsigned kFseGroups = 4, kFseGroupThreads = 256;
-struct FseGroupSmem {
-    FseSmem w;
     int mode;
-    unsigned tl, hdr, s0, s1, maxsv, i0, i1, minsv, fast, high;
-    unsigned lead[2];
+    unsigned tl, hdr, fin[2], maxsv, high, bits;
     uint32_t sh[32];
-    unsigned long long tend[2];  // traced calls: when each chain walk ended
+    unsigned long long tend;  // traced calls: when the walk ended
 };
+static_assert(sizeof(uint32_t) * 256 * kCountCopies <= sizeof(uint16_t) * kFseRows &&
+              sizeof(uint32_t) * kFseGroupWarps * kPackWords <= sizeof(uint16_t) * kFseRows, "in the rows' space");
 
 // A group's barrier.  bar.sync counts whole warps, so the warp is made convergent first (after
 // code where some lanes ran on alone, such as the two chain lanes).
@@ -187,65 +189,66 @@ __device__ __forceinline__ uint32_t group_excl_scan(uint32_t v, uint32_t *sh, ui
 }
 
 template <unsigned G>
-__global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
+__global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
     k_fse_encode_blocks(const uint8_t *__restrict__ cls, const BlockJob *__restrict__ jobs, unsigned njobs,
                         uint8_t *__restrict__ slots, unsigned long long *__restrict__ sizes,
                         uint8_t *__restrict__ scratch, uint32_t part, FseCkpt *__restrict__ cks,
-                        uint32_t *__restrict__ recs, const uint32_t *__restrict__ order,
+                        uint32_t *recs, const uint32_t *__restrict__ order,
                         unsigned long long *__restrict__ phase) {
-    __shared__ FseGroupSmem groups[G];
-    extern __shared__ uint4 s_nxt_all[];  // the groups' next-state tables (kFseNxtBytes each)
+    extern __shared__ uint4 s_groups[];  // G groups' FseGroupSmem
     const unsigned grp = threadIdx.x / kFseGroupThreads, tid = threadIdx.x % kFseGroupThreads;
+    const unsigned lane = tid & 31u, wid = tid >> 5;
     const unsigned slot = blockIdx.x * G + grp;
     if (slot >= njobs) return;  // the other groups synchronise on barriers of their own
     const unsigned bar = 1 + grp;  // named barrier of this group (0 is the CTA's)
-    FseGroupSmem &gm = groups[grp];
-    FseSmem &w = gm.w;
-    uint4 *s_nxt4 = s_nxt_all + (size_t)grp * (kFseNxtBytes / 16);
-    int &s_mode = gm.mode;  // 0 raw, 1 RLE, 2 FSE
-    unsigned &s_tl = gm.tl, &s_hdr = gm.hdr, &s_s0 = gm.s0, &s_s1 = gm.s1, &s_maxsv = gm.maxsv, &s_i0 = gm.i0,
-             &s_i1 = gm.i1, &s_minsv = gm.minsv, &s_fast = gm.fast, &s_high = gm.high;
-    unsigned *s_lead = gm.lead;
-    uint32_t *s_sh = gm.sh;
+    FseGroupSmem &w = reinterpret_cast<FseGroupSmem *>(s_groups)[grp];
     const unsigned b = order[slot];  // the largest blocks first
     if (tid == 0) fse_phase(phase, slot, 0);
     const BlockJob jb = jobs[b];
     const uint8_t *src = cls + jb.src;
     uint8_t *out = slots + (size_t)b * kBlockSlot;
     uint32_t *bw = reinterpret_cast<uint32_t *>(scratch + (size_t)b * kBlockSlot);
-    uint32_t *rec = recs + (size_t)b * kFseRecWords;
+    uint16_t *rec = reinterpret_cast<uint16_t *>(recs + (size_t)b * kFseRecWords);
     FseCkpt *ck = cks ? cks + (size_t)b * (FBLK / part) : nullptr;
     const unsigned n = jb.n;
-    for (int s = tid; s < 256; s += kFseGroupThreads) w.count[s] = 0;
+    // the block in aligned 16-byte words (the pool's allocations are 16-byte aligned with slack behind them)
+    const unsigned lead = (unsigned)(jb.src & 15u);
+    const uint4 *g4 = reinterpret_cast<const uint4 *>(src - lead);
+    for (unsigned s = tid; s < 256 * kCountCopies; s += kFseGroupThreads) w.copies[s] = 0;
     group_sync(bar);
-    // Count the symbols: every thread reads a contiguous run of aligned 16-byte words (the pool's
-    // allocations are 16-byte aligned with slack behind them) and adds runs of equal symbols with
-    // one atomic (the class streams are dominated by a few symbols).
+    // Count the symbols: runs of equal symbols within a word are added with one atomic, and neighbouring
+    // lanes add to copies of their own, in banks of their own (a few symbols dominate the class streams).
     {
-        const unsigned lead = (unsigned)(jb.src & 15u);
-        const uint4 *g4 = reinterpret_cast<const uint4 *>(src - lead);
-        const unsigned nw = (lead + n + 15) / 16, per = (nw + kFseGroupThreads - 1) / kFseGroupThreads;
-        const unsigned w0 = min(nw, tid * per), cnt = min(nw, w0 + per) - w0;
-        unsigned cur = 256, run = 0;
-        for (unsigned j = 0; j < cnt; j++) {
-            const unsigned wi = w0 + j;
-            const uint4 v = g4[wi];
+        const unsigned nw = (lead + n + 15) / 16;
+        uint32_t *h = w.copies + (lane % kCountCopies);
+        uint4 v = tid < nw ? g4[tid] : make_uint4(0, 0, 0, 0);
+        for (unsigned wi = tid; wi < nw; wi += kFseGroupThreads) {
+            const uint4 c = v;
+            if (wi + kFseGroupThreads < nw) v = g4[wi + kFseGroupThreads];
+            // the word's bytes [t0, t1) belong to the block
+            const unsigned t0 = wi ? 0u : lead, t1 = min(16u, lead + n - wi * 16);
+            unsigned cur = 0, run = 0;
 #pragma unroll
-            for (int h = 0; h < 16; h++) {
-                const unsigned bi = wi * 16 + h;
-                if (bi < lead || bi >= lead + n) continue;
-                const uint32_t qw = h < 4 ? v.x : h < 8 ? v.y : h < 12 ? v.z : v.w;
-                const unsigned sy = (qw >> ((h & 3) * 8)) & 0xFFu;
-                if (sy == cur) {
-                    run++;
-                } else {
-                    if (run) atomicAdd(&w.count[cur], run);
-                    cur = sy;
-                    run = 1;
+            for (unsigned t = 0; t < 16; t++) {
+                if (t < t0 || t >= t1) continue;
+                const uint32_t q = t < 4 ? c.x : t < 8 ? c.y : t < 12 ? c.z : c.w;
+                const unsigned sy = (q >> ((t & 3) * 8)) & 0xFFu;
+                if (run && sy != cur) {
+                    atomicAdd(h + cur * kCountCopies, run);
+                    run = 0;
                 }
+                cur = sy;
+                run++;
             }
+            atomicAdd(h + cur * kCountCopies, run);
         }
-        if (run) atomicAdd(&w.count[cur], run);
+    }
+    group_sync(bar);
+    for (unsigned s = tid; s < 256; s += kFseGroupThreads) {
+        uint32_t v = 0;
+#pragma unroll
+        for (unsigned c = 0; c < kCountCopies; c++) v += w.copies[s * kCountCopies + c];
+        w.count[s] = v;
     }
     group_sync(bar);
     if (tid == 0) fse_phase(phase, slot, 1);
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
                         else if (w.norm[s2] == -1) w.sym[high--] = (uint8_t)s2;
                     }
                     w.scan[maxSV + 1] = c;
-                    s_high = high;
+                    w.high = high;
                     if (hdr && c == high + 1) {
                         mode = 2;
                         w.cumul[0] = 0;
@@ -281,24 +284,24 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
                 }
             }
         }
-        s_mode = mode;
-        s_tl = tl;
-        s_hdr = hdr;
-        s_maxsv = maxSV;
+        w.mode = mode;
+        w.tl = tl;
+        w.hdr = hdr;
+        w.maxsv = maxSV;
     }
     group_sync(bar);
     if (tid == 0) fse_phase(phase, slot, 2);
-    if (s_mode == 2) {
-        const unsigned tl = s_tl, L = 1u << tl, maxSV = s_maxsv;
+    if (w.mode == 2) {
+        const unsigned tl = w.tl, L = 1u << tl, maxSV = w.maxsv;
         {
             // parallel spread: thread t ranks the kept positions of j in [t * per, (t + 1) * per)
-            const uint32_t step = fse::table_step(L), mask = L - 1, high = s_high;
+            const uint32_t step = fse::table_step(L), mask = L - 1, high = w.high;
             const unsigned per = (L + kFseGroupThreads - 1) / kFseGroupThreads;
             const unsigned j0 = min(L, tid * per), j1 = min(L, j0 + per);
             uint32_t cnt = 0;
             for (unsigned j = j0; j < j1; j++) cnt += ((j * step) & mask) <= high;
             uint32_t tot;
-            uint32_t kc = group_excl_scan(cnt, s_sh, tot, tid, bar);
+            uint32_t kc = group_excl_scan(cnt, w.sh, tot, tid, bar);
             unsigned sy = 0;  // the symbol of cell kc: the last one whose first cell is <= kc
             for (unsigned lo = 0, hi = maxSV + 1; hi - lo > 1;) {
                 const unsigned mid = (lo + hi) >> 1;
@@ -316,8 +319,7 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
             group_sync(bar);
         }
         // state table: the cells of every symbol in increasing order (match ranks within a warp)
-        if (tid < 32) {
-            const unsigned lane = tid;
+        if (wid == 0) {
             for (unsigned u0 = 0; u0 < L; u0 += 32) {
                 const unsigned u = u0 + lane;
                 const unsigned sy = u < L ? w.sym[u] : 256u + lane;
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
             const int nn = w.norm[sy];
             uint32_t total = 0;  // cells of the symbols before sy
             for (unsigned s2 = 0; s2 < sy; s2++) total += w.norm[s2] == -1 ? 1u : (uint32_t)max(0, (int)w.norm[s2]);
+            uint32_t low = tl;  // the smaller of the symbol's bit counts
             if (nn == 0) {
                 w.sym_tt[sy].deltaNbBits = ((tl + 1) << 16) - L;
                 w.sym_tt[sy].deltaFindState = 0;
@@ -344,278 +347,249 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
                 const uint32_t minStatePlus = (uint32_t)nn << maxBitsOut;
                 w.sym_tt[sy].deltaNbBits = (maxBitsOut << 16) - minStatePlus;
                 w.sym_tt[sy].deltaFindState = (int32_t)total - nn;
+                low = maxBitsOut - 1;
+            }
+            // the row starts at twice the cells before it (a row of L >> low entries has at most twice its cells)
+            w.step[sy] = (((uint32_t)__cvta_generic_to_shared(w.row) + 4 * min(total, L - 1)) << 5) | (low + 4);
+        }
+        group_sync(bar);
+        for (unsigned sy = 0; sy <= maxSV; sy++) {
+            if (w.norm[sy] == 0) continue;
+            const unsigned low = (w.step[sy] & 31u) - 4;
+            uint16_t *row = w.row + ((w.step[sy] >> 5) - (uint32_t)__cvta_generic_to_shared(w.row)) / 2;
+            const fse::SymTT t = w.sym_tt[sy];
+            for (unsigned c = tid; c < L >> low; c += kFseGroupThreads) {
+                const uint32_t x = L + (c << low), nb = (x + t.deltaNbBits) >> 16;
+                row[c] = (uint16_t)((w.state_table[(int32_t)(x >> nb) + t.deltaFindState] - L) << 4 | nb);
             }
         }
         group_sync(bar);
-        if (tid == 0) {
-            unsigned lo = 0;
-            while (lo < maxSV && w.count[lo] == 0) lo++;
-            s_minsv = lo;
-            s_fast = (size_t)(maxSV - lo + 1) * L * 2 <= kFseNxtBytes;
-        }
-        group_sync(bar);
-        uint16_t *nxt = reinterpret_cast<uint16_t *>(s_nxt4);
-        const unsigned minSV = s_minsv;
-        const bool fast = s_fast != 0;
-        if (fast) {
-            for (unsigned e = tid; e < (maxSV - minSV + 1) * L; e += kFseGroupThreads) {
-                const unsigned sy = minSV + (e >> tl), x = L + (e & (L - 1));
-                if (!w.count[sy]) continue;
-                const fse::SymTT t = w.sym_tt[sy];
-                const uint32_t nb = (x + t.deltaNbBits) >> 16;
-                nxt[e] = (uint16_t)((w.state_table[(int32_t)(x >> nb) + t.deltaFindState] - L) << 1);
-            }
-            group_sync(bar);
-        }
-        // The chains run on the group's warps cw, cw + 1, chosen so that the CTA's eight chain warps
-        // sit two on each SM sub-partition (warp w of a CTA issues from sub-partition w mod 4).
-        const unsigned cw = (2u * grp) & 3u;
         if (tid == 0) fse_phase(phase, slot, 3);
-        if ((tid & 31u) == 0 && (tid >> 5) - cw < 2u) {
-            // The two state chains, one per warp: chain k codes the symbols i <= n - 3 of parity k
-            // from the top down (step j codes symbol top - 2 j), starting from the state that
-            // symbol n-1 or n-2 (of parity k) initialised.  Each step records twice the state
-            // before it minus L (16 bits, table log <= 11): its low bits are the emitted ones, and
-            // the record of the chain's next step holds the state after it.
-            const unsigned k = (tid >> 5) - cw;
-            uint32_t v;  // the state minus L
-            {
-                const unsigned i0 = ((n - 1) % 2 == k) ? n - 1 : n - 2;
-                const fse::SymTT t = w.sym_tt[src[i0]];
+        const unsigned ns = n - 2;  // emission position e codes symbol n - 3 - e, even positions by chain 0
+        // The chains run on a warp that puts a CTA's eight two on each SM sub-partition (warp w of a CTA
+        // issues from sub-partition w mod 4).
+        if (wid == (grp & 3u)) {
+            // Lane c < 2 codes chain c: the symbols n - 3 - c, n - 5 - c, .., starting from the state that
+            // symbol n - 1 - c initialised.  A record is the state minus L, times 16, plus the bits that the
+            // step to it emitted; a step shifts it down, adds the symbol's row and loads the next record.  What
+            // a step needs of its symbol is laid out by the whole warp for kFseBatch steps at a time, its
+            // symbols loaded a batch ahead, so that little but the chain itself is left to the two lanes: a
+            // step waits for two additions and one load (22.5 ns; with the symbols unpacked by the chain's own
+            // lane, 26).
+            const unsigned m = lane < 2 ? (ns + 1 - lane) / 2 : 0;  // steps
+            uint16_t *rk = rec + (lane & 1u) * kFseChainRec;
+            uint32_t e = 0;
+            if (lane < 2) {
+                const fse::SymTT t = w.sym_tt[src[n - 1 - lane]];
                 const uint32_t nb = (t.deltaNbBits + (1u << 15)) >> 16;
                 const uint32_t u = (nb << 16) - t.deltaNbBits;
-                v = w.state_table[(int32_t)(u >> nb) + t.deltaFindState] - L;
+                e = (w.state_table[(int32_t)(u >> nb) + t.deltaFindState] - L) << 4;
             }
-            // the decoder's states before symbols n-3 and n-4 (for checkpoints next to them)
-            if (k == 0) s_i0 = v;
-            else s_i1 = v;
-            const int top = (int)n - 3 - (int)(((n - 3) & 1u) != k);
-            const unsigned m = top >= 0 ? (unsigned)top / 2 + 1 : 0;  // steps
-            uint16_t *rk = reinterpret_cast<uint16_t *>(rec) + k * kFseChainRec;
-            unsigned lead = 0;
-            if (fast && m > 0) {
-                // The chain's symbols are every other byte of the aligned 16-byte words from the one
-                // holding symbol `top` down: eight steps per word (whole words loaded three words
-                // ahead), the first word holding `lead` steps above the chain's start.  A step is
-                // one add and one load from the next-state table (its entries and the row offsets
-                // are byte offsets); the records of a whole word leave as one 16-byte store.
-                const uintptr_t a0 = reinterpret_cast<uintptr_t>(src + top);
-                const unsigned par = (unsigned)(a0 & 1u), sh = 8u * par;
-                lead = (14u + par - (unsigned)(a0 & 15u)) >> 1;
-                const unsigned nv = lead + m;
-                const uint4 *wp = reinterpret_cast<const uint4 *>(a0 & ~(uintptr_t)15);  // word g at wp - g
-                // shared memory: the row of symbol s at byte (s - minSV) << (tl + 1)
-                const unsigned char *tb = reinterpret_cast<const unsigned char *>(nxt);
-                const unsigned rsh = tl + 1;
-                auto step = [&](uint32_t o, uint32_t v2) -> uint32_t {
-                    return *reinterpret_cast<const uint16_t *>(tb + o + v2);
-                };
-                // the chain's bytes of a word at even offsets 14, 12, .., 0 (descending steps), as the
-                // byte offsets of their rows in the next-state table
-                auto offsets = [&](const uint4 &q, uint32_t *o) {
-                    const uint32_t h0 = __funnelshift_r(q.x, q.y, sh), h1 = __funnelshift_r(q.y, q.z, sh);
-                    const uint32_t h2 = __funnelshift_r(q.z, q.w, sh), h3 = q.w >> sh;
-                    o[0] = (((h3 >> 16) & 0xFFu) - minSV) << rsh;
-                    o[1] = ((h3 & 0xFFu) - minSV) << rsh;
-                    o[2] = (((h2 >> 16) & 0xFFu) - minSV) << rsh;
-                    o[3] = ((h2 & 0xFFu) - minSV) << rsh;
-                    o[4] = (((h1 >> 16) & 0xFFu) - minSV) << rsh;
-                    o[5] = ((h1 & 0xFFu) - minSV) << rsh;
-                    o[6] = (((h0 >> 16) & 0xFFu) - minSV) << rsh;
-                    o[7] = ((h0 & 0xFFu) - minSV) << rsh;
-                };
-                uint32_t v2 = v << 1;  // twice the state minus L
-                // steps [t0, t1) of word g one at a time (the partial first and last words)
-                auto partial = [&](unsigned g, unsigned t0, unsigned t1) {
-                    uint32_t o[8];
-                    offsets(wp[-(int)g], o);
+            // the two words that hold positions [e0, e0 + 16), the last of them first
+            auto load = [&](unsigned e0, uint4 &x0, uint4 &x1) {
+                x0 = x1 = make_uint4(0, 0, 0, 0);
+                if (e0 >= ns) return;
+                const unsigned w1 = (lead + n - 3 - e0) >> 4;
+                x1 = __ldg(g4 + w1);
+                if (w1) x0 = __ldg(g4 + w1 - 1);
+            };
+            const unsigned rot = ((lead + n - 3) & 15u) + 1, wrot = rot >> 2, brot = (rot & 3u) * 8;
+            uint4 x0, x1;
+            load(16 * lane, x0, x1);
+            for (unsigned j0 = 0; 2 * j0 < ns; j0 += kFseBatch) {
+                {
+                    uint32_t x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, o[16];
+                    if (wrot & 1u) {
 #pragma unroll
-                    for (unsigned t = 0; t < 8; t++) {
-                        if (t < t0 || t >= t1) continue;
-                        rk[8 * g + t] = (uint16_t)v2;
-                        v2 = step(o[t], v2);
+                        for (int q = 0; q < 7; q++) x[q] = x[q + 1];
                     }
-                };
-                const unsigned gs = lead ? 1u : 0u, ge = nv >> 3;  // the whole words [gs, ge)
-                if (lead) partial(0, lead, min(8u, nv));
-                if (gs < ge) {
-                    // Whole words; the symbol words are loaded three words ahead and their row
-                    // offsets formed a word ahead, so that only the adds and lookups stay on the chain.
-                    uint4 q1 = gs + 1 < ge ? wp[-(int)(gs + 1)] : make_uint4(0, 0, 0, 0);
-                    uint4 q2 = gs + 2 < ge ? wp[-(int)(gs + 2)] : make_uint4(0, 0, 0, 0);
-                    uint32_t o[8];
-                    offsets(wp[-(int)gs], o);
-                    for (unsigned g = gs; g < ge; g++) {
-                        const uint4 qn = q1;
-                        q1 = q2;
-                        if (g + 3 < ge) q2 = wp[-(int)(g + 3)];
-                        uint32_t on[8];
-                        offsets(qn, on);
+                    if (wrot & 2u) {
+#pragma unroll
+                        for (int q = 0; q < 6; q++) x[q] = x[q + 2];
+                    }
+                    if (wrot & 4u) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) x[q] = x[q + 4];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) x[q] = __funnelshift_r(x[q], x[q + 1], brot);
+#pragma unroll
+                    for (int t = 0; t < 16; t++) o[t] = w.step[(x[(15 - t) >> 2] >> (8 * ((15 - t) & 3))) & 0xFFu];
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        w.ring[c][2 * lane] = make_uint4(o[c], o[c + 2], o[c + 4], o[c + 6]);
+                        w.ring[c][2 * lane + 1] = make_uint4(o[c + 8], o[c + 10], o[c + 12], o[c + 14]);
+                    }
+                }
+                load(2 * (j0 + kFseBatch) + 16 * lane, x0, x1);
+                __syncwarp();
+                if (lane < 2) {
+                    auto step = [](uint32_t o, uint32_t e2) -> uint32_t {
+                        const uint32_t at = (o >> 5) + 2 * __funnelshift_r(e2, 0u, o);
+                        uint16_t r;
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(at));
+                        return r;
+                    };
+                    const uint4 *rg = w.ring[lane];
+                    const unsigned steps = min(kFseBatch, m - min(m, j0)), ng = steps / 8;
+                    uint4 a = rg[0], c = rg[1];
+                    for (unsigned g = 0; g < ng; g++) {
+                        const unsigned gn = (g + 1) % (kFseBatch / 8);
+                        const uint4 an = rg[2 * gn], cn = rg[2 * gn + 1];
+                        const uint32_t o[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
                         uint32_t r[8];
 #pragma unroll
                         for (int t = 0; t < 8; t++) {
-                            r[t] = v2;
-                            v2 = step(o[t], v2);
+                            r[t] = e;
+                            e = step(o[t], e);
                         }
-                        *reinterpret_cast<uint4 *>(rk + 8 * g) =
+                        *reinterpret_cast<uint4 *>(rk + j0 + 8 * g) =
                             make_uint4(r[0] | (r[1] << 16), r[2] | (r[3] << 16), r[4] | (r[5] << 16), r[6] | (r[7] << 16));
-#pragma unroll
-                        for (int t = 0; t < 8; t++) o[t] = on[t];
+                        a = an;
+                        c = cn;
+                    }
+                    const uint32_t *o = reinterpret_cast<const uint32_t *>(rg);
+                    for (unsigned t = 8 * ng; t < steps; t++) {
+                        rk[j0 + t] = (uint16_t)e;
+                        e = step(o[t], e);
                     }
                 }
-                if (ge >= gs && 8 * ge < nv && (ge > 0 || !lead)) partial(ge, 0, nv - 8 * ge);
-                v = v2 >> 1;
-            } else if (m > 0) {
-                // the state-table path: the symbol transform of the next symbol and the symbol
-                // after it are loaded ahead, so that only the state table lookup stays on the chain
-                uint32_t sA = v + L;
-                int i = top;
-                fse::SymTT ta = w.sym_tt[src[i]];
-                unsigned ya = src[max(i - 2, 0)];
-                for (unsigned j = 0; j < m; j++, i -= 2) {
-                    const fse::SymTT na = w.sym_tt[ya];
-                    ya = __ldg(src + max(i - 4, 0));
-                    const uint32_t nba = (sA + ta.deltaNbBits) >> 16;
-                    const uint32_t xa = w.state_table[(int32_t)(sA >> nba) + ta.deltaFindState];
-                    rk[j] = (uint16_t)((sA - L) << 1);
-                    sA = xa;
-                    ta = na;
-                }
-                v = sA - L;
+                __syncwarp();  // the batch's steps are read
             }
-            s_lead[k] = lead;
-            if (k == 0) s_s0 = v + L;
-            else s_s1 = v + L;
-            // the walk's end, taken by the chain lane itself (a lane that waits at the barrier
-            // below may read the timer before the barrier completes)
-            if (phase) gm.tend[k] = global_ns();
+            if (lane < 2) {
+                rk[m] = (uint16_t)e;
+                w.fin[lane] = e >> 4;
+            }
+            if (lane == 0 && phase) w.tend = global_ns();
+        } else {  // the bits' scratch starts at zero
+            const unsigned long long most = (unsigned long long)ns * tl + 2 * tl + 1;
+            constexpr unsigned kCap = (unsigned)(kBlockSlot / 4);
+            const unsigned zw = (unsigned)((most + 31) / 32 + 1 < kCap ? (most + 31) / 32 + 1 : kCap);
+            const unsigned t = tid - (wid > (grp & 3u) ? 32u : 0u);
+            for (unsigned z = t; z < zw; z += kFseGroupThreads - 32) bw[z] = 0u;
         }
     }
     group_sync(bar);
-    if (tid == 0 && phase) phase[(size_t)slot * kFsePhases + 4] = s_mode == 2 ? max(gm.tend[0], gm.tend[1]) : global_ns();
-    int mode = s_mode;
+    if (tid == 0 && phase) phase[(size_t)slot * kFsePhases + 4] = w.mode == 2 ? w.tend : global_ns();
+    int mode = w.mode;
     size_t body = 0;
     if (mode == 2) {
-        const unsigned tl = s_tl;
-        const unsigned ns = n - 2;  // emission position e codes symbol n - 3 - e
-        // the record of emission position e: even positions belong to the chain of n-3's parity
-        const unsigned ka = (n - 3) & 1u;
-        const unsigned offA = ka * kFseChainRec + s_lead[ka], offB = (ka ^ 1u) * kFseChainRec + s_lead[ka ^ 1u];
-        const uint16_t *rec16 = reinterpret_cast<const uint16_t *>(rec);
-        // the state minus L before emission position e (symbol n - 3 - e)
-        auto V = [&](unsigned e) -> uint32_t { return rec16[((e & 1u) ? offB : offA) + (e >> 1)] >> 1; };
-        // the number of bits that state v + L emits for symbol sy
-        const uint32_t Lb = 1u << tl;
-        auto NB = [&](uint32_t v, unsigned sy) -> uint32_t { return (v + Lb + w.sym_tt[sy].deltaNbBits) >> 16; };
-        // The bits leave in chunks of kPackChunk emission positions.  A chunk's records and symbols
-        // are staged in shared memory (the next-state table's space, free once the chains are
-        // done); lane l of a warp takes position 32 s + l of the chunk's slice s; the slices' bit
-        // totals, scanned, and a warp scan within the slice give every position its bit offset; the
-        // bits are merged into a shared word buffer, whose words then leave as whole-word stores
-        // (the chunk's two edge words, shared with the neighbouring chunks, by atomicOr into the
-        // zeroed scratch).  Words past the block's slot are dropped: such a block is stored raw.
-        uint16_t *sv = reinterpret_cast<uint16_t *>(s_nxt4);
-        uint8_t *ss = reinterpret_cast<uint8_t *>(sv + kPackChunk);
-        uint32_t *sw = reinterpret_cast<uint32_t *>(ss + kPackChunk);
-        uint32_t *slice = sw + kPackWords;  // kPackChunk / 32 slice offsets, then the chunk's total
-        const unsigned lane = tid & 31u, wid = tid >> 5;
+        const unsigned tl = w.tl, ns = n - 2, nunits = (ns + kPackUnit - 1) / kPackUnit;
         constexpr unsigned kCap = (unsigned)(kBlockSlot / 4);
-        {
-            const unsigned long long most = (unsigned long long)ns * tl + 2 * tl + 1;
-            const unsigned zw = (unsigned)((most + 31) / 32 + 1 < kCap ? (most + 31) / 32 + 1 : kCap);
-            for (unsigned z = tid; z < zw; z += kFseGroupThreads) bw[z] = 0u;
+        // A lane takes 16 emission positions from 16 x on: eight records of each chain and the one after
+        // them (a record's low bits are those that its step emitted, the count is in the next record).
+        auto fetch = [&](unsigned x, uint4 &ra, uint4 &rb, uint32_t &na, uint32_t &nb) {
+            ra = rb = make_uint4(0, 0, 0, 0);
+            const bool in = 16 * x < ns;
+            if (in) {
+                ra = *reinterpret_cast<const uint4 *>(rec + 8 * x);
+                rb = *reinterpret_cast<const uint4 *>(rec + kFseChainRec + 8 * x);
+            }
+            na = __shfl_down_sync(0xffffffffu, ra.x & 0xFFFFu, 1);
+            nb = __shfl_down_sync(0xffffffffu, rb.x & 0xFFFFu, 1);
+            if (in && (lane == 31 || 16 * x + 16 >= ns)) {
+                na = rec[8 * x + 8];
+                nb = rec[kFseChainRec + 8 * x + 8];
+            }
+        };
+        auto rec_of = [](const uint4 &r, uint32_t after, unsigned j) -> uint32_t {
+            const uint32_t q = j < 2 ? r.x : j < 4 ? r.y : j < 6 ? r.z : j < 8 ? r.w : after;
+            return j & 1u ? q >> 16 : q & 0xFFFFu;
+        };
+        // the bits of a lane's positions
+        auto bits_of = [&](unsigned x, const uint4 &ra, const uint4 &rb, uint32_t na, uint32_t nb) -> uint32_t {
+            if (16 * x + 16 <= ns) {
+                const uint32_t k = 0x000F000Fu;
+                const uint32_t t = (ra.x & k) + (ra.y & k) + (ra.z & k) + (ra.w & k) + (rb.x & k) + (rb.y & k) + (rb.z & k) + (rb.w & k);
+                return (t & 0xFFFFu) + (t >> 16) - (ra.x & 15u) - (rb.x & 15u) + (na & 15u) + (nb & 15u);
+            }
+            uint32_t t = 0;
+#pragma unroll
+            for (unsigned i = 0; i < 16; i++)
+                if (16 * x + i < ns) t += (i & 1u ? rec_of(rb, nb, i / 2 + 1) : rec_of(ra, na, i / 2 + 1)) & 15u;
+            return t;
+        };
+        for (unsigned u = wid; u < nunits; u += kFseGroupWarps) {
+            uint4 ra, rb;
+            uint32_t na, nb;
+            fetch(32 * u + lane, ra, rb, na, nb);
+            const uint32_t t = __reduce_add_sync(0xffffffffu, bits_of(32 * u + lane, ra, rb, na, nb));
+            if (lane == 0) w.unit[u] = t;
         }
-        uint32_t base = 0;  // bits of the chunks before
-        for (unsigned c0 = 0; c0 < ns; c0 += kPackChunk) {
-            const unsigned cn = min(kPackChunk, ns - c0), nsl = (cn + 31) / 32;
-            group_sync(bar);  // the previous chunk's words are out (the first time: the scratch is zero)
-            // the records come from L2: each thread issues a batch of loads before it stores any
+        group_sync(bar);
+        if (wid == 0) {
+            constexpr unsigned kPer = FBLK / kPackUnit / 32;
+            uint32_t a[kPer], sum = 0;
 #pragma unroll
-            for (unsigned h = 0; h < kPackChunk / kFseGroupThreads; h += kStageBatch) {
-                uint32_t r[kStageBatch], y[kStageBatch];
+            for (unsigned q = 0; q < kPer; q++) {
+                a[q] = lane * kPer + q < nunits ? w.unit[lane * kPer + q] : 0u;
+                sum += a[q];
+            }
+            const uint32_t incl = warp_incl_scan(sum);
+            uint32_t run = incl - sum;
 #pragma unroll
-                for (unsigned u = 0; u < kStageBatch; u++) {
-                    const unsigned j = tid + (h + u) * kFseGroupThreads, e = c0 + j;
-                    r[u] = j < cn ? rec16[((e & 1u) ? offB : offA) + (e >> 1)] : 0u;
-                    y[u] = j < cn ? src[n - 3 - e] : 0u;
+            for (unsigned q = 0; q < kPer; q++) {
+                if (lane * kPer + q < nunits) w.unit[lane * kPer + q] = run;
+                run += a[q];
+            }
+            if (lane == 31) w.bits = incl;
+        }
+        group_sync(bar);
+        // The units' bits: merged into the warp's words, which leave as whole-word stores (a unit's two edge
+        // words, shared with its neighbours, by atomicOr into the zeroed scratch).  Words past the block's slot
+        // are dropped: such a block is stored raw.
+        uint32_t *pw = w.pack[wid];
+        for (unsigned u = wid; u < nunits; u += kFseGroupWarps) {
+            const unsigned x = 32 * u + lane;
+            uint4 ra, rb;
+            uint32_t na, nb;
+            fetch(x, ra, rb, na, nb);
+            const uint32_t mine = bits_of(x, ra, rb, na, nb), incl = warp_incl_scan(mine);
+            const uint32_t u0 = w.unit[u], b0 = u0 & 31u;
+            const uint32_t nw = (b0 + __shfl_sync(0xffffffffu, incl, 31) + 31) >> 5;
+            for (unsigned z = lane; z < nw; z += 32) pw[z] = 0;
+            __syncwarp();
+            uint32_t p = b0 + incl - mine, fill = p & 31u;
+            uint32_t *o = pw + (p >> 5);
+            unsigned long long acc = 0;
+            // whether one of these positions codes a symbol with a checkpoint before it
+            const bool marked = ck && 16 * x < ns && (part < 16 || ((n - 3 - 16 * x) & (part - 1)) < 16);
+#pragma unroll
+            for (unsigned i = 0; i < 16; i++) {
+                if (16 * x + i >= ns) continue;
+                const uint32_t v = (i & 1u ? rec_of(rb, nb, i / 2) : rec_of(ra, na, i / 2)) >> 4;
+                const uint32_t k = (i & 1u ? rec_of(rb, nb, i / 2 + 1) : rec_of(ra, na, i / 2 + 1)) & 15u;
+                acc |= (unsigned long long)(v & ((1u << k) - 1u)) << fill;
+                fill += k;
+                p += k;
+                if (fill >= 32) {
+                    atomicOr(o++, (uint32_t)acc);
+                    acc >>= 32;
+                    fill -= 32;
                 }
-#pragma unroll
-                for (unsigned u = 0; u < kStageBatch; u++) {
-                    const unsigned j = tid + (h + u) * kFseGroupThreads;
-                    if (j < cn) {
-                        sv[j] = (uint16_t)r[u];
-                        ss[j] = (uint8_t)y[u];
-                    }
+                if (marked) {
+                    const unsigned e = 16 * x + i, s = n - 3 - e;
+                    // the decoder's states before symbol s: those after symbols s and s + 1, which are the
+                    // states before the chains' next symbols
+                    if (s > 0 && (s & (part - 1)) == 0)
+                        ck[s / part - 1] = FseCkpt{u0 - b0 + p, (uint16_t)(rec[(e & 1u) * kFseChainRec + e / 2 + 1] >> 4),
+                                                   (uint16_t)(rec[((e + 1) & 1u) * kFseChainRec + (e + 1) / 2] >> 4)};
                 }
             }
-            for (unsigned z = tid; z < kPackWords; z += kFseGroupThreads) sw[z] = 0u;
-            group_sync(bar);
-            for (unsigned sl = wid; sl < nsl; sl += kFseGroupThreads / 32) {
-                const unsigned j = sl * 32 + lane;
-                const uint32_t nb = j < cn ? NB(sv[j] >> 1, ss[j]) : 0u;
-                const uint32_t t = __reduce_add_sync(0xffffffffu, nb);
-                if (lane == 0) slice[sl] = t;
-            }
-            group_sync(bar);
-            if (wid == 0) {  // exclusive scan of the slice totals; the chunk's total after them
-                constexpr unsigned kPer = kPackChunk / 32 / 32;
-                uint32_t a[kPer], sum = 0;
-#pragma unroll
-                for (unsigned q = 0; q < kPer; q++) {
-                    const unsigned sl = lane * kPer + q;
-                    a[q] = sl < nsl ? slice[sl] : 0u;
-                    sum += a[q];
-                }
-                const uint32_t incl = warp_incl_scan(sum);
-                uint32_t run = incl - sum;
-#pragma unroll
-                for (unsigned q = 0; q < kPer; q++) {
-                    const unsigned sl = lane * kPer + q;
-                    if (sl < nsl) slice[sl] = run;
-                    run += a[q];
-                }
-                if (lane == 31) slice[kPackChunk / 32] = incl;
-            }
-            group_sync(bar);
-            const uint32_t ctot = slice[kPackChunk / 32], b0 = base & 31u;
-            for (unsigned sl = wid; sl < nsl; sl += kFseGroupThreads / 32) {
-                const unsigned j = sl * 32 + lane;
-                uint32_t v = 0, nb = 0;
-                if (j < cn) {
-                    v = sv[j] >> 1;
-                    nb = NB(v, ss[j]);
-                }
-                const uint32_t incl = warp_incl_scan(nb);
-                const uint32_t p = b0 + slice[sl] + incl - nb;  // bit offset in the chunk's words
-                if (nb) {
-                    const uint32_t bits = v & ((1u << nb) - 1u), w0 = p >> 5, sh = p & 31u;
-                    atomicOr(sw + w0, bits << sh);
-                    if (sh + nb > 32) atomicOr(sw + w0 + 1, bits >> (32 - sh));
-                }
-                if (ck && j < cn) {
-                    const unsigned e = c0 + j, i = n - 3 - e;
-                    if (i > 0 && (i & (part - 1)) == 0) {
-                        // decoder states before symbol i: the states after symbol i (the state
-                        // before symbol i - 2 of its chain) and after symbol i + 1 (before i - 1)
-                        const uint32_t odd = i + 1 <= n - 3 ? V(e + 1) : ((n - 2) & 1 ? s_i1 : s_i0);
-                        ck[i / part - 1] = FseCkpt{base + slice[sl] + incl, (uint16_t)V(e + 2), (uint16_t)odd};
-                    }
-                }
-            }
-            group_sync(bar);
-            const unsigned wfirst = base >> 5, nw = (b0 + ctot + 31) >> 5;
-            for (unsigned z = tid; z < nw; z += kFseGroupThreads) {
-                const unsigned gw = wfirst + z;
+            if ((uint32_t)acc) atomicOr(o, (uint32_t)acc);
+            __syncwarp();
+            for (unsigned z = lane; z < nw; z += 32) {
+                const unsigned gw = (u0 >> 5) + z;
                 if (gw >= kCap) continue;
-                if (z == 0 || z == nw - 1) atomicOr(bw + gw, sw[z]);
-                else bw[gw] = sw[z];
+                if (z == 0 || z == nw - 1) atomicOr(bw + gw, pw[z]);
+                else bw[gw] = pw[z];
             }
-            base += ctot;
+            __syncwarp();
         }
-        const uint32_t sym_bits = base;  // bits of all symbols
+        const uint32_t sym_bits = w.bits;  // bits of all symbols
         const uint32_t total = sym_bits + 2 * tl + 1;
         body = (total + 7) / 8;
-        if (body + 8 > kBlockSlot - 5 - s_hdr || s_hdr + body >= n - 1) mode = 0;  // not worth coding: raw
+        if (body + 8 > kBlockSlot - 5 - w.hdr || w.hdr + body >= n - 1) mode = 0;  // not worth coding: raw
         group_sync(bar);
         if (mode == 2 && tid == 0) {  // final states (odd, then even) and the end mark
             uint32_t p2 = sym_bits;
@@ -623,8 +597,8 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
                 for (uint32_t b = 0; b < nb; b++, p2++)
                     if ((v >> b) & 1u) atomicOr(bw + (p2 >> 5), 1u << (p2 & 31u));
             };
-            put(s_s1 & ((1u << tl) - 1), tl);
-            put(s_s0 & ((1u << tl) - 1), tl);
+            put(w.fin[n & 1u], tl);  // chain 0 codes the symbols of n - 1's parity
+            put(w.fin[(n & 1u) ^ 1u], tl);
             put(1u, 1u);
         }
         group_sync(bar);
@@ -641,8 +615,8 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, 4 / G)
             sizes[b] = 2 | (2ULL << 56);
         }
     } else {
-        const size_t r = s_hdr + body;
-        uint8_t *d = out + 5 + s_hdr;
+        const size_t r = w.hdr + body;
+        uint8_t *d = out + 5 + w.hdr;
         const uint8_t *bb = reinterpret_cast<const uint8_t *>(bw);
         for (size_t i = tid; i < body; i += kFseGroupThreads) d[i] = bb[i];
         if (tid == 0) {
@@ -1099,9 +1073,9 @@ void enable_fse_smem() {
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
     FB2_CUDA(cudaFuncSetAttribute(k_fse_encode_blocks<kFseGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(kFseGroups * kFseNxtBytes)));
+                                  (int)(kFseGroups * sizeof(FseGroupSmem))));
     FB2_CUDA(cudaFuncSetAttribute(k_fse_encode_blocks<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kFseNxtBytes));
+                                  (int)sizeof(FseGroupSmem)));
     FB2_CUDA(cudaFuncSetAttribute(k_fse_decode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fse_dec_smem(64)));
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -1164,11 +1138,11 @@ GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned lo
     enable_fse_smem();
     if (nj + beside > (size_t)sm_count()) {
         constexpr unsigned G = kFseGroups;
-        constexpr int smem = (int)(G * kFseNxtBytes);
+        constexpr int smem = (int)(G * sizeof(FseGroupSmem));
         k_fse_encode_blocks<G><<<(unsigned)((nj + G - 1) / G), G * kFseGroupThreads, smem, st>>>(
             cls, d_jobs, (unsigned)nj, gb.slots, gb.sizes, bits, part, gb.cks, recs, d_order, gb.phase);
     } else {
-        constexpr int smem = (int)kFseNxtBytes;
+        constexpr int smem = (int)sizeof(FseGroupSmem);
         k_fse_encode_blocks<1><<<(unsigned)nj, kFseGroupThreads, smem, st>>>(
             cls, d_jobs, (unsigned)nj, gb.slots, gb.sizes, bits, part, gb.cks, recs, d_order, gb.phase);
     }
