@@ -1080,8 +1080,8 @@ void enable_fse_smem() {
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
 
-// The FSE class blocks of the gamma classes, launched by gamma_launch; gamma_finish packs the
-// mantissas and collects the blocks.  Between the two the caller may launch other work: the class
+// The FSE class blocks of the gamma classes, launched by gamma_launch; gamma_pack packs the
+// mantissas and gamma_finish collects both.  Between the two the caller may launch other work: the class
 // blocks are long sequential chains, so they go to the GPU before the order-1 chain encoder.
 struct GammaBlocks {
     long long T = 0;
@@ -1094,6 +1094,11 @@ struct GammaBlocks {
     FseCkpt *cks = nullptr;
     size_t ck_per_block = 0;
     unsigned long long *phase = nullptr;  // per-block phase times, traced calls only
+    unsigned longest() const {
+        unsigned n = 0;
+        for (const BlockJob &j : jobs) n = std::max(n, j.n);
+        return n;
+    }
 };
 
 // `beside`: CTAs of whole SMs that run next to the class blocks (the chain encoder's).
@@ -1150,12 +1155,55 @@ GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned lo
     return gb;
 }
 
+// The packed mantissas of the groups: words on the device, where each group's start in them.
+struct GammaWords {
+    uint32_t *buf = nullptr;
+    std::vector<unsigned long long> gword;
+    unsigned long long *d_gb = nullptr;  // bits per group
+};
+
+// Packs the mantissas (needs the classes and the values, not the class blocks).
 template <class V>
-GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const V *d_vals, cudaStream_t st) {
-    Trace tr("gamma");
-    const std::vector<unsigned long long> &gstart = gb.gstart;
+GammaWords gamma_pack(Pool &pool, const uint8_t *cls, const std::vector<unsigned long long> &gstart, const V *d_vals,
+                      cudaStream_t st) {
+    GammaWords w;
     const int G = (int)gstart.size() - 1;
-    const long long T = gb.T;
+    if (gstart.back() == 0) return w;
+    // every group's words: room for the longest mantissas (16 bits of an escape code's value, 31 of any)
+    constexpr unsigned long long kMost = sizeof(V) == 2 ? 16 : 31;
+    std::vector<unsigned long long> ust(G + 1, 0);
+    w.gword.assign(G, 0);
+    unsigned long long words = 0;
+    for (int g = 0; g < G; g++) {
+        const unsigned long long c = gstart[g + 1] - gstart[g];
+        w.gword[g] = words;
+        words += (c * kMost + 31) / 32 + 2;
+        ust[g + 1] = ust[g] + (c + kUnit - 1) / kUnit;
+    }
+    const unsigned long long NU = ust[G];
+    w.buf = pool.get<uint32_t>(words + 4);
+    unsigned long long *d_gstart = h2d(pool, gstart, st);
+    unsigned long long *d_ust = h2d(pool, ust, st);
+    unsigned long long *d_gword = h2d(pool, w.gword, st);
+    unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);
+    w.d_gb = pool.get<unsigned long long>(G);
+    k_unit_bits<<<grid_for((long long)NU * 32, 256), 256, 0, st>>>(cls, d_gstart, d_ust, G, NU, uoff);
+    FB2_CHECK_LAUNCH();
+    k_scan_small<unsigned long long><<<1, 1024, 0, st>>>(uoff, (long long)NU);
+    FB2_CHECK_LAUNCH();
+    k_gamma_heads<<<grid_for((long long)std::max<unsigned long long>(NU, G), 256), 256, 0, st>>>(uoff, d_ust, G, NU, d_gword,
+                                                                                                w.d_gb, w.buf);
+    FB2_CHECK_LAUNCH();
+    k_gamma_pack_units<V><<<(unsigned)((NU + kUnitWarps - 1) / kUnitWarps), kUnitWarps * 32, 0, st>>>(
+        d_vals, cls, d_gstart, d_ust, G, NU, uoff, d_gword, w.buf);
+    FB2_CHECK_LAUNCH();
+    return w;
+}
+
+// Collects the groups: the mantissas packed on stream ms, the class blocks coded on stream st.
+GammaOut gamma_finish(const GammaBlocks &gb, const GammaWords &w, cudaStream_t st, cudaStream_t ms) {
+    Trace tr("gamma");
+    const int G = (int)gb.gstart.size() - 1;
     GammaOut out;
     out.cls_pieces.resize(G);
     out.cls_n.resize(G);
@@ -1164,40 +1212,12 @@ GammaOut gamma_finish(Pool &pool, const GammaBlocks &gb, const V *d_vals, cudaSt
     out.cls_bytes.assign(G, 0);
     out.man_ptr.assign(G, nullptr);
     out.man_bytes.assign(G, 0);
-    if (T == 0) return out;
-    const uint8_t *cls = gb.cls;
-    // every group's words: room for the longest mantissas (16 bits of an escape code's value, 31 of any)
-    constexpr unsigned long long kMost = sizeof(V) == 2 ? 16 : 31;
-    std::vector<unsigned long long> gword(G), ust(G + 1, 0);
-    unsigned long long words = 0;
-    for (int g = 0; g < G; g++) {
-        const unsigned long long c = gstart[g + 1] - gstart[g];
-        gword[g] = words;
-        words += (c * kMost + 31) / 32 + 2;
-        ust[g + 1] = ust[g] + (c + kUnit - 1) / kUnit;
-    }
-    const unsigned long long NU = ust[G];
-    uint32_t *wbuf = pool.get<uint32_t>(words + 4);
-    unsigned long long *d_gstart = h2d(pool, gstart, st);
-    unsigned long long *d_ust = h2d(pool, ust, st);
-    unsigned long long *d_gword = h2d(pool, gword, st);
-    unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);
-    unsigned long long *d_gb = pool.get<unsigned long long>(G);
-    k_unit_bits<<<grid_for((long long)NU * 32, 256), 256, 0, st>>>(cls, d_gstart, d_ust, G, NU, uoff);
-    FB2_CHECK_LAUNCH();
-    k_scan_small<unsigned long long><<<1, 1024, 0, st>>>(uoff, (long long)NU);
-    FB2_CHECK_LAUNCH();
-    k_gamma_heads<<<grid_for((long long)std::max<unsigned long long>(NU, G), 256), 256, 0, st>>>(uoff, d_ust, G, NU, d_gword,
-                                                                                                d_gb, wbuf);
-    FB2_CHECK_LAUNCH();
-    k_gamma_pack_units<V><<<(unsigned)((NU + kUnitWarps - 1) / kUnitWarps), kUnitWarps * 32, 0, st>>>(
-        d_vals, cls, d_gstart, d_ust, G, NU, uoff, d_gword, wbuf);
-    FB2_CHECK_LAUNCH();
-    const std::vector<unsigned long long> gbits = d2h(d_gb, (size_t)G, st);
+    if (gb.T == 0) return out;
+    const std::vector<unsigned long long> gbits = d2h(w.d_gb, (size_t)G, ms);
     tr.mark("group bits known");
     for (int g = 0; g < G; g++) {
         out.man_bytes[g] = (size_t)((gbits[g] + 7) / 8);
-        out.man_ptr[g] = reinterpret_cast<const uint8_t *>(wbuf + gword[g]);
+        out.man_ptr[g] = reinterpret_cast<const uint8_t *>(w.buf + w.gword[g]);
     }
     std::vector<unsigned long long> hs = d2h(gb.sizes, gb.jobs.size(), st);
     tr.mark("class blocks coded");
@@ -1240,7 +1260,7 @@ GammaOut gamma_encode(Pool &pool, const uint32_t *d_vals, const std::vector<unsi
         FB2_CHECK_LAUNCH();
     }
     const GammaBlocks gb = gamma_launch(pool, cls, gstart, st, ckpt_part);
-    return gamma_finish(pool, gb, d_vals, st);
+    return gamma_finish(gb, gamma_pack(pool, cls, gstart, d_vals, st), st, st);
 }
 
 // Adds the fse_enc records of group g, recording each record's header bytes for the index.
@@ -3797,8 +3817,19 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         encode_chains(pool, cp, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
         tr.gpu("chain encoder done", st);
         tr.mark("chains launched");
-        GammaOut go = gamma_finish(spool, gblocks, eraw, es);
-        tr.gpu("escape mantissas packed", es);
+        // The mantissas go behind the one that ends first: the chain encoder (0.4 ms and 5 ps a code) or the
+        // class blocks (15 ns a symbol of the longest block, 1 ms for a full one, kFseGroups blocks an SM in a
+        // wave).  384^3 f64, 758 blocks beside 56 M codes: behind the blocks 2.63 ms a call, behind the chains
+        // 2.50; 512^3 f32, where both take as long, the same; 211 x 307 x 401 f32, 3 short blocks: 2.56 ms a
+        // round trip behind the blocks, 2.67 behind the chains.
+        const double chain_ns = 4e5 + 5e-3 * (double)N;
+        const double blocks_ns = 15.0 * (double)gblocks.longest() *
+                                 (double)((gblocks.jobs.size() + kFseGroups * sm_count() - 1) / (kFseGroups * sm_count()));
+        const bool behind_chains = queue_first && chain_ns < blocks_ns;
+        cudaStream_t ms = behind_chains ? st : es;
+        const GammaWords gwords = gamma_pack(behind_chains ? pool : spool, ecls, gstart, eraw, ms);
+        tr.gpu("escape mantissas packed", ms);
+        GammaOut go = gamma_finish(gblocks, gwords, es, ms);
         // the chains' escape counts (stream header) from the histogram pass; their sums per segment
         // are the escape groups counted above
         const std::vector<uint32_t> h_nvk = d2h(nvk, (size_t)S * kMaxK, st);
