@@ -22,18 +22,44 @@ namespace fb2 {
 constexpr size_t kZstdBlock = 128 * 1024;   // Block_Maximum_Size
 constexpr uint32_t kZstdMagic = 0xFD2FB528u;
 
+// A call on a small field takes some fifty blocks of scratch of a few KB at 1 to 3 us each, which is as long as
+// its kernels run: blocks below kSlabLimit are cut from slabs of kSlabBytes.
+constexpr size_t kSlabBytes = 1 << 20, kSlabLimit = kSlabBytes / 4;
 struct Pool {
     cudaStream_t st;
     std::vector<void *> ptrs;
+    uint8_t *slab = nullptr;  // the rest of the last slab
+    size_t left = 0;
     explicit Pool(cudaStream_t s);
     template <class T>
     T *get(size_t count) {
-        void *p = nullptr;
-        FB2_CUDA(cudaMallocAsync(&p, std::max<size_t>(count * sizeof(T), 16) + 64, st));
-        ptrs.push_back(p);
-        return static_cast<T *>(p);
+        // blocks start on 256 bytes, with at least 64 readable ones behind them
+        const size_t bytes = (std::max<size_t>(count * sizeof(T), 16) + 64 + 255) & ~size_t(255);
+        if (bytes >= kSlabLimit) return static_cast<T *>(block(bytes));
+        if (bytes > left) {
+            slab = static_cast<uint8_t *>(block(kSlabBytes));
+            left = kSlabBytes;
+        }
+        T *p = reinterpret_cast<T *>(slab);
+        slab += bytes;
+        left -= bytes;
+        return p;
+    }
+    // Takes over another pool's blocks (its stream's work is done before this pool's ends).
+    void take(Pool &other) {
+        ptrs.insert(ptrs.end(), other.ptrs.begin(), other.ptrs.end());
+        other.ptrs.clear();
+        other.left = 0;
     }
     ~Pool();
+
+  private:
+    void *block(size_t bytes) {
+        void *p = nullptr;
+        FB2_CUDA(cudaMallocAsync(&p, bytes, st));
+        ptrs.push_back(p);
+        return p;
+    }
 };
 
 // Pinned host staging for small device-to-host reads: a process-wide free list of page-locked
@@ -73,6 +99,23 @@ T *h2d(Pool &pool, const std::vector<T> &h, cudaStream_t st) {
     if (!h.empty()) FB2_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
     return d;
 }
+
+// Several host arrays that go to the device in one copy (a copy costs the host 3 us and the stream a gap, however
+// small): add() each, send() them, then get() the device address of each.
+struct Upload {
+    std::vector<uint8_t> host;
+    uint8_t *dev = nullptr;
+    template <class T>
+    size_t add(const std::vector<T> &v) {
+        const size_t at = host.size(), bytes = v.size() * sizeof(T);
+        host.resize(at + ((bytes + 15) & ~size_t(15)));
+        if (bytes) std::memcpy(host.data() + at, v.data(), bytes);
+        return at;
+    }
+    void send(Pool &pool, cudaStream_t st) { dev = h2d(pool, host, st); }
+    template <class T>
+    T *get(size_t at) const { return reinterpret_cast<T *>(dev + at); }
+};
 
 inline unsigned grid_for(long long n, int threads, long long cap = 1 << 20) {
     return (unsigned)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, cap));

@@ -1123,7 +1123,6 @@ GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned lo
     const size_t nj = gb.jobs.size();
     if (std::getenv("FALCONS_TRACE"))
         std::fprintf(stderr, "[falcons trace] escapes: %lld values in %d groups, %zu class blocks\n", T, G, nj);
-    BlockJob *d_jobs = h2d(pool, gb.jobs, st);
     gb.slots = pool.get<uint8_t>(nj * kBlockSlot);
     uint8_t *bits = pool.get<uint8_t>(nj * kBlockSlot);
     gb.sizes = pool.get<unsigned long long>(nj);
@@ -1133,7 +1132,11 @@ GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned lo
     std::vector<uint32_t> order(nj);
     for (size_t j = 0; j < nj; j++) order[j] = (uint32_t)j;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return gb.jobs[a].n > gb.jobs[b].n; });
-    uint32_t *d_order = h2d(pool, order, st);
+    Upload up;
+    const size_t u_jobs = up.add(gb.jobs), u_order = up.add(order);
+    up.send(pool, st);
+    const BlockJob *d_jobs = up.get<BlockJob>(u_jobs);
+    const uint32_t *d_order = up.get<uint32_t>(u_order);
     if (queued) FB2_CUDA(cudaEventRecord(queued, st));  // what the blocks wait for is on the stream
     const uint32_t part = ckpt_part ? ckpt_part : 4096u;
     if (std::getenv("FALCONS_TRACE")) {
@@ -1182,9 +1185,11 @@ GammaWords gamma_pack(Pool &pool, const uint8_t *cls, const std::vector<unsigned
     }
     const unsigned long long NU = ust[G];
     w.buf = pool.get<uint32_t>(words + 4);
-    unsigned long long *d_gstart = h2d(pool, gstart, st);
-    unsigned long long *d_ust = h2d(pool, ust, st);
-    unsigned long long *d_gword = h2d(pool, w.gword, st);
+    Upload up;
+    const size_t u_gstart = up.add(gstart), u_ust = up.add(ust), u_gword = up.add(w.gword);
+    up.send(pool, st);
+    const unsigned long long *d_gstart = up.get<unsigned long long>(u_gstart), *d_ust = up.get<unsigned long long>(u_ust),
+                             *d_gword = up.get<unsigned long long>(u_gword);
     unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);
     w.d_gb = pool.get<unsigned long long>(G);
     k_unit_bits<<<grid_for((long long)NU * 32, 256), 256, 0, st>>>(cls, d_gstart, d_ust, G, NU, uoff);
@@ -3267,6 +3272,15 @@ struct ChainParts {
     uint32_t spp = 1;               // parts per super part
     std::vector<EncCta> ctas, map_ctas;
     unsigned long long records = 0;
+    size_t u_chains, u_table, u_pstart, u_sstart, u_ctas, u_map_ctas;  // the lists in an upload
+    void add(Upload &up) {
+        u_chains = up.add(chains);
+        u_table = up.add(table);
+        u_pstart = up.add(pstart);
+        u_sstart = up.add(sstart);
+        u_ctas = up.add(ctas);
+        u_map_ctas = up.add(map_ctas);
+    }
 };
 ChainParts chain_parts(const std::vector<SegInfo> &segs, const std::vector<int> &seg_region, int K, uint32_t part) {
     ChainParts cp;
@@ -3296,20 +3310,20 @@ ChainParts chain_parts(const std::vector<SegInfo> &segs, const std::vector<int> 
     return cp;
 }
 
-void encode_chains(Pool &pool, const ChainParts &cp, const uint16_t *keys, size_t N, const uint32_t *image, uint32_t part,
+void encode_chains(Pool &pool, const ChainParts &cp, const Upload &up, const uint16_t *keys, size_t N, const uint32_t *image, uint32_t part,
                    uint8_t *slots, const unsigned long long *d_soff, unsigned long long *blen, O1Ckpt *cks,
                    const unsigned long long *d_ck_off, uint32_t ck_every, int *d_err, cudaStream_t st) {
     const uint32_t nchains = (uint32_t)cp.chains.size(), nparts = cp.pstart.back(), nsuper = cp.sstart.back();
-    int *d_table = h2d(pool, cp.table, st);
+    const int *d_table = up.get<int>(cp.u_table);
     EncArgs A{};
     A.keys = keys;
-    A.chains = h2d(pool, cp.chains, st);
-    A.pstart = h2d(pool, cp.pstart, st);
+    A.chains = up.get<EncChain>(cp.u_chains);
+    A.pstart = up.get<uint32_t>(cp.u_pstart);
     A.nchains = nchains;
     A.part = part;
     A.recs = part_records(part);
     A.image = image;
-    A.ctas = h2d(pool, cp.ctas, st);
+    A.ctas = up.get<EncCta>(cp.u_ctas);
     uint16_t *p16 = pool.get<uint16_t>((size_t)nparts * 3);
     A.exit1 = p16;
     A.exit2 = p16 + nparts;
@@ -3325,14 +3339,14 @@ void encode_chains(Pool &pool, const ChainParts &cp, const uint16_t *keys, size_
     A.err = d_err;
     // The maps' scratch takes the records' place: the map path writes them anew after its maps are used.
     MapArgs M{};
-    M.sstart = h2d(pool, cp.sstart, st);
+    M.sstart = up.get<uint32_t>(cp.u_sstart);
     M.spp = cp.spp;
     M.cap = (uint32_t)(O1_M + 28 * 1024 + 320 * cp.spp);
     uint8_t *area = pool.get<uint8_t>(std::max((size_t)cp.records * sizeof(uint4), (size_t)nsuper * M.cap * 2));
     A.rec = reinterpret_cast<uint4 *>(area);
     M.scratch = reinterpret_cast<uint16_t *>(area);
     M.hdr = pool.get<uint32_t>((size_t)nsuper * kMapHdr);
-    M.ctas = h2d(pool, cp.map_ctas, st);
+    M.ctas = up.get<EncCta>(cp.u_map_ctas);
     enable_big_smem();
     const unsigned nc = (unsigned)cp.ctas.size();
     k_o1_walk<false><<<nc, kEncThreads, kEncSmem, st>>>(A);
@@ -3466,7 +3480,7 @@ void gamma_decode(Pool &pool, const uint8_t *d, const ByteView &h,
                   const std::vector<size_t> &cls_off, const std::vector<size_t> &man_off,
                   const std::vector<size_t> &man_len, const std::vector<unsigned long long> &gstart,
                   uint32_t *d_vals, int *d_err, cudaStream_t st, const FseCkpt *d_fck = nullptr,
-                  uint32_t fpart = 0, unsigned long long n_fck = 0, const unsigned long long *d_gdst = nullptr,
+                  uint32_t fpart = 0, unsigned long long n_fck = 0, const std::vector<unsigned long long> &gdst = {},
                   int16_t *d_ovf = nullptr) {
     const int G = (int)gstart.size() - 1;
     const long long T = (long long)gstart.back();
@@ -3485,13 +3499,6 @@ void gamma_decode(Pool &pool, const uint8_t *d, const ByteView &h,
         if (used != n_fck)
             for (auto &j : jobs) j.ck = 0xFFFFFFFFu;
     }
-    uint8_t *cls = pool.get<uint8_t>(T);
-    BlockJob *dj = h2d(pool, jobs, st);
-    enable_fse_smem();
-    fse::DEntry *big = pool.get<fse::DEntry>(jobs.size() << fse::kMaxTableLog);
-    const uint32_t dpart = fpart ? fpart : FBLK;
-    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, fse_dec_smem(dpart), st>>>(d, dj, cls, d_err, dpart, d_fck, big);
-    FB2_CHECK_LAUNCH();
     std::vector<unsigned long long> gman(G), glen(G), ust(G + 1, 0);
     for (int g = 0; g < G; g++) {
         gman[g] = man_off[g];
@@ -3499,10 +3506,20 @@ void gamma_decode(Pool &pool, const uint8_t *d, const ByteView &h,
         ust[g + 1] = ust[g] + (gstart[g + 1] - gstart[g] + kUnit - 1) / kUnit;
     }
     const unsigned long long NU = ust[G];
-    unsigned long long *d_gstart = h2d(pool, gstart, st);
-    unsigned long long *d_gman = h2d(pool, gman, st);
-    unsigned long long *d_glen = h2d(pool, glen, st);
-    unsigned long long *d_ust = h2d(pool, ust, st);
+    Upload up;
+    const size_t u_jobs = up.add(jobs), u_gstart = up.add(gstart), u_gman = up.add(gman), u_glen = up.add(glen),
+                 u_ust = up.add(ust), u_gdst = up.add(gdst);
+    up.send(pool, st);
+    const BlockJob *dj = up.get<BlockJob>(u_jobs);
+    const unsigned long long *d_gstart = up.get<unsigned long long>(u_gstart), *d_gman = up.get<unsigned long long>(u_gman),
+                             *d_glen = up.get<unsigned long long>(u_glen), *d_ust = up.get<unsigned long long>(u_ust),
+                             *d_gdst = gdst.empty() ? nullptr : up.get<unsigned long long>(u_gdst);
+    uint8_t *cls = pool.get<uint8_t>(T);
+    enable_fse_smem();
+    fse::DEntry *big = pool.get<fse::DEntry>(jobs.size() << fse::kMaxTableLog);
+    const uint32_t dpart = fpart ? fpart : FBLK;
+    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, fse_dec_smem(dpart), st>>>(d, dj, cls, d_err, dpart, d_fck, big);
+    FB2_CHECK_LAUNCH();
     unsigned long long *usum = pool.get<unsigned long long>(NU + 1);
     unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);
     void *sc = pool.get<uint8_t>(scan_scratch_bytes((long long)NU, 8));
@@ -3647,7 +3664,6 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
             segs[g] = SegInfo{(unsigned long long)lo, (unsigned long long)ng,
                               (unsigned long long)((ng + K - 1) / K), K, 0};
         }
-        SegInfo *d_segs = h2d(pool, segs, st);
         // encoder part size, a power of two up to the decode checkpoint spacing: a chain's parts fit one
         // CTA's threads, and a part is shorter than the spacing where the parts would not give every SM
         // four full warps (a walk's time is then the length of a part: 64^3 codes 67 us in parts of 1024,
@@ -3679,12 +3695,53 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         cc.n_o1 = ck_off.back();
         O1Ckpt *o1ck = cc.n_o1 ? pool.get<O1Ckpt>(cc.n_o1) : nullptr;
         cc.o1 = o1ck;
-        unsigned long long *d_ck_off = o1ck ? h2d(pool, ck_off, st) : nullptr;
-        uint32_t *hist = pool.get<uint32_t>((size_t)S * O1_NCTX * O1_NSYM);
-        uint32_t *nvk = pool.get<uint32_t>((size_t)S * kMaxK);
+        // table regions: segments whose statistics come from the same part of the code stream
+        // share one table set (tune.regions holds the code positions where statistics change)
+        std::vector<int> seg_region(S, 0), rs{0};
+        if (tune.per_segment_tables) {
+            for (long long g = 0; g < S; g++) seg_region[g] = (int)g;
+            for (long long g = 1; g <= S; g++) rs.push_back((int)g);
+        } else {
+            int prev_rr = -1;
+            for (long long g = 0; g < S; g++) {
+                int rr = 0;
+                for (long long b : tune.regions)
+                    if (b > 0 && (unsigned long long)b <= segs[g].lo) rr++;
+                if (g > 0 && rr != prev_rr) rs.push_back((int)g);
+                seg_region[g] = (int)rs.size() - 1;
+                prev_rr = rr;
+            }
+            rs.push_back((int)S);
+        }
+        const int R = (int)rs.size() - 1;
+        // chain output slots
+        std::vector<unsigned long long> soff(nchains_all + 1, 0);
+        for (long long g = 0; g < S; g++)
+            for (int k = 0; k < kMaxK; k++) {
+                const unsigned long long c = (k < K) ? segs[g].cs * 2 + 64 : 0;
+                soff[g * kMaxK + k + 1] = soff[g * kMaxK + k] + ((c + 15) & ~15ULL);
+            }
+        // the segments' starts and the end, before which the escapes are counted
+        std::vector<unsigned long long> pos(S + 1, (unsigned long long)N);
+        for (long long g = 0; g < S; g++) pos[g] = segs[g].lo;
+        // what the kernels need to know of segments, chains and slots goes to the device in one copy
+        Upload up;
+        const size_t u_segs = up.add(segs), u_ck_off = up.add(ck_off), u_rs = up.add(rs),
+                     u_soff = up.add(soff), u_pos = up.add(pos);
+        ChainParts cp = chain_parts(segs, seg_region, K, enc_part);
+        cp.add(up);
+        up.send(pool, st);
+        const SegInfo *d_segs = up.get<SegInfo>(u_segs);
+        const unsigned long long *d_ck_off = o1ck ? up.get<unsigned long long>(u_ck_off) : nullptr;
+        // the key counts, the chains' escape counts and the error words, cleared together; the last two and the
+        // chains' lengths, read together at the end
+        const size_t n_hist = (size_t)S * O1_NCTX * O1_NSYM, n_nvk = (size_t)nchains_all;
+        uint32_t *hist = pool.get<uint32_t>(n_hist + n_nvk + 8 + 2 * n_nvk);
+        uint32_t *nvk = hist + n_hist;
+        int *d_err = reinterpret_cast<int *>(nvk + n_nvk);
+        unsigned long long *blen = reinterpret_cast<unsigned long long *>(d_err + 8);
         uint16_t *keys = pool.get<uint16_t>((size_t)N + 8);
-        FB2_CUDA(cudaMemsetAsync(hist, 0, (size_t)S * O1_NCTX * O1_NSYM * 4, st));
-        FB2_CUDA(cudaMemsetAsync(nvk, 0, (size_t)S * kMaxK * 4, st));
+        FB2_CUDA(cudaMemsetAsync(hist, 0, (n_hist + n_nvk + 8) * 4, st));
         // The escape side stream (escape values in index order, their gamma classes, the FSE class
         // blocks) needs only the codes, so it forks before the histogram pass and runs next to it,
         // the table builds and the chain encoder.
@@ -3719,14 +3776,9 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         FB2_CHECK_LAUNCH();
         // escapes before every segment start (the groups of the escape stream)
         unsigned long long *d_gstart = spool.get<unsigned long long>(S + 1);
-        {
-            std::vector<unsigned long long> pos(S + 1);
-            for (long long g = 0; g < S; g++) pos[g] = segs[g].lo;
-            pos[S] = (unsigned long long)N;
-            unsigned long long *d_pos = h2d(spool, pos, es);
-            k_esc_before<<<(unsigned)((S + 1 + 7) / 8), 256, 0, es>>>(q, tcnt, d_pos, (int)(S + 1), d_gstart);
-            FB2_CHECK_LAUNCH();
-        }
+        k_esc_before<<<(unsigned)((S + 1 + 7) / 8), 256, 0, es>>>(q, tcnt, up.get<unsigned long long>(u_pos), (int)(S + 1),
+                                                                 d_gstart);
+        FB2_CHECK_LAUNCH();
         tr.gpu("escape counts done", es);
         enable_big_smem();
         tr.gpu("histogram start", st);
@@ -3744,45 +3796,21 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         }
         FB2_CHECK_LAUNCH();
         tr.gpu("histogram done", st);
-        // table regions: segments whose statistics come from the same part of the code stream
-        // share one table set (tune.regions holds the code positions where statistics change)
-        std::vector<int> seg_region(S, 0), rs{0};
-        if (tune.per_segment_tables) {
-            for (long long g = 0; g < S; g++) seg_region[g] = (int)g;
-            for (long long g = 1; g <= S; g++) rs.push_back((int)g);
-        } else {
-            int prev_rr = -1;
-            for (long long g = 0; g < S; g++) {
-                int rr = 0;
-                for (long long b : tune.regions)
-                    if (b > 0 && (unsigned long long)b <= segs[g].lo) rr++;
-                if (g > 0 && rr != prev_rr) rs.push_back((int)g);
-                seg_region[g] = (int)rs.size() - 1;
-                prev_rr = rr;
-            }
-            rs.push_back((int)S);
-        }
-        const int R = (int)rs.size() - 1;
         uint32_t *rhist = hist;
         if (!tune.per_segment_tables) {
             rhist = pool.get<uint32_t>((size_t)R * O1_NCTX * O1_NSYM);
-            int *d_rs = h2d(pool, rs, st);
+            const int *d_rs = up.get<int>(u_rs);
             k_region_hist<<<dim3((O1_NCTX * O1_NSYM + 255) / 256, R), 256, 0, st>>>(hist, d_rs, rhist);
             FB2_CHECK_LAUNCH();
         }
-        int *d_tab = h2d(pool, seg_region, st);
         const int ntab = R * O1_NCTX;
         uint16_t *nf = pool.get<uint16_t>((size_t)ntab * O1_NSYM);
         k_o1_norm<<<(ntab + 7) / 8, 256, 0, st>>>(rhist, ntab, nf);
         FB2_CHECK_LAUNCH();
-        int *d_err = pool.get<int>(8);
-        FB2_CUDA(cudaMemsetAsync(d_err, 0, 32, st));
         // the chain encoder's shared-memory image of every table set
         uint32_t *image = pool.get<uint32_t>((size_t)R * (kEncSmem / 4));
         k_o1_ctable<<<ntab, kTabThreads, 0, st>>>(nf, image, d_err);
         FB2_CHECK_LAUNCH();
-        const long long nchains = S * kMaxK;
-        const ChainParts cp = chain_parts(segs, seg_region, K, enc_part);
         // escapes in index order, on the second stream (the host waits here for their count; the
         // histogram pass and the table builds, launched above, run meanwhile)
         const std::vector<unsigned long long> gstart = d2h(d_gstart, (size_t)S + 1, es);
@@ -3802,19 +3830,11 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         tr.gpu("class blocks done", es);
         if (queue_first) FB2_CUDA(cudaStreamWaitEvent(st, tune.queued_ev, 0));
         tr.mark("class blocks launched");
-        // chain output slots
-        std::vector<unsigned long long> soff(nchains + 1, 0);
-        for (long long g = 0; g < S; g++)
-            for (int k = 0; k < kMaxK; k++) {
-                const unsigned long long c = (k < K) ? segs[g].cs * 2 + 64 : 0;
-                soff[g * kMaxK + k + 1] = soff[g * kMaxK + k] + ((c + 15) & ~15ULL);
-            }
-        unsigned long long *d_soff = h2d(pool, soff, st);
+        const unsigned long long *d_soff = up.get<unsigned long long>(u_soff);
         uint8_t *slots = pool.get<uint8_t>(soff.back() + 16);
-        unsigned long long *blen = pool.get<unsigned long long>(nchains);
         tr.mark("tables launched");
         tr.gpu("chain encoder start", st);
-        encode_chains(pool, cp, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
+        encode_chains(pool, cp, up, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
         tr.gpu("chain encoder done", st);
         tr.mark("chains launched");
         // The mantissas go behind the one that ends first: the chain encoder (0.4 ms and 5 ps a code) or the
@@ -3832,15 +3852,18 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         GammaOut go = gamma_finish(gblocks, gwords, es, ms);
         // the chains' escape counts (stream header) from the histogram pass; their sums per segment
         // are the escape groups counted above
-        const std::vector<uint32_t> h_nvk = d2h(nvk, (size_t)S * kMaxK, st);
+        const std::vector<uint32_t> ends = d2h(nvk, n_nvk + 8 + 2 * n_nvk, st);
+        const uint32_t *h_nvk = ends.data();
         for (long long g = 0; g < S; g++) {
             unsigned long long e = 0;
             for (int k = 0; k < K; k++) e += h_nvk[g * kMaxK + k];
             if (e != gstart[g + 1] - gstart[g]) throw std::runtime_error("escape counts of the two passes differ");
         }
         tr.mark("escapes coded");
-        std::vector<unsigned long long> h_blen = d2h(blen, (size_t)nchains, st);
-        std::vector<int> h_err = d2h(d_err, 7, st);
+        int h_err[8];
+        std::memcpy(h_err, h_nvk + n_nvk, sizeof(h_err));
+        std::vector<unsigned long long> h_blen(n_nvk);
+        std::memcpy(h_blen.data(), h_nvk + n_nvk + 8, n_nvk * 8);
         tr.gpu_dump();
         if (h_err[0]) throw std::runtime_error("tANS encoding failed (table construction or chain repair)");
         // Decode checkpoints cost 12 bytes each: keep them within 1.5 % of the chains' bytes by
@@ -3882,8 +3905,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
                          "%lld segments, %d chains each\n", h_err[2], h_err[3], h_err[5], cp.pstart.back(), h_err[6], S, K);
         tr.mark("chains done");
         join();
-        pool.ptrs.insert(pool.ptrs.end(), spool.ptrs.begin(), spool.ptrs.end());
-        spool.ptrs.clear();
+        pool.take(spool);
         for (auto b : h_blen)
             if (b == ~0ULL) throw std::runtime_error("tANS chain overflow");
         as.val<uint64_t>((uint64_t)S);
@@ -4091,9 +4113,8 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
                 else conv_dst.push_back(r.dst);
             }
             if (!conv_dst.empty()) {
-                unsigned long long *d_cd = h2d(spool, conv_dst, fork.side);
                 gamma_decode(spool, d_in, h, cls_off, man_off, man_len, gstart, nullptr, d_err, fork.side, fck, f_part,
-                             n_fck, d_cd, ovf);
+                             n_fck, conv_dst, ovf);
             }
             launch_gather(spool, pcs, reinterpret_cast<uint8_t *>(ovf), fork.side);
             if (ovf_total > 0) {
@@ -4144,10 +4165,13 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         std::vector<EncCta> ctas = item_ctas(chain_table, pstart, kDecThreads);
         for (auto &c : ctas) c.lanes = std::min(32u, (c.count + kDecWarps - 1) / kDecWarps);
         A.in = d_in;
-        A.chains = h2d(pool, chains, st);
-        A.pstart = h2d(pool, pstart, st);
+        Upload up;
+        const size_t u_chains = up.add(chains), u_pstart = up.add(pstart), u_ctas = up.add(ctas);
+        up.send(pool, st);
+        A.chains = up.get<DecChain>(u_chains);
+        A.pstart = up.get<uint32_t>(u_pstart);
         A.nchains = (uint32_t)chains.size();
-        A.ctas = h2d(pool, ctas, st);
+        A.ctas = up.get<EncCta>(u_ctas);
         A.cells = cells;
         A.info = info;
         A.rank = rank;
