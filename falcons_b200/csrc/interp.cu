@@ -801,22 +801,32 @@ __global__ void __launch_bounds__(kFuseThreads, sizeof(T) == 4 ? 8 : 6) k_yx_fus
     const int yl = max(0, y0 - H), yr = min(ny, y1 + H), TR = yr - yl;
     T *plane = xf + a * F.x.sa;
     const long long sy = F.x.sb, sx = F.x.step;  // element steps of one grid unit in y and x
-    // stage rows [yl, yr) x columns [xl, xr) (tile row r, column c: y = yl + r, x = xl + c)
+    const bool zplane = F.has_z && (a & 1);
+    // stage rows [yl, yr) x columns [xl, xr) (tile row r, column c: y = yl + r, x = xl + c).  Decompress needs
+    // the even rows' even columns alone, and nothing of an odd plane: the passes below produce all other points
+    // of the tile before they read them (384^3 f64, the finest level: 340 us with all points staged, now 317).
     constexpr int V = 16 / sizeof(T);
     const bool vec = sx == 1 && ((reinterpret_cast<uintptr_t>(plane + xl) & 15) == 0) && (sy % V == 0) && (TW % V == 0);
     if (vec) {
         // thread (vector slot qq of a row, row group); kFusePW / V slots per row at most
         constexpr int NQ = kFusePW / V, NG = kFuseThreads / NQ;
         const int nq = TW / V, qq = threadIdx.x % NQ, g = threadIdx.x / NQ;
-        if (qq < nq && g < NG) {
-            const T *src = plane + (long long)(yl + g) * sy + xl + qq * V;
-            T *dstp = tile + g * P + qq * V;
-            for (int rr = g; rr < TR; rr += NG, src += NG * sy, dstp += NG * P) {
+        constexpr int RS = DECOMP ? 2 : 1;  // yl is even
+        if (qq < nq && g < NG && !(DECOMP && zplane)) {
+            const T *src = plane + (long long)(yl + RS * g) * sy + xl + qq * V;
+            T *dstp = tile + RS * g * P + qq * V;
+            for (int rr = RS * g; rr < TR; rr += RS * NG, src += RS * NG * sy, dstp += RS * NG * P) {
                 const unsigned sa = (unsigned)__cvta_generic_to_shared(dstp);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
             }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
+    } else if (DECOMP) {
+        const int TR2 = zplane ? 0 : (TR + 1) / 2, TW2 = (TW + 1) / 2;  // yl and xl are even
+        for (int i = threadIdx.x; i < TR2 * TW2; i += blockDim.x) {
+            const int rr = i / TW2, cc = i - rr * TW2;
+            tile[2 * rr * P + 2 * cc] = plane[(yl + 2 * rr) * sy + (xl + 2 * cc) * sx];
+        }
     } else {
         for (int i = threadIdx.x; i < TR * TW; i += blockDim.x) {
             const int rr = i / TW, cc = i - rr * TW;
@@ -825,7 +835,6 @@ __global__ void __launch_bounds__(kFuseThreads, sizeof(T) == 4 ? 8 : 6) k_yx_fus
     }
     __syncthreads();
     // z pass of an odd plane: even rows x even columns of the staged tile
-    const bool zplane = F.has_z && (a & 1);
     if (zplane) {
         const int nz = F.z.n, t = (int)a;
         const bool zl = F.has_zlate && t == nz - 1;
@@ -1074,17 +1083,40 @@ __global__ void __launch_bounds__(kL1Threads, 6) k_l1_fused(const FusedYX F, flo
     const long long sy = F.x.sb, sz = F.x.sa;
     float *plane = xf + (long long)a * sz;
     const int tid = threadIdx.x;
+    const bool zplane = F.has_z && (a & 1);
+    // ---- decompress: the tile's codes on their way to L2 while it is staged (the passes load them where they
+    // use them, each load waiting for memory otherwise)
+    if (DECOMP && x0 + 1 < nx) {
+        const long long c0 = x0 >> 1;
+        long long p = -1;
+        if (tid < 64) {
+            if (y0 + tid < y1) p = F.x.p_base + ((long long)a * F.x.B + y0 + tid) * F.x.C + c0;
+        } else if (tid < 96) {
+            const int t = y0 + 1 + 2 * (tid - 64);
+            if (t < y1 && !(F.has_late && t == ny - 1))
+                p = F.y.p_base + ((long long)a * F.y.rows_in_group + F.y.b_off + ((t - 1) >> 1)) * F.y.C + c0;
+        } else if (tid < 128 && zplane && !(F.has_zlate && a == F.z.n - 1)) {
+            const int y = y0 + 2 * (tid - 96);
+            if (y < y1)
+                p = F.z.p_base + ((long long)((a - 1) >> 1) + F.z.b_off) * F.z.C + (long long)(y >> 1) * F.z.rows_in_group * F.z.C + c0;
+        }
+        if (p >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(codes + p));
+    }
     // ---- stage rows [yo, yo + 72) x grid columns [xo, xo + 72), 16 bytes at a time: four grid
-    // columns per vector at a grid step of one element, two (at element offsets 0 and 2) at two
+    // columns per vector at a grid step of one element, two (at element offsets 0 and 2) at two.  Decompress
+    // needs the even rows' even columns alone, and nothing of an odd plane: the passes below produce all other
+    // points of the tile before they read them (a field of 512^3, this level: 464 us with all points staged,
+    // now 379).
     constexpr int VPR = 72 / (4 / STEP);  // vectors per row
-    constexpr int NV = kL1Rows * VPR;
+    constexpr int RS = DECOMP ? 2 : 1;    // yo is even
+    constexpr int NV = kL1Rows / RS * VPR;
     constexpr int ITER = 3;               // loads in flight per thread before their stores
-    for (int base = 0; base < NV; base += ITER * kL1Threads) {
+    for (int base = 0; base < (DECOMP && zplane ? 0 : NV); base += ITER * kL1Threads) {
         float4 v[ITER];
 #pragma unroll
         for (int k = 0; k < ITER; k++) {
             const int idx = base + tid + k * kL1Threads;
-            const int r = idx / VPR, i = idx - r * VPR;
+            const int r = RS * (idx / VPR), i = idx % VPR;
             const int y = yo + r, x = xo + (4 / STEP) * i;  // the vector's first grid column
             v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (idx < NV && y >= 0 && y < ny) {
@@ -1106,20 +1138,19 @@ __global__ void __launch_bounds__(kL1Threads, 6) k_l1_fused(const FusedYX F, flo
         for (int k = 0; k < ITER; k++) {
             const int idx = base + tid + k * kL1Threads;
             if (idx >= NV) break;
-            const int r = idx / VPR, i = idx - r * VPR;
+            const int r = RS * (idx / VPR), i = idx % VPR;
             if (STEP == 1) {
                 *reinterpret_cast<float2 *>(l1_e(E, r, 2 * i)) = make_float2(v[k].x, v[k].z);
-                *reinterpret_cast<float2 *>(l1_o(O, r, 2 * i)) = make_float2(v[k].y, v[k].w);
+                if (!DECOMP) *reinterpret_cast<float2 *>(l1_o(O, r, 2 * i)) = make_float2(v[k].y, v[k].w);
             } else {
                 *l1_e(E, r, i) = v[k].x;
-                *l1_o(O, r, i) = v[k].z;
+                if (!DECOMP) *l1_o(O, r, i) = v[k].z;
             }
         }
     }
     __syncthreads();
     // ---- z pass of an odd plane t = a: even rows x even columns, operands in the even planes
     // around it (points of coarser levels, which this level never writes)
-    const bool zplane = F.has_z && (a & 1);
     if (zplane) {
         const int nz = F.z.n, t = a;
         const bool zl = F.has_zlate && t == nz - 1;
