@@ -3384,25 +3384,45 @@ __global__ void k_region_hist(const uint32_t *__restrict__ seg_hist, const int *
     reg_hist[(size_t)r * O1_NCTX * O1_NSYM + i] = s;
 }
 
+// Sixteen codes of a thread in eight words (16-byte vectors when the code array is 16-byte aligned: tile starts
+// are multiples of 16 codes), zeros past the end, and which of them are escapes (bit j: code j).  An escape is
+// what clamping to -127 .. 127 changes, two codes at a time.
+__device__ __forceinline__ uint32_t escape_mask(const int16_t *__restrict__ q, long long n, long long base,
+                                                uint32_t (&w)[8]) {
+    static_assert(kScanItems == 16, "two 16-byte vectors per thread");
+    if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+        const uint4 *p4 = reinterpret_cast<const uint4 *>(q + base);
+        const uint4 a = __ldg(p4), b = __ldg(p4 + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const long long i = base + 2 * k;
+            w[k] = (i < n ? (uint32_t)(uint16_t)q[i] : 0u) | (i + 1 < n ? (uint32_t)(uint16_t)q[i + 1] << 16 : 0u);
+        }
+    }
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint32_t d = __vmins2(__vmaxs2(w[k], 0xFF81FF81u), 0x007F007Fu) ^ w[k];
+        if (d & 0xFFFFu) m |= 1u << (2 * k);
+        if (d >> 16) m |= 2u << (2 * k);
+    }
+    return m;
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_esc_tiles(const int16_t *__restrict__ q, long long n,
                                                            uint32_t *__restrict__ cnt) {
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
-    uint32_t c = 0;
-    // 16-byte vectors when the code array is 16-byte aligned (tile starts are multiples of 16 codes)
-    if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
-        const int4 *p4 = reinterpret_cast<const int4 *>(q + base);
-        const int4 a = __ldg(p4), b = __ldg(p4 + 1);
-        const int32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int j = 0; j < kScanItems; j++)
-            c += o1_sym((int16_t)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xFFFF)) == O1_NSYM - 1;
-    } else {
-        for (long long i = base; i < n && i < base + kScanItems; i++) c += o1_sym(q[i]) == O1_NSYM - 1;
-    }
-    __shared__ uint32_t sh[32];
-    uint32_t tot;
-    block_excl_scan<uint32_t>(c, sh, tot);
-    if (threadIdx.x == 0) cnt[blockIdx.x] = tot;
+    uint32_t w[8];
+    const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(escape_mask(q, n, base, w)));
+    __shared__ uint32_t total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31u) == 0 && c) atomicAdd(&total, c);
+    __syncthreads();
+    if (threadIdx.x == 0) cnt[blockIdx.x] = total;
 }
 
 // Escapes before each of npos code positions: the tile offset of the position's tile (exclusive
@@ -3415,38 +3435,30 @@ __global__ void __launch_bounds__(256) k_esc_before(const int16_t *__restrict__ 
     if (w >= npos) return;
     const unsigned long long p = pos[w], t = p / kScanTile;
     uint32_t c = 0;
-    for (unsigned long long i = t * kScanTile + lane; i < p; i += 32) c += o1_sym(q[i]) == O1_NSYM - 1;
+    uint32_t v[8];
+    for (unsigned long long i = t * kScanTile + kScanItems * lane; i < p; i += 32 * kScanItems)
+        c += (uint32_t)__popc(escape_mask(q, (long long)p, (long long)i, v));
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) out[w] = (unsigned long long)tile_off[t] + c;
 }
 
+// The escapes in index order, and their classes.  Bound by issue: testing the codes as symbols, twice, took 33
+// instructions a code (134 M codes: 183 us; k_esc_tiles 62), the masks take 97 (56).
 __global__ void __launch_bounds__(kScanThreads) k_esc_extract(const int16_t *__restrict__ q, long long n,
                                                              const uint32_t *__restrict__ tile_off,
                                                              uint8_t *__restrict__ cls, int16_t *__restrict__ raw) {
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
-    int16_t v[kScanItems];
-    uint32_t c = 0;
-    static_assert(kScanItems == 16, "two 16-byte vectors per thread");
-    if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
-        const int4 *p4 = reinterpret_cast<const int4 *>(q + base);
-        const int4 a = __ldg(p4), b = __ldg(p4 + 1);
-        const int32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int j = 0; j < kScanItems; j++) v[j] = (int16_t)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xFFFF);
-    } else {
-#pragma unroll
-        for (int j = 0; j < kScanItems; j++) v[j] = base + j < n ? q[base + j] : (int16_t)0;
-    }
-#pragma unroll
-    for (int j = 0; j < kScanItems; j++) c += (base + j < n && o1_sym(v[j]) == O1_NSYM - 1);
+    uint32_t w[8];
+    const uint32_t m = escape_mask(q, n, base, w);
     __shared__ uint32_t sh[32];
     // the tile's escapes are staged in shared memory in order, then leave as contiguous runs
     __shared__ int16_t sv[kScanTile];
     uint32_t tot;
-    uint32_t r = block_excl_scan<uint32_t>(c, sh, tot);
+    int16_t *at = sv + block_excl_scan<uint32_t>((uint32_t)__popc(m), sh, tot);
+    if (m) {
 #pragma unroll
-    for (int j = 0; j < kScanItems; j++) {
-        if (base + j < n && o1_sym(v[j]) == O1_NSYM - 1) sv[r++] = v[j];
+        for (int j = 0; j < kScanItems; j++)
+            if ((m >> j) & 1u) *at++ = (int16_t)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xFFFFu);
     }
     __syncthreads();
     const uint32_t t0 = tile_off[blockIdx.x];
@@ -3456,8 +3468,6 @@ __global__ void __launch_bounds__(kScanThreads) k_esc_extract(const int16_t *__r
         raw[t0 + k] = e;
     }
 }
-
-
 
 __global__ void k_m0_scatter(const uint32_t *__restrict__ runs, const uint32_t *__restrict__ vals,
                              const unsigned long long *__restrict__ start, long long nv, long long n,
