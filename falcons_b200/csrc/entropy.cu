@@ -2118,7 +2118,8 @@ struct ChainCta {
 // All 15 context state tables stay in shared memory, as 13-bit entries (state - 8192) packed into
 // words, so that no lookup leaves the SM and every context takes the same instructions (two 16-bit
 // tables beside 13 packed ones cost every warp both paths); two words per key hold the symbol
-// transform (one word fits too, but takes a dozen more instructions a code to unpack).  k_o1_ctable lays this image out once per table set; every CTA copies it in.
+// transform (one word fits too, but takes a dozen more instructions a code to unpack).  k_o1_ctable
+// lays this image out once per table set; every CTA copies it in.
 constexpr int kEncThreads = 1024;
 constexpr uint32_t kEncWarps = 4, kMinEncPart = 512;
 constexpr int kKeptShift = 6;  // kept states: every 64th index
@@ -2142,8 +2143,8 @@ struct EncArgs {
     const uint32_t *image;       // table sets, kEncSmem bytes each
     const EncCta *ctas;
     // per part: exit state of the first walk and of the last one, entering state of the last one (map
-    // path: the exact one, written ahead of its walk), bits, escapes, first record | lanes << 56, first bit in the slots, records to place (bit
-    // 31: and the final state's)
+    // path: the exact one, written ahead of its walk), bits, escapes, first record | lanes << 56, first bit
+    // in the slots, records to place (bit 31: and the final state's)
     uint16_t *exit1, *exit2, *entry;
     uint32_t *bits, *esc, *nrec;
     unsigned long long *column, *at;
@@ -2276,8 +2277,8 @@ struct EncTables {
     }
 };
 
-// Codes keys[first] down to keys[a] by the vectors of 8 keys they lie in, fetched ahead: f(i, r, n, v) for every record r of n bits, i its lowest index and v its keys (only whole
-// vectors: `whole`); stops and returns true where f does.
+// Codes keys[first] down to keys[a] by the vectors of 8 keys they lie in, fetched ahead: f(i, r, n, v)
+// for every record r of n bits, i its lowest index and v its keys (only whole vectors: `whole`); stops and returns true where f does.
 template <class F>
 __device__ __forceinline__ bool walk_records(const uint16_t *__restrict__ keys, long long first,
                                              long long a, uint32_t &x, F &&f) {
@@ -2436,7 +2437,7 @@ __global__ void __launch_bounds__(kEncThreads) k_o1_repair(const EncArgs A) {
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31u, item = wid * w.lanes + lane;
     uint32_t steps = 0, unmet = 0;
     if (lane < w.lanes && item < w.count) {
-            const uint32_t id = w.first + item;
+        const uint32_t id = w.first + item;
         const EncPartPos P = enc_part(A, id, w.chain);
         if (!P.is_top) {
             uint32_t x = A.exit1[id + 1], bits = A.bits[id];
@@ -2460,9 +2461,9 @@ __global__ void __launch_bounds__(kEncThreads) k_o1_repair(const EncArgs A) {
 // millions of codes, and the exact states would have to pass down a chain part by part (249 rounds,
 // 36 ms, for 1800 x 3600 points at 1.4 bits a code).  Instead every run of parts (a super part) is
 // coded from all 8192 entering states at once, as the map from its entering to its leaving state:
-//   k_o1_maps     W warps a super part (four where the SMs hold few of them).  A step keeps the cyclic order of the states (within a
-//                 symbol the next state grows with the state), so states that have become equal are
-//                 neighbours: after 8, 16, 32 .. 512 codes and at every part end, neighbours that are equal
+//   k_o1_maps     W warps a super part (four where the SMs hold few of them).  A step keeps the cyclic
+//                 order of the states (within a symbol the next state grows with the state), so states
+//                 that have become equal are neighbours: after 8, 16, 32 .. 512 codes and at every part end, neighbours that are equal
 //                 are merged into one class (about 8192 / (s sqrt(n)) classes are left after n codes,
 //                 with s the rounding of a step).  Every merge stores the map from the classes
 //                 before it to those after, and the classes' states.
@@ -3778,6 +3779,17 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
             ~Join() { (*this)(); }
         } join{fork, st, es, tune.join_ev};
         Pool spool(es);  // scratch of the escape side stream, handed to `pool` once joined
+        struct Hold {  // should a call fail: scratch of `es` that `st` reads is not given back before it is read
+            bool on;
+            cudaStream_t st, es;
+            cudaEvent_t ev;
+            ~Hold() {
+                if (on) {
+                    cudaEventRecord(ev, st);
+                    cudaStreamWaitEvent(es, ev, 0);
+                }
+            }
+        } hold{false, st, es, tune.fork_ev};
         if (N > 0) {
             k_esc_tiles<<<(unsigned)tiles, kScanThreads, 0, es>>>(q, N, tcnt);
             FB2_CHECK_LAUNCH();
@@ -3857,6 +3869,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
                                  (double)((gblocks.jobs.size() + kFseGroups * sm_count() - 1) / (kFseGroups * sm_count()));
         const bool behind_chains = queue_first && chain_ns < blocks_ns;
         cudaStream_t ms = behind_chains ? st : es;
+        hold.on = behind_chains;
         const GammaWords gwords = gamma_pack(behind_chains ? pool : spool, ecls, gstart, eraw, ms);
         tr.gpu("escape mantissas packed", ms);
         GammaOut go = gamma_finish(gblocks, gwords, es, ms);
@@ -3916,6 +3929,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         tr.mark("chains done");
         join();
         pool.take(spool);
+        hold.on = false;
         for (auto b : h_blen)
             if (b == ~0ULL) throw std::runtime_error("tANS chain overflow");
         as.val<uint64_t>((uint64_t)S);
