@@ -4058,6 +4058,9 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         if (S == 0) S = 1;
         if (S > (unsigned long long)std::max<long long>(N, 1)) throw std::invalid_argument("invalid segment count");
         const unsigned long long seg = ((unsigned long long)N + S - 1) / S;
+        // the decoder and the fill store codes as 16-byte vectors: for an output off 16 bytes they work on scratch
+        const bool aligned = (reinterpret_cast<uintptr_t>(d_codes) & 15) == 0;
+        int16_t *const out = aligned ? d_codes : pool.get<int16_t>((size_t)N);
         std::vector<DecChain> chains;
         std::vector<size_t> nf_off(S);
         std::vector<size_t> cls_off, man_off, man_len;
@@ -4203,7 +4206,7 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         A.n_ovf = ovf_total;
         A.cks = parts_ok ? o1ck : nullptr;
         A.part = part;
-        A.out = d_codes;
+        A.out = out;
         A.tile = pool.get<unsigned long long>((size_t)N / kFillTile + 1);
         A.err = d_err;
         enable_big_smem();
@@ -4216,9 +4219,10 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         tr.gpu("chains decoded", st);
         if (ovf_total > 0) {
             const long long per = 8ll * kFillTiles * kFillTile;  // codes a CTA
-            k_o1_fill<<<(unsigned)((N + per - 1) / per), 256, 0, st>>>(d_codes, N, A.tile, ovf, ovf_total);
+            k_o1_fill<<<(unsigned)((N + per - 1) / per), 256, 0, st>>>(out, N, A.tile, ovf, ovf_total);
             FB2_CHECK_LAUNCH();
         }
+        if (!aligned) FB2_CUDA(cudaMemcpyAsync(d_codes, out, (size_t)N * 2, cudaMemcpyDeviceToDevice, st));
     } else {
         throw std::invalid_argument("unsupported entropy method");
     }

@@ -131,6 +131,8 @@ int falcons_interp_decompress(falcons_ctx *ctx, int dtype, const size_t *dims, i
 int falcons_device_range(falcons_ctx *ctx, int dtype, const void *d_data, size_t n, double *range_out, void *stream);
 int falcons_encode_codes(falcons_ctx *ctx, const int16_t *d_codes, size_t n, void *d_out, size_t cap,
                          size_t *out_len, void *stream);
+/* d_codes may start at any int16_t address; from one off 16 bytes on, order-1 payloads take n codes of scratch
+ * and a copy more. */
 int falcons_decode_codes(falcons_ctx *ctx, const void *d_in, size_t len, size_t n, int16_t *d_codes, void *stream);
 
 /* ---- batches of fields (device memory) ----
