@@ -19,6 +19,7 @@
 
 #include "assemble.cuh"
 #include "entropy.cuh"
+#include "entropy_rules.cuh"
 #include "fse.cuh"
 #include "scan.cuh"
 
@@ -3159,7 +3160,9 @@ __global__ void __launch_bounds__(256) k_o1_fill(int16_t *__restrict__ codes, lo
         if (cnt == 0) continue;
         const unsigned long long e = at[k] + incl - cnt;
         const int16_t *src = ovf + e;
-        const bool have = e + cnt <= n_ovf;  // else a damaged stream: its values are not read
+        // else a damaged stream, whose values are not read: a part that gave up has written neither its codes nor
+        // its tiles, so e can be any number
+        const bool have = range_within(e, cnt, n_ovf);
         uint32_t val[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {

@@ -1,0 +1,37 @@
+"""Rules of the entropy stage that guard its memory accesses, compiled for the host (tests/native/entropy_rules.cu)
+and checked against unbounded integers."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SRC = os.path.join(ROOT, "tests", "native", "entropy_rules.cu")
+HDR = os.path.join(ROOT, "falcons_b200", "csrc", "entropy_rules.cuh")
+OUT = os.path.join(ROOT, "tests", "native", "_build", "libentropy_rules.so")
+
+
+@pytest.fixture(scope="module")
+def rules():
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    if not os.path.exists(OUT) or os.path.getmtime(OUT) < max(os.path.getmtime(SRC), os.path.getmtime(HDR)):
+        os.makedirs(os.path.dirname(OUT), exist_ok=True)
+        subprocess.check_call([nvcc, "-std=c++17", "-O2", "-shared", "-Xcompiler", "-fPIC", "-x", "cu",
+                               "-gencode", "arch=compute_100a,code=sm_100a", SRC, "-o", OUT])
+    lib = ctypes.CDLL(OUT)
+    lib.rules_range_within.argtypes = [ctypes.c_ulonglong] * 3
+    return lib
+
+
+@pytest.mark.parametrize("n", [0, 1, 7, 8, 1000, 1 << 33])
+@pytest.mark.parametrize("count", [0, 1, 2, 8])
+def test_escapes_of_a_lane_lie_in_the_list(rules, n, count):
+    """The fill takes a lane's first escape from scratch that a damaged stream's part may not have written: a
+    number near 2^64, whose sum with the count wraps, must not pass as a place in the list."""
+    firsts = [0, 1, max(n - count, 0), max(n - count, 0) + 1, n, n + 1, 1 << 63] + [2 ** 64 - d for d in range(1, 10)]
+    for first in firsts:
+        assert bool(rules.rules_range_within(first, count, n)) == (first + count <= n), (first, count, n)
