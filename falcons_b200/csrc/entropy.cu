@@ -3094,10 +3094,10 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
     };
     // where no lane of the warp is to meet an escape, a quarter of a step's instructions are left out
     if (__all_sync(__activemask(), oi0 + oi == eend)) {
-        while (j + 8 <= n) eight(std::false_type());
+        while (n - j >= 8) eight(std::false_type());
         if (seen & 0x10000u) atomicExch(A.cks ? A.err + 1 : A.err, 7);
     } else {
-        while (j + 8 <= n) eight(std::true_type());
+        while (n - j >= 8) eight(std::true_type());
     }
     signs();
     for (; j < n; j++) single(j);
@@ -4185,11 +4185,13 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
             parts_ok = tot == n_o1ck;
         }
         // without checkpoints a chain is one part
-        const unsigned long long part = parts_ok ? o1_part : 1ull << 31;
+        const unsigned long long part = parts_ok ? o1_part : kWholeChain;
         std::vector<uint32_t> pstart(chains.size() + 1, 0);
         std::vector<int> chain_table(chains.size());
         for (size_t i = 0; i < chains.size(); i++) {
-            pstart[i + 1] = pstart[i] + (chains[i].n ? 1 + (uint32_t)((chains[i].n - 1) / part) : 0);
+            const unsigned long long np = chain_part_count(chains[i].n, parts_ok ? o1_part : 0);
+            if (np == ~0ull) throw std::invalid_argument("tANS chain without checkpoints too long");
+            pstart[i + 1] = pstart[i] + (uint32_t)np;
             chain_table[i] = chains[i].table;
         }
         std::vector<EncCta> ctas = item_ctas(chain_table, pstart, kDecThreads);

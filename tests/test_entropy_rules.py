@@ -24,6 +24,8 @@ def rules():
                                "-gencode", "arch=compute_100a,code=sm_100a", SRC, "-o", OUT])
     lib = ctypes.CDLL(OUT)
     lib.rules_range_within.argtypes = [ctypes.c_ulonglong] * 3
+    lib.rules_chain_part_count.argtypes = [ctypes.c_ulonglong] * 2
+    lib.rules_chain_part_count.restype = ctypes.c_ulonglong
     return lib
 
 
@@ -35,3 +37,13 @@ def test_escapes_of_a_lane_lie_in_the_list(rules, n, count):
     firsts = [0, 1, max(n - count, 0), max(n - count, 0) + 1, n, n + 1, 1 << 63] + [2 ** 64 - d for d in range(1, 10)]
     for first in firsts:
         assert bool(rules.rules_range_within(first, count, n)) == (first + count <= n), (first, count, n)
+
+
+@pytest.mark.parametrize("n", [0, 1, 1 << 20, (1 << 31) - 1, 1 << 31, (1 << 31) + 1, (1 << 32) - 1, 1 << 32, 1 << 40])
+def test_parts_of_a_chain(rules, n):
+    """A chain without checkpoints is one part whatever its length (a second part would start from a checkpoint
+    that there is none of); one beyond the decoder's 32-bit count is refused."""
+    whole = 0 if n == 0 else 1 if n < 1 << 32 else 2 ** 64 - 1
+    assert rules.rules_chain_part_count(n, 0) == whole
+    for part in (64, 1024, 65536):
+        assert rules.rules_chain_part_count(n, part) == -(-n // part)
