@@ -2953,6 +2953,7 @@ struct DecArgs {
     int16_t *out;
     unsigned long long *tile;  // escapes before every kFillTile-th code
     int *err;
+    int *over;                 // set by a chain with more escapes than `nesc`
 };
 __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A) {
     extern __shared__ uint4 smem_raw[];
@@ -3095,13 +3096,13 @@ __global__ void __launch_bounds__(kDecThreads) k_o1_decode_parts(const DecArgs A
     // where no lane of the warp is to meet an escape, a quarter of a step's instructions are left out
     if (__all_sync(__activemask(), oi0 + oi == eend)) {
         while (n - j >= 8) eight(std::false_type());
-        if (seen & 0x10000u) atomicExch(A.cks ? A.err + 1 : A.err, 7);
+        if (seen & 0x10000u) atomicExch(A.cks ? A.err + 1 : A.over, 7);
     } else {
         while (n - j >= 8) eight(std::true_type());
     }
     signs();
     for (; j < n; j++) single(j);
-    if (oi > avail) atomicExch(A.err, 7);
+    if (oi > avail) atomicExch(A.over, 7);
     if (!last) {
         const O1Ckpt k = A.cks[ch.ck + pt];
         if (k.state != s - O1_M || k.ctx != ctx_of(slot) || br.pos != bit0 + (int32_t)k.bitpos ||
@@ -4000,8 +4001,9 @@ bool parse_ckpt_header(const uint8_t *h, const uint8_t *d_content, size_t avail,
     return true;
 }
 
-size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size_t n, int16_t *d_codes,
-                      cudaStream_t st, const DecodeCheckpoints *ck) {
+// `counts`: a chain's escape count in the header bounds its escapes; else it only says where its values start.
+static size_t decode_payload(Context &ctx, const uint8_t *d_in, const ByteView &h, size_t n, int16_t *d_codes,
+                             cudaStream_t st, const DecodeCheckpoints *ck, bool counts) {
     Trace tr("decode");
     Pool pool(st);
     tr.gpu("decode begin", st);
@@ -4184,6 +4186,9 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
             }
             parts_ok = tot == n_o1ck;
         }
+        if (!counts)
+            for (auto &c : chains)
+                c.nesc = (uint32_t)std::min<unsigned long long>(ovf_total - std::min(ovf_total, c.ovf), 0xFFFFFFFFull);
         // without checkpoints a chain is one part
         const unsigned long long part = parts_ok ? o1_part : kWholeChain;
         std::vector<uint32_t> pstart(chains.size() + 1, 0);
@@ -4214,6 +4219,8 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
         A.out = out;
         A.tile = pool.get<unsigned long long>((size_t)N / kFillTile + 1);
         A.err = d_err;
+        // without checkpoints, more escapes than the header counts have the payload decoded again without the counts
+        A.over = counts && !parts_ok ? d_err + 1 : d_err;
         enable_big_smem();
         fork.join();  // the chains consume the escapes' signs
         tr.mark("parts listed");
@@ -4240,10 +4247,16 @@ size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size
     if (he[1] && ck) {
         // a checkpoint did not match the stream: decode again, sequentially
         if (tr.on) std::fprintf(stderr, "[falcons trace] decode checkpoint mismatch: decoding sequentially\n");
-        return entropy_decode(ctx, d_in, h, n, d_codes, st, nullptr);
+        return decode_payload(ctx, d_in, h, n, d_codes, st, nullptr, true);
     }
+    if (he[1]) return decode_payload(ctx, d_in, h, n, d_codes, st, nullptr, false);
     if (he[0]) throw std::invalid_argument("Invalid or corrupted Falcons entropy payload");
     return off;
+}
+
+size_t entropy_decode(Context &ctx, const uint8_t *d_in, const ByteView &h, size_t n, int16_t *d_codes,
+                      cudaStream_t st, const DecodeCheckpoints *ck) {
+    return decode_payload(ctx, d_in, h, n, d_codes, st, ck, true);
 }
 
 

@@ -71,3 +71,36 @@ def test_a_checkpoint_out_of_range_is_not_used(cuda, field, value):
         got, _ = D.decompress(torch.from_numpy(b).to(cuda), torch.float32)
         s.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("spread", ["some", "none in the first", "none counted"])
+def test_escape_counts_of_the_header_only_place_the_values(cuda, spread):
+    """A chain's escape count says where its values start, no more: with equal values the counts of neighbours may
+    differ from what the chains hold, and the payload decodes as it is."""
+    import torch
+    from falcons_b200 import device as D
+    n = 76800 + 41
+    rng = np.random.default_rng(5)
+    q = rng.integers(-20, 21, n)
+    at = rng.choice(n, 3000, replace=False)
+    if spread == "none in the first":
+        at = at[at > n // 2]
+    q[at] = 777
+    q = torch.from_numpy(q.astype(np.int16)).to(cuda)
+    torch.cuda.synchronize()
+    enc = D.encode_codes(q).cpu().numpy()
+    k = int(enc[21:29].view(np.uint64)[0])
+    nvk = enc[29 + 8 * k:29 + 16 * k].view(np.uint64)
+    assert k == 16 and int(nvk.sum()) == at.size and nvk[8] > 2 and (nvk[0] == 0) == (spread == "none in the first")
+    d = enc.copy()
+    counts = d[29 + 8 * k:29 + 16 * k].view(np.uint64)
+    moved = counts[8] if spread == "none counted" else 2
+    counts[8] -= moved
+    counts[15] += moved - 1
+    counts[0] += 1
+    back = D.decode_codes(torch.from_numpy(d).to(cuda), n)
+    torch.cuda.synchronize()
+    assert torch.equal(back, q)
+    counts[0] += 1  # more values than the payload holds
+    with pytest.raises(ValueError):
+        D.decode_codes(torch.from_numpy(d).to(cuda), n)
