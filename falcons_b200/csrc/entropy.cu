@@ -697,23 +697,21 @@ constexpr int kFseDecThreads = 64;  // parts of a block decode one per thread
 constexpr unsigned kPartPad = 4;     // bytes between the parts' regions of the decoded block (>= 2:
                                      // the last part may hold two symbols past `part`)
 // Dynamic shared memory: the decoded block (FBLK symbols plus kPartPad per part), which the table's spread
-// uses first, then the decode table, when its log is at most kFseDecLog (a larger one, which no encoder
-// here writes, goes to `big`): 76 KB at parts of 1024 symbols, three blocks an SM.  (With room for the
-// largest table two fitted: 310 against 217 us for 758 blocks.)
+// uses first, then the decode table: 76 KB at parts of 1024 symbols, three blocks an SM.  (With room for the
+// largest table two fitted: 310 against 217 us for 758 blocks.)  A table of a log above kFseDecLog, which no
+// encoder here writes, takes the decoded block's place behind the spread, and its symbols go straight out.
 constexpr unsigned kFseDecLog = 11;
+static_assert((1 << fse::kMaxTableLog) * (1 + sizeof(fse::DEntry)) <= FBLK, "spread and largest table fit the block's place");
 inline size_t fse_dec_smem(uint32_t part) { return FBLK + (FBLK / part) * kPartPad + (sizeof(fse::DEntry) << kFseDecLog); }
 __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint8_t *__restrict__ in,
                                                          const BlockJob *__restrict__ jobs,
                                                          uint8_t *__restrict__ cls, int *__restrict__ err,
-                                                         uint32_t part, const FseCkpt *__restrict__ cks,
-                                                         fse::DEntry *__restrict__ big) {
+                                                         uint32_t part, const FseCkpt *__restrict__ cks) {
     __shared__ int16_t s_norm[256];
     __shared__ uint32_t s_scan[257], s_next[256];
     __shared__ unsigned tl_sh, hdr_sh, maxsv_sh, high_sh;
     extern __shared__ uint4 s_out4[];
     uint8_t *s_out = reinterpret_cast<uint8_t *>(s_out4), *sym = s_out;
-    fse::DEntry *const s_dt = reinterpret_cast<fse::DEntry *>(s_out + FBLK + (FBLK / part) * kPartPad);
-    fse::DEntry *const g_dt = big + ((size_t)blockIdx.x << fse::kMaxTableLog);
     const BlockJob jb = jobs[blockIdx.x];
     uint8_t *dst = cls + jb.src;
     const uint8_t *p = in + jb.in;
@@ -756,6 +754,9 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
     __syncthreads();
     const unsigned tl = tl_sh;
     if (tl == 0xFFFFFFFFu) return;
+    const bool big = tl > kFseDecLog;
+    fse::DEntry *const dt = reinterpret_cast<fse::DEntry *>(
+        s_out + (big ? 1u << fse::kMaxTableLog : FBLK + (FBLK / part) * kPartPad));
     if (threadIdx.x < 32) {  // the table, by the first warp
         const unsigned lane = threadIdx.x, L = 1u << tl, maxSV = maxsv_sh;
         const uint32_t step = fse::table_step(L), mask = L - 1, high = high_sh;
@@ -796,8 +797,7 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
                 e.symbol = (uint8_t)sv;
                 e.nbBits = (uint8_t)nb;
                 e.newState = (uint16_t)((ns << nb) - L);
-                if (tl <= kFseDecLog) s_dt[u] = e;
-                else g_dt[u] = e;
+                dt[u] = e;
             }
             __syncwarp();
             if (u < L && rank == (unsigned)__popc(peers) - 1u) s_next[sv] += rank + 1;
@@ -809,7 +809,8 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
     const uint32_t ssz = (uint32_t)(size - hdr_sh);
     const unsigned n = jb.n;
     const unsigned nparts = jb.ck == 0xFFFFFFFFu ? 1u : 1u + fse_ckpt_count(n, part);
-    auto decode = [&](unsigned q, const fse::DEntry *dt) {
+    auto decode = [&](unsigned q, auto big_tag) {
+        constexpr bool BIG = decltype(big_tag)::value;
         BackWindow br;
         uint32_t s0, s1;
         int32_t bit0;
@@ -838,7 +839,7 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
         }
         // Part q's symbols go to its own region of shared memory, kPartPad bytes more than a part
         // apart, four to a word: the parts' word stores then fall on different banks.
-        uint8_t *so = s_out + (size_t)q * (nparts > 1 ? part + kPartPad : 0u);
+        uint8_t *so = BIG ? dst + start : s_out + (size_t)q * (nparts > 1 ? part + kPartPad : 0u);
         auto pair = [&]() -> uint32_t {  // two symbols; at most 2 * 13 bits
             const fse::DEntry e0 = dt[s0];
             const fse::DEntry e1 = dt[s1];
@@ -847,7 +848,7 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
             return (uint32_t)e0.symbol | ((uint32_t)e1.symbol << 8);
         };
         unsigned i = start;
-        for (; i + 3 < end; i += 4) {
+        for (; !BIG && i + 3 < end; i += 4) {
             const uint32_t lo = pair(), hi = pair();
             br.align();
             *reinterpret_cast<uint32_t *>(so + (i - start)) = lo | (hi << 16);
@@ -864,10 +865,11 @@ __global__ void __launch_bounds__(kFseDecThreads) k_fse_decode_blocks(const uint
             if (c.s0 != s0 || c.s1 != s1 || br.pos != bit0 + (int32_t)c.bitpos) atomicExch(err + 1, 1);
         }
     };
-    if (tl <= kFseDecLog)
-        for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, s_dt);
-    else
-        for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, g_dt);
+    if (big) {
+        for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, std::true_type());
+        return;
+    }
+    for (unsigned q = threadIdx.x; q < nparts; q += blockDim.x) decode(q, std::false_type());
     // the symbols leave in consecutive bytes across the CTA (each thread's part decoded into
     // shared memory, so that no warp store scatters over the parts)
     __syncthreads();
@@ -3531,9 +3533,8 @@ void gamma_decode(Pool &pool, const uint8_t *d, const ByteView &h,
                              *d_gdst = gdst.empty() ? nullptr : up.get<unsigned long long>(u_gdst);
     uint8_t *cls = pool.get<uint8_t>(T);
     enable_fse_smem();
-    fse::DEntry *big = pool.get<fse::DEntry>(jobs.size() << fse::kMaxTableLog);
     const uint32_t dpart = fpart ? fpart : FBLK;
-    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, fse_dec_smem(dpart), st>>>(d, dj, cls, d_err, dpart, d_fck, big);
+    k_fse_decode_blocks<<<(unsigned)jobs.size(), kFseDecThreads, fse_dec_smem(dpart), st>>>(d, dj, cls, d_err, dpart, d_fck);
     FB2_CHECK_LAUNCH();
     unsigned long long *usum = pool.get<unsigned long long>(NU + 1);
     unsigned long long *uoff = pool.get<unsigned long long>(NU + 1);

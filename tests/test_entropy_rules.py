@@ -9,7 +9,7 @@ import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "native", "entropy_rules.cu")
-HDR = os.path.join(ROOT, "falcons_b200", "csrc", "entropy_rules.cuh")
+HDRS = [os.path.join(ROOT, "falcons_b200", "csrc", h) for h in ("entropy_rules.cuh", "fse.cuh")]
 OUT = os.path.join(ROOT, "tests", "native", "_build", "libentropy_rules.so")
 
 
@@ -18,7 +18,7 @@ def rules():
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not available")
-    if not os.path.exists(OUT) or os.path.getmtime(OUT) < max(os.path.getmtime(SRC), os.path.getmtime(HDR)):
+    if not os.path.exists(OUT) or os.path.getmtime(OUT) < max(map(os.path.getmtime, [SRC, *HDRS])):
         os.makedirs(os.path.dirname(OUT), exist_ok=True)
         subprocess.check_call([nvcc, "-std=c++17", "-O2", "-shared", "-Xcompiler", "-fPIC", "-x", "cu",
                                "-gencode", "arch=compute_100a,code=sm_100a", SRC, "-o", OUT])
@@ -26,6 +26,7 @@ def rules():
     lib.rules_range_within.argtypes = [ctypes.c_ulonglong] * 3
     lib.rules_chain_part_count.argtypes = [ctypes.c_ulonglong] * 2
     lib.rules_chain_part_count.restype = ctypes.c_ulonglong
+    lib.rules_fse_block.restype = ctypes.c_longlong
     return lib
 
 
