@@ -3131,7 +3131,8 @@ __global__ void __launch_bounds__(256) k_sign_bits(const int16_t *__restrict__ v
 constexpr uint32_t kFillTiles = 4;
 __global__ void __launch_bounds__(256) k_o1_fill(int16_t *__restrict__ codes, long long n,
                                                  const unsigned long long *__restrict__ tile,
-                                                 const int16_t *__restrict__ ovf, unsigned long long n_ovf) {
+                                                 const int16_t *__restrict__ ovf, unsigned long long n_ovf,
+                                                 const int2 *__restrict__ err) {
     const uint32_t lane = threadIdx.x & 31u;
     const long long t0 = ((long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * kFillTiles;
     uint4 v[kFillTiles];
@@ -3142,6 +3143,9 @@ __global__ void __launch_bounds__(256) k_o1_fill(int16_t *__restrict__ codes, lo
         v[k] = i0 + 8 <= n ? *reinterpret_cast<const uint4 *>(codes + i0) : make_uint4(0, 0, 0, 0);
         at[k] = (t0 + k) * (long long)kFillTile < n ? tile[t0 + k] : 0;
     }
+    // a part that gave up has written neither its codes nor its tiles, and the call fails or decodes again
+    const int2 failed = *err;
+    if (failed.x | failed.y) return;
 #pragma unroll
     for (uint32_t k = 0; k < kFillTiles; k++) {
         const long long i0 = (t0 + k) * kFillTile + lane * 8;
@@ -3163,9 +3167,7 @@ __global__ void __launch_bounds__(256) k_o1_fill(int16_t *__restrict__ codes, lo
         if (cnt == 0) continue;
         const unsigned long long e = at[k] + incl - cnt;
         const int16_t *src = ovf + e;
-        // else a damaged stream, whose values are not read: a part that gave up has written neither its codes nor
-        // its tiles, so e can be any number
-        const bool have = range_within(e, cnt, n_ovf);
+        const bool have = e + cnt <= n_ovf;  // else a damaged stream: its values are not read
         uint32_t val[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
@@ -4232,7 +4234,7 @@ static size_t decode_payload(Context &ctx, const uint8_t *d_in, const ByteView &
         tr.gpu("chains decoded", st);
         if (ovf_total > 0) {
             const long long per = 8ll * kFillTiles * kFillTile;  // codes a CTA
-            k_o1_fill<<<(unsigned)((N + per - 1) / per), 256, 0, st>>>(out, N, A.tile, ovf, ovf_total);
+            k_o1_fill<<<(unsigned)((N + per - 1) / per), 256, 0, st>>>(out, N, A.tile, ovf, ovf_total, reinterpret_cast<const int2 *>(d_err));
             FB2_CHECK_LAUNCH();
         }
         if (!aligned) FB2_CUDA(cudaMemcpyAsync(d_codes, out, (size_t)N * 2, cudaMemcpyDeviceToDevice, st));

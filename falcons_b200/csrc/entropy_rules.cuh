@@ -4,12 +4,6 @@
 
 namespace fb2 {
 
-// Whether the items [first, first + count) are among the first n, for any `first` (the sum itself could wrap).
-__host__ __device__ __forceinline__ bool range_within(unsigned long long first, unsigned long long count,
-                                                      unsigned long long n) {
-    return count <= n && first <= n - count;
-}
-
 // Parts of a chain of n codes that decode side by side: one every `part` codes, or (part 0: no checkpoints) one in
 // all, which takes at most kWholeChain codes, the decoder's 32-bit count.  ~0: more than that.
 constexpr unsigned long long kWholeChain = 0xFFFFFFFFull;
