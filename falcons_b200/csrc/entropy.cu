@@ -1979,37 +1979,47 @@ constexpr uint32_t kChunkBits = 7, kChunks = O1_NSYM + (O1_M >> kChunkBits);
 // counts imply (the next context is a function of the decoded code; escapes split between the two
 // large-magnitude contexts 13 and 14).  Those two take slots 0 and 1, so that an escape's sign is the slot.
 __device__ void rank_contexts(const uint16_t *__restrict__ nf, DecRank *__restrict__ out) {
-    __shared__ float P[2][O1_NCTX * O1_NCTX];
-    __shared__ float s_pi[O1_NCTX];
+    __shared__ double P[2][O1_NCTX * O1_NCTX];
+    __shared__ double s_pi[O1_NCTX];
+    __shared__ uint32_t s_n[O1_NCTX * O1_NCTX];  // half cells of a context whose code leads to another
+    __shared__ int s_rank[13];
     const uint32_t t = threadIdx.x;
-    if (t < O1_NCTX * O1_NCTX) P[0][t] = 0;
+    if (t < O1_NCTX * O1_NCTX) s_n[t] = 0;
     __syncthreads();
     for (uint32_t k = t; k < O1_NCTX * O1_NSYM; k += blockDim.x) {
         const int nn = (int16_t)nf[k];
         if (nn == 0 || nn < -1) continue;
-        const uint32_t c = k / O1_NSYM, sy = k % O1_NSYM;
-        const float pr = (float)(nn < 0 ? 1 : nn) / O1_M;
+        const uint32_t c = k / O1_NSYM, sy = k % O1_NSYM, cells = nn < 0 ? 1u : (uint32_t)nn;
         if (sy == O1_NSYM - 1) {
-            atomicAdd(&P[0][c * O1_NCTX + 13], pr / 2);
-            atomicAdd(&P[0][c * O1_NCTX + 14], pr / 2);
+            atomicAdd(&s_n[c * O1_NCTX + 13], cells);
+            atomicAdd(&s_n[c * O1_NCTX + 14], cells);
         } else {
-            atomicAdd(&P[0][c * O1_NCTX + o1_ctx(unzz(sy))], pr);
+            atomicAdd(&s_n[c * O1_NCTX + o1_ctx(unzz(sy))], 2 * cells);
         }
     }
+    __syncthreads();
+    if (t < O1_NCTX * O1_NCTX) P[0][t] = (double)s_n[t] / (2 * O1_M);
     __syncthreads();
     int cur = 0;
     for (int it = 0; it < 7; it++, cur ^= 1) {  // the chain's 128th power by squaring
         if (t < O1_NCTX * O1_NCTX) {
-            float v = 0;
+            double v = 0;
             for (int k = 0; k < O1_NCTX; k++) v += P[cur][t / O1_NCTX * O1_NCTX + k] * P[cur][k * O1_NCTX + t % O1_NCTX];
             P[cur ^ 1][t] = v;
         }
         __syncthreads();
     }
     if (t < O1_NCTX) {
-        float v = 0;
+        double v = 0;
         for (int k = 0; k < O1_NCTX; k++) v += P[cur][k * O1_NCTX + t];
         s_pi[t] = v;
+    }
+    __syncthreads();
+    if (t < 13) {
+        int rank = 2;
+#pragma unroll 1
+        for (uint32_t d = 0; d < 13; d++) rank += s_pi[d] > s_pi[t] || (s_pi[d] == s_pi[t] && d < t);
+        s_rank[t] = rank;
     }
     __syncthreads();
     if (t == 0) {
@@ -2020,11 +2030,7 @@ __device__ void rank_contexts(const uint16_t *__restrict__ nf, DecRank *__restri
         };
         put(13, 0);
         put(14, 1);
-        for (int c = 0; c < 13; c++) {
-            int rank = 2;
-            for (int d = 0; d < 13; d++) rank += s_pi[d] > s_pi[c] || (s_pi[d] == s_pi[c] && d < c);
-            put(c, rank);
-        }
+        for (int c = 0; c < 13; c++) put(c, s_rank[c]);
         *out = r;
     }
 }
