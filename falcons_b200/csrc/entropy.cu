@@ -2149,6 +2149,7 @@ struct EncArgs {
     const EncChain *chains;
     const uint32_t *pstart;      // first part of every chain, then the number of parts
     uint32_t nchains, part, recs;  // codes per part, records per part
+    uint32_t max_rounds;
     const uint32_t *image;       // table sets, kEncSmem bytes each
     const EncCta *ctas;
     // per part: exit state of the first walk and of the last one, entering state of the last one (map
@@ -2166,11 +2167,11 @@ struct EncArgs {
 // Records of one part: its groups of 8 codes (by index) and the final state's.
 inline uint32_t part_records(uint32_t part) { return part / 8 + 2; }
 
-// Whether rounds are left out, and whether the map path codes this call: where more than one part in
-// eight did not meet its kept states, rounds pass a changed state down part by part, and where fewer did
-// not, but several in a row, kMaxRounds do not settle them.  A round is a part's walk, 55 us, the map path
-// 0.9 ms at 6.5 M codes and 4.2 ms at 134 M.
-constexpr uint32_t kMaxRounds = 16;
+// Whether rounds are left out, and whether the map path codes this call: where more than half of the parts did
+// not meet their kept states, rounds pass a changed state down part by part, and where fewer did not, some chains
+// may take more than max_rounds.  A round is a part's walk, 30 to 55 us, the map path 0.9 ms at 12.7 K parts (6.5 M
+// codes) and 4 ms at 98 K (100 M), so the larger the call, the more rounds come before the maps.
+inline uint32_t max_rounds(uint32_t nparts) { return 16 + nparts / 4096; }
 __device__ __forceinline__ bool many_unmet(const EncArgs &A) {
     return (uint32_t)__ldcg(A.err + 5) > __ldg(A.pstart + A.nchains) / 2;
 }
@@ -2757,9 +2758,28 @@ __global__ void __launch_bounds__(kComposeThreads) k_o1_compose(const EncArgs A,
     }
 }
 
+// Whether a chain's rounds end after `round` for the maps' sake, by the parts it has left to run again: they fall by
+// about the same factor from round to round, so those after rounds 4 and 8 tell how many more it takes; from
+// there on, whether another chain's did.
+__device__ __noinline__ bool rounds_too_many(const EncArgs &A, uint32_t round, bool need, uint32_t limit, int &left4) {
+    if (round == 4) left4 = __syncthreads_count(need);
+    if (round < 8) return false;
+    if (round == 8) {
+        const int left = __syncthreads_count(need);
+        if (left > 1 && (left >= left4 || 8.f + 4.f * log2f((float)left) / log2f((float)left4 / (float)left) > (float)limit))
+            return true;
+    }
+    return __syncthreads_or(threadIdx.x == 0 && __ldcg(A.err + 6) != 0);
+}
+
 // Rounds over the parts of this CTA's chain (one a thread, at most): a part runs again while the exit
 // state of the part above is not the state it was last run from.  Returns whether all are settled after
-// `limit` rounds; s_exit holds the exit states.
+// `limit` rounds; s_exit holds the exit states.  With FORECAST it may end after round 8: the parts left fall by about
+// the same factor from round to round, so those after rounds 4 and 8 tell how many more it takes.
+// (With 16 rounds for all: 100 M codes of which 48 % of the parts did not meet ran them and then the maps for 5
+// chains of 176, 5.7 ms, where 29 rounds take 2.6; 384^3 float32 at REL 5e-3, where the parts left of three chains fall by
+// 11 % a round, 4.5 ms, where 8 rounds tell and the maps follow, 3.7.)
+template <bool FORECAST>
 __device__ __forceinline__ bool repair_rounds(const EncArgs &A, uint32_t chain, int table, uint32_t limit,
                                               uint16_t *s_exit) {
     extern __shared__ uint4 smem_raw[];
@@ -2779,6 +2799,7 @@ __device__ __forceinline__ bool repair_rounds(const EncArgs &A, uint32_t chain, 
         bits = A.bits[id];
     }
     bool settled = false;
+    int left4 = 0;
     for (uint32_t round = 1; round <= limit && !settled; round++) {
         uint32_t x = need ? s_exit[t + 1] & (kChanged - 1u) : 0u;
         __syncthreads();
@@ -2795,6 +2816,7 @@ __device__ __forceinline__ bool repair_rounds(const EncArgs &A, uint32_t chain, 
         __syncthreads();
         need = t + 1 < nparts && (s_exit[t + 1] & kChanged);
         settled = !__syncthreads_or(need);
+        if (FORECAST && !settled && round >= 4 && rounds_too_many(A, round, need, limit, left4)) break;
     }
     if (active) {
         s_exit[t] &= kChanged - 1u;
@@ -2809,7 +2831,7 @@ __device__ __forceinline__ bool repair_rounds(const EncArgs &A, uint32_t chain, 
 __global__ void __launch_bounds__(kEncThreads) k_o1_rounds(const EncArgs A, const int *__restrict__ chain_table) {
     __shared__ uint16_t s_exit[kEncThreads];
     if (many_unmet(A) || A.pstart[blockIdx.x + 1] == A.pstart[blockIdx.x]) return;
-    if (!repair_rounds(A, blockIdx.x, chain_table[blockIdx.x], kMaxRounds, s_exit) && threadIdx.x == 0)
+    if (!repair_rounds<true>(A, blockIdx.x, chain_table[blockIdx.x], A.max_rounds, s_exit) && threadIdx.x == 0)
         atomicAdd(A.err + 6, 1);
 }
 
@@ -2830,7 +2852,7 @@ __global__ void __launch_bounds__(kEncThreads) k_o1_settle(const EncArgs A, cons
         if (t == 0) blen[chain] = 0;
         return;
     }
-    if (!repair_rounds(A, chain, chain_table[chain], nparts + 2, s_exit) && t == 0) atomicExch(A.err, 5);
+    if (!repair_rounds<false>(A, chain, chain_table[chain], nparts + 2, s_exit) && t == 0) atomicExch(A.err, 5);
     const bool active = t < nparts;
     const uint32_t id = part0 + t;
     EncPartPos P{};
@@ -3337,6 +3359,7 @@ void encode_chains(Pool &pool, const ChainParts &cp, const Upload &up, const uin
     A.nchains = nchains;
     A.part = part;
     A.recs = part_records(part);
+    A.max_rounds = max_rounds(nparts);
     A.image = image;
     A.ctas = up.get<EncCta>(cp.u_ctas);
     uint16_t *p16 = pool.get<uint16_t>((size_t)nparts * 3);
