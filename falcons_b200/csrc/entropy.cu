@@ -98,8 +98,8 @@ __host__ __device__ __forceinline__ uint32_t fse_ckpt_count(uint32_t n, uint32_t
 // the state of its index parity) side by side, recording every state with the bits that led to it;
 // the group then packs in parallel: warps sum the bits of units of positions, a scan gives every
 // unit its bit position, and the warps write the units (words shared with a neighbour merged with
-// atomicOr); thread 0 appends the two final states and the end mark.  (The chains of these skewed
-// class streams converge too slowly for a speculative split.)  Writes the complete fse_enc record
+// atomicOr); thread 0 appends the two final states and the end mark.  (Parts coded from guessed states
+// do not meet the exact ones within a block of these skewed class streams.)  Writes the complete fse_enc record
 // ([1][u32 len][data] | [0][raw] | [2][sym]) to the block's slot; the record flag goes into bits
 // 56-63 of `sizes`.  `recs` is scratch of kFseRecWords words per block (the 16-bit step records of
 // both chains).
@@ -110,6 +110,10 @@ constexpr unsigned kFseMaxLog = 11;               // the block coder's table log
 // (A row of all L states a symbol saves the shift, but takes 40 KB for ten symbols, so that only four
 // blocks fitted an SM: 758 blocks in two waves, 2.23 ms, now 1.05.)
 constexpr unsigned kFseRows = 2u << kFseMaxLog;
+// A block alone on its SM has room for a row of all L states a symbol instead, where its symbols are few enough: 32-bit
+// cells, the next state times 4, which with the next symbol's row is the next cell's address, and its record.  A
+// step then waits for one addition and one load: a full block's walk takes 520 us, with step rows 650 to 720.
+constexpr unsigned kWideBytes = 24u << (kFseMaxLog + 2);
 // Records per chain: every state (times 16, plus the bits emitted on the way to it), the last one too.
 constexpr unsigned kFseChainRec = FBLK / 2 + 32;
 constexpr unsigned kFseRecWords = kFseChainRec;  // both chains, 2 records per word
@@ -118,9 +122,9 @@ constexpr unsigned kFseBatch = 256;              // steps of a chain staged at a
 constexpr unsigned kPackUnit = 512;              // emission positions a warp packs at a time, 16 a lane
 constexpr unsigned kPackWords = (kPackUnit * kFseMaxLog + 31) / 32 + 1;
 // A CTA codes G blocks side by side, one group of kFseGroupThreads threads each, with its own
-// shared memory and its own named barrier.  G = 1 when the blocks and the chain encoder's CTAs
-// together fit the SMs (a block alone on an SM codes fastest); G = kFseGroups otherwise: the CTA
-// fills an SM (registers), so the blocks sit on an eighth as many SMs as one CTA per block would
+// shared memory and its own named barrier.  G = 1, on an SM of its own (wide rows above), where the blocks and the
+// chain encoder's CTAs together fit the SMs, or where few blocks outlast the chain encoder; G = kFseGroups
+// otherwise: the CTA fills an SM (registers), so the blocks sit on an eighth as many SMs as one CTA per block would
 // spread over, and the chain encoder launched beside them keeps the other SMs.
 constexpr unsigned kFseGroups = 8, kFseGroupThreads = 128, kFseGroupWarps = kFseGroupThreads / 32;
 constexpr unsigned kCountCopies = 8;  // histograms of the count, interleaved
@@ -143,7 +147,7 @@ struct FseGroupSmem {
     uint16_t state_table[1 << kFseMaxLog];
     uint8_t sym[1 << kFseMaxLog];
     int mode;
-    unsigned tl, hdr, fin[2], maxsv, high, bits;
+    unsigned tl, hdr, fin[2], maxsv, high, bits, wide;
     uint32_t sh[32];
     unsigned long long tend;  // traced calls: when the walk ended
 };
@@ -202,6 +206,7 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
     const unsigned slot = blockIdx.x * G + grp;
     if (slot >= njobs) return;  // the other groups synchronise on barriers of their own
     const unsigned bar = 1 + grp;  // named barrier of this group (0 is the CTA's)
+    uint32_t *const wide_rows = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(s_groups) + sizeof(FseGroupSmem));
     FseGroupSmem &w = reinterpret_cast<FseGroupSmem *>(s_groups)[grp];
     const unsigned b = order[slot];  // the largest blocks first
     if (tid == 0) fse_phase(phase, slot, 0);
@@ -285,6 +290,9 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
                 }
             }
         }
+        unsigned present = 0;
+        for (unsigned s2 = 0; s2 <= maxSV && mode == 2; s2++) present += w.norm[s2] != 0;
+        w.wide = G == 1 && ((size_t)present << (tl + 2)) <= kWideBytes;
         w.mode = mode;
         w.tl = tl;
         w.hdr = hdr;
@@ -334,8 +342,11 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
         }
         for (unsigned sy = tid; sy <= maxSV; sy += kFseGroupThreads) {
             const int nn = w.norm[sy];
-            uint32_t total = 0;  // cells of the symbols before sy
-            for (unsigned s2 = 0; s2 < sy; s2++) total += w.norm[s2] == -1 ? 1u : (uint32_t)max(0, (int)w.norm[s2]);
+            uint32_t total = 0, rows = 0;  // cells of the symbols before sy, and how many are present
+            for (unsigned s2 = 0; s2 < sy; s2++) {
+                total += w.norm[s2] == -1 ? 1u : (uint32_t)max(0, (int)w.norm[s2]);
+                rows += w.norm[s2] != 0;
+            }
             uint32_t low = tl;  // the smaller of the symbol's bit counts
             if (nn == 0) {
                 w.sym_tt[sy].deltaNbBits = ((tl + 1) << 16) - L;
@@ -351,11 +362,22 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
                 low = maxBitsOut - 1;
             }
             // the row starts at twice the cells before it (a row of L >> low entries has at most twice its cells)
-            w.step[sy] = (((uint32_t)__cvta_generic_to_shared(w.row) + 4 * min(total, L - 1)) << 5) | (low + 4);
+            w.step[sy] = w.wide ? (uint32_t)__cvta_generic_to_shared(wide_rows) + (rows << (tl + 2))
+                                : (((uint32_t)__cvta_generic_to_shared(w.row) + 4 * min(total, L - 1)) << 5) | (low + 4);
         }
         group_sync(bar);
-        for (unsigned sy = 0; sy <= maxSV; sy++) {
+        for (unsigned sy = 0, rows = 0; sy <= maxSV; sy++) {
             if (w.norm[sy] == 0) continue;
+            if (w.wide) {
+                const fse::SymTT t = w.sym_tt[sy];
+                for (unsigned c = tid; c < L; c += kFseGroupThreads) {
+                    const uint32_t nb = (L + c + t.deltaNbBits) >> 16;
+                    const uint32_t x = w.state_table[(int32_t)((L + c) >> nb) + t.deltaFindState] - L;
+                    wide_rows[(rows << tl) + c] = (x << 2) | (x << 4 | nb) << 16;
+                }
+                rows++;
+                continue;
+            }
             const unsigned low = (w.step[sy] & 31u) - 4;
             uint16_t *row = w.row + ((w.step[sy] >> 5) - (uint32_t)__cvta_generic_to_shared(w.row)) / 2;
             const fse::SymTT t = w.sym_tt[sy];
@@ -397,66 +419,80 @@ __global__ void __launch_bounds__(G * kFseGroupThreads, kFseGroups / G)
             const unsigned rot = ((lead + n - 3) & 15u) + 1, wrot = rot >> 2, brot = (rot & 3u) * 8;
             uint4 x0, x1;
             load(16 * lane, x0, x1);
-            for (unsigned j0 = 0; 2 * j0 < ns; j0 += kFseBatch) {
-                {
-                    uint32_t x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, o[16];
-                    if (wrot & 1u) {
+            auto walk = [&](auto wide_tag) {
+                constexpr bool WIDE = decltype(wide_tag)::value;
+                uint32_t f = e >> 2;  // four times the state minus L
+                for (unsigned j0 = 0; 2 * j0 < ns; j0 += kFseBatch) {
+                    {
+                        uint32_t x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, o[16];
+                        if (wrot & 1u) {
 #pragma unroll
-                        for (int q = 0; q < 7; q++) x[q] = x[q + 1];
+                            for (int q = 0; q < 7; q++) x[q] = x[q + 1];
+                        }
+                        if (wrot & 2u) {
+#pragma unroll
+                            for (int q = 0; q < 6; q++) x[q] = x[q + 2];
+                        }
+                        if (wrot & 4u) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++) x[q] = x[q + 4];
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) x[q] = __funnelshift_r(x[q], x[q + 1], brot);
+#pragma unroll
+                        for (int t = 0; t < 16; t++) o[t] = w.step[(x[(15 - t) >> 2] >> (8 * ((15 - t) & 3))) & 0xFFu];
+#pragma unroll
+                        for (int c = 0; c < 2; c++) {
+                            w.ring[c][2 * lane] = make_uint4(o[c], o[c + 2], o[c + 4], o[c + 6]);
+                            w.ring[c][2 * lane + 1] = make_uint4(o[c + 8], o[c + 10], o[c + 12], o[c + 14]);
+                        }
                     }
-                    if (wrot & 2u) {
+                    load(2 * (j0 + kFseBatch) + 16 * lane, x0, x1);
+                    __syncwarp();
+                    if (lane < 2) {
+                        auto step = [&f](uint32_t o, uint32_t e2) -> uint32_t {
+                            uint16_t r;
+                            if (WIDE) {
+                                const uint32_t at = o + f;
+                                uint16_t g;
+                                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(g) : "r"(at));
+                                asm volatile("ld.shared.u16 %0, [%1+2];" : "=h"(r) : "r"(at));
+                                f = g;
+                            } else {
+                                const uint32_t at = (o >> 5) + 2 * __funnelshift_r(e2, 0u, o);
+                                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(at));
+                            }
+                            return r;
+                        };
+                        const uint4 *rg = w.ring[lane];
+                        const unsigned steps = min(kFseBatch, m - min(m, j0)), ng = steps / 8;
+                        uint4 a = rg[0], c = rg[1];
+                        for (unsigned g = 0; g < ng; g++) {
+                            const unsigned gn = (g + 1) % (kFseBatch / 8);
+                            const uint4 an = rg[2 * gn], cn = rg[2 * gn + 1];
+                            const uint32_t o[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+                            uint32_t r[8];
 #pragma unroll
-                        for (int q = 0; q < 6; q++) x[q] = x[q + 2];
-                    }
-                    if (wrot & 4u) {
-#pragma unroll
-                        for (int q = 0; q < 4; q++) x[q] = x[q + 4];
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) x[q] = __funnelshift_r(x[q], x[q + 1], brot);
-#pragma unroll
-                    for (int t = 0; t < 16; t++) o[t] = w.step[(x[(15 - t) >> 2] >> (8 * ((15 - t) & 3))) & 0xFFu];
-#pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        w.ring[c][2 * lane] = make_uint4(o[c], o[c + 2], o[c + 4], o[c + 6]);
-                        w.ring[c][2 * lane + 1] = make_uint4(o[c + 8], o[c + 10], o[c + 12], o[c + 14]);
-                    }
-                }
-                load(2 * (j0 + kFseBatch) + 16 * lane, x0, x1);
-                __syncwarp();
-                if (lane < 2) {
-                    auto step = [](uint32_t o, uint32_t e2) -> uint32_t {
-                        const uint32_t at = (o >> 5) + 2 * __funnelshift_r(e2, 0u, o);
-                        uint16_t r;
-                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(at));
-                        return r;
-                    };
-                    const uint4 *rg = w.ring[lane];
-                    const unsigned steps = min(kFseBatch, m - min(m, j0)), ng = steps / 8;
-                    uint4 a = rg[0], c = rg[1];
-                    for (unsigned g = 0; g < ng; g++) {
-                        const unsigned gn = (g + 1) % (kFseBatch / 8);
-                        const uint4 an = rg[2 * gn], cn = rg[2 * gn + 1];
-                        const uint32_t o[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-                        uint32_t r[8];
-#pragma unroll
-                        for (int t = 0; t < 8; t++) {
-                            r[t] = e;
+                            for (int t = 0; t < 8; t++) {
+                                r[t] = e;
+                                e = step(o[t], e);
+                            }
+                            *reinterpret_cast<uint4 *>(rk + j0 + 8 * g) =
+                                make_uint4(r[0] | (r[1] << 16), r[2] | (r[3] << 16), r[4] | (r[5] << 16), r[6] | (r[7] << 16));
+                            a = an;
+                            c = cn;
+                        }
+                        const uint32_t *o = reinterpret_cast<const uint32_t *>(rg);
+                        for (unsigned t = 8 * ng; t < steps; t++) {
+                            rk[j0 + t] = (uint16_t)e;
                             e = step(o[t], e);
                         }
-                        *reinterpret_cast<uint4 *>(rk + j0 + 8 * g) =
-                            make_uint4(r[0] | (r[1] << 16), r[2] | (r[3] << 16), r[4] | (r[5] << 16), r[6] | (r[7] << 16));
-                        a = an;
-                        c = cn;
                     }
-                    const uint32_t *o = reinterpret_cast<const uint32_t *>(rg);
-                    for (unsigned t = 8 * ng; t < steps; t++) {
-                        rk[j0 + t] = (uint16_t)e;
-                        e = step(o[t], e);
-                    }
+                    __syncwarp();  // the batch's steps are read
                 }
-                __syncwarp();  // the batch's steps are read
-            }
+            };
+            if (G == 1 && w.wide) walk(std::true_type());
+            else walk(std::false_type());
             if (lane < 2) {
                 rk[m] = (uint16_t)e;
                 w.fin[lane] = e >> 4;
@@ -1078,7 +1114,7 @@ void enable_fse_smem() {
     FB2_CUDA(cudaFuncSetAttribute(k_fse_encode_blocks<kFseGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(kFseGroups * sizeof(FseGroupSmem))));
     FB2_CUDA(cudaFuncSetAttribute(k_fse_encode_blocks<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(FseGroupSmem)));
+                                  (int)(sizeof(FseGroupSmem) + kWideBytes)));
     FB2_CUDA(cudaFuncSetAttribute(k_fse_decode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fse_dec_smem(64)));
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -1097,16 +1133,19 @@ struct GammaBlocks {
     FseCkpt *cks = nullptr;
     size_t ck_per_block = 0;
     unsigned long long *phase = nullptr;  // per-block phase times, traced calls only
-    unsigned longest() const {
+    // About how long the blocks take: 15 ns a symbol of the longest one, 1 ms for a full one, kFseGroups an SM in a wave.
+    double ns() const {
         unsigned n = 0;
         for (const BlockJob &j : jobs) n = std::max(n, j.n);
-        return n;
+        return 15.0 * n * (double)((jobs.size() + kFseGroups * sm_count() - 1) / (kFseGroups * sm_count()));
     }
 };
+// About how long the chain encoder takes for N codes, where most of its parts meet.
+inline double chains_ns(long long N) { return 4e5 + 5e-3 * (double)N; }
 
-// `beside`: CTAs of whole SMs that run next to the class blocks (the chain encoder's).
+// `beside`: CTAs of whole SMs that run next to the class blocks (the chain encoder's), for about `beside_ns`.
 GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned long long> &gstart, cudaStream_t st,
-                         uint32_t ckpt_part, cudaEvent_t queued = nullptr, size_t beside = 0) {
+                         uint32_t ckpt_part, cudaEvent_t queued = nullptr, size_t beside = 0, double beside_ns = 0) {
     GammaBlocks gb;
     gb.gstart = gstart;
     const int G = (int)gstart.size() - 1;
@@ -1147,13 +1186,17 @@ GammaBlocks gamma_launch(Pool &pool, uint8_t *cls, const std::vector<unsigned lo
         FB2_CUDA(cudaMemsetAsync(gb.phase, 0, nj * kFsePhases * 8, st));
     }
     enable_fse_smem();
-    if (nj + beside > (size_t)sm_count()) {
+    // a block an SM where there are SMs for all, or where the few blocks outlast the other CTAs even if those come to two
+    // waves without their SMs: 7 full blocks beside 6.5 M codes end at 1.02 ms eight a CTA and at 0.79 an SM each (the
+    // chains at 0.29 and 0.31)
+    const size_t sms = (size_t)sm_count();
+    if (nj + beside > sms && !(4 * nj <= sms && 2 * beside_ns < gb.ns())) {
         constexpr unsigned G = kFseGroups;
         constexpr int smem = (int)(G * sizeof(FseGroupSmem));
         k_fse_encode_blocks<G><<<(unsigned)((nj + G - 1) / G), G * kFseGroupThreads, smem, st>>>(
             cls, d_jobs, (unsigned)nj, gb.slots, gb.sizes, bits, part, gb.cks, recs, d_order, gb.phase);
     } else {
-        constexpr int smem = (int)sizeof(FseGroupSmem);
+        constexpr int smem = (int)(sizeof(FseGroupSmem) + kWideBytes);
         k_fse_encode_blocks<1><<<(unsigned)nj, kFseGroupThreads, smem, st>>>(
             cls, d_jobs, (unsigned)nj, gb.slots, gb.sizes, bits, part, gb.cks, recs, d_order, gb.phase);
     }
@@ -3884,7 +3927,7 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         // they take a few SMs of their own instead of waiting for the chain encoder's last wave
         const bool queue_first = fork && tune.queued_ev != nullptr;
         const GammaBlocks gblocks = gamma_launch(spool, ecls, gstart, es, cc.fse_part,
-                                                 queue_first ? tune.queued_ev : nullptr, cp.ctas.size());
+                                                 queue_first ? tune.queued_ev : nullptr, cp.ctas.size(), chains_ns(N));
         tr.gpu("class blocks done", es);
         if (queue_first) FB2_CUDA(cudaStreamWaitEvent(st, tune.queued_ev, 0));
         tr.mark("class blocks launched");
@@ -3895,15 +3938,12 @@ void entropy_encode_into(Pool &pool, Assembler &as, const int16_t *d_codes_in, s
         encode_chains(pool, cp, up, keys, (size_t)N, image, enc_part, slots, d_soff, blen, o1ck, d_ck_off, ck_every, d_err, st);
         tr.gpu("chain encoder done", st);
         tr.mark("chains launched");
-        // The mantissas go behind the one that ends first: the chain encoder (0.4 ms and 5 ps a code) or the
-        // class blocks (15 ns a symbol of the longest block, 1 ms for a full one, kFseGroups blocks an SM in a
-        // wave).  384^3 f64, 758 blocks beside 56 M codes: behind the blocks 2.63 ms a call, behind the chains
-        // 2.50; 512^3 f32, where both take as long, the same; 211 x 307 x 401 f32, 3 short blocks: 2.56 ms a
-        // round trip behind the blocks, 2.67 behind the chains.
-        const double chain_ns = 4e5 + 5e-3 * (double)N;
-        const double blocks_ns = 15.0 * (double)gblocks.longest() *
-                                 (double)((gblocks.jobs.size() + kFseGroups * sm_count() - 1) / (kFseGroups * sm_count()));
-        const bool behind_chains = queue_first && chain_ns < blocks_ns;
+        // The mantissas go behind the one that is to end first, the chain encoder or the class blocks (whether the
+        // chains take the map path, 0.9 ms at 6.5 M codes, is known on the device alone).  384^3 f64, 758 blocks
+        // beside 56 M codes: behind the blocks 2.63 ms a call, behind the chains 2.50; 512^3 f32, where both take
+        // as long, the same; 211 x 307 x 401 f32, 3 short blocks: 2.56 ms a round trip behind the blocks, 2.67
+        // behind the chains.
+        const bool behind_chains = queue_first && chains_ns(N) < gblocks.ns();
         cudaStream_t ms = behind_chains ? st : es;
         hold.on = behind_chains;
         const GammaWords gwords = gamma_pack(behind_chains ? pool : spool, ecls, gstart, eraw, ms);
